@@ -87,6 +87,23 @@ LFD_FN LFD_INLINE void lf_flag(u32* error, u32 v) {
 #endif
 }
 
+#ifdef __CUDA_ARCH__
+// One step of a carry chain: a + b with the carry going out (add_cc), in and out (addc_cc), in only (addc).
+__device__ __forceinline__ u32 add_cc(u32 a, u32 b) { u32 r; asm volatile("add.cc.u32 %0, %1, %2;" : "=r"(r) : "r"(a), "r"(b)); return r; }
+__device__ __forceinline__ u32 addc_cc(u32 a, u32 b) { u32 r; asm volatile("addc.cc.u32 %0, %1, %2;" : "=r"(r) : "r"(a), "r"(b)); return r; }
+__device__ __forceinline__ u32 addc(u32 a, u32 b) { u32 r; asm volatile("addc.u32 %0, %1, %2;" : "=r"(r) : "r"(a), "r"(b)); return r; }
+#endif
+
+// Whether any lane here takes a step that shifts by 2^b words: exponent gaps are mostly small, so a warp skips the long
+// steps of a barrel shift altogether (the lanes that do shift still select, so every index stays static).
+LFD_FN LFD_INLINE bool lf_any(bool on) {
+#ifdef __CUDA_ARCH__
+    return __any_sync(__activemask(), on);
+#else
+    return on;
+#endif
+}
+
 template <int N> LFD_FN LFD_INLINE Num<N> zero(u32 st = 0) {
     Num<N> r;
 LFD_UNROLL
@@ -137,8 +154,14 @@ LFD_UNROLL
 // Rounded result r = sign * m * 2^(e-(32N-1)) with the increment decided by the caller.
 template <int N> LFD_FN LFD_INLINE Num<N> finish(u32 (&m)[N], i64 e, int sign, bool up, u32 status) {
     u32 c = up ? 1u : 0u;
+#ifdef __CUDA_ARCH__
+    m[0] = add_cc(m[0], c);
 LFD_UNROLL
+    for (int i = 1; i < N; ++i) m[i] = addc_cc(m[i], 0);
+    c = addc(0, 0);
+#else
     for (int i = 0; i < N; ++i) { u32 t = m[i] + c; c = (c && t == 0) ? 1u : 0u; m[i] = t; }
+#endif
     if (c) { m[N - 1] = 0x80000000u; e += 1; }
     if (e > kEmax || e < -kEmax) return zero<N>(status | kOverflow);
     Num<N> r;
@@ -159,6 +182,7 @@ LFD_UNROLL
                 for (int k = 0; k < W; ++k) x[k] = 0; }
             continue; }
         const bool on = (q >> b) & 1u;
+        if (!lf_any(on)) continue;
 LFD_UNROLL
         for (int k = W - 1; k >= 0; --k) x[k] = on ? (k >= s ? x[k - s] : 0u) : x[k];
     }
@@ -197,26 +221,65 @@ LFD_UNROLL
 }
 
 // ---------------------------------------------------------------- mul
-// Carry-chain primitives (PTX add/mad with .cc): one IMAD per half word product.  GPU only; the host forms
-// of the products below use 64-bit arithmetic instead.
+// Word products in carry chains.  wide_mad_cc / wide_madc_cc add the 64-bit product a * b to the word pair (lo, hi),
+// without and with the incoming carry, and leave the outgoing carry in the condition code: one wide integer
+// multiply-add each (32 a clock and SM, the pipe that bounds every product).  That instruction takes its addend as an
+// aligned register pair, so the products below keep two accumulators: E holds the pairs that start at an even word, O
+// those that start at an odd one, and every row of the schoolbook adds to each by one chain.  Explicit 64-bit carries
+// (product, then two adds to split and carry) and separate chains of low and high halves both issue about three
+// instructions a word product: 16 dependent 1024-bit products of 65,536 values took 120 and 137 us against 92 us.
 #ifdef __CUDA_ARCH__
-__device__ __forceinline__ u32 mad_lo_cc(u32 a, u32 b, u32 c) { u32 r; asm volatile("mad.lo.cc.u32 %0, %1, %2, %3;" : "=r"(r) : "r"(a), "r"(b), "r"(c)); return r; }
-__device__ __forceinline__ u32 madc_lo_cc(u32 a, u32 b, u32 c) { u32 r; asm volatile("madc.lo.cc.u32 %0, %1, %2, %3;" : "=r"(r) : "r"(a), "r"(b), "r"(c)); return r; }
-__device__ __forceinline__ u32 mad_hi_cc(u32 a, u32 b, u32 c) { u32 r; asm volatile("mad.hi.cc.u32 %0, %1, %2, %3;" : "=r"(r) : "r"(a), "r"(b), "r"(c)); return r; }
-__device__ __forceinline__ u32 madc_hi_cc(u32 a, u32 b, u32 c) { u32 r; asm volatile("madc.hi.cc.u32 %0, %1, %2, %3;" : "=r"(r) : "r"(a), "r"(b), "r"(c)); return r; }
-__device__ __forceinline__ u32 madc_hi(u32 a, u32 b, u32 c) { u32 r; asm volatile("madc.hi.u32 %0, %1, %2, %3;" : "=r"(r) : "r"(a), "r"(b), "r"(c)); return r; }
-__device__ __forceinline__ u32 carry_out() { u32 r; asm volatile("addc.u32 %0, 0, 0;" : "=r"(r)); return r; }
+__device__ __forceinline__ void wide_mad_cc(u32& lo, u32& hi, u32 a, u32 b) {
+    asm volatile("mad.lo.cc.u32 %0, %2, %3, %0;\n\tmadc.hi.cc.u32 %1, %2, %3, %1;" : "+r"(lo), "+r"(hi) : "r"(a), "r"(b));
+}
+__device__ __forceinline__ void wide_madc_cc(u32& lo, u32& hi, u32 a, u32 b) {
+    asm volatile("madc.lo.cc.u32 %0, %2, %3, %0;\n\tmadc.hi.cc.u32 %1, %2, %3, %1;" : "+r"(lo), "+r"(hi) : "r"(a), "r"(b));
+}
 
+// The products a_i b_j with i + j >= LO, summed: h[k] is word LO + k.  b: an array or a pointer of B words.  Row j
+// adds b_j a to words LO .. j + A; a row's sum stays below 2^(32(j+A+1)), so the chain that ends at word j + A cannot
+// carry out, and the other chain's carry starts word j + A of its accumulator afresh.
+template <int A, int B, int LO, class Y> __device__ __forceinline__ void mul_rows(const u32 (&a)[A], const Y& b, u32 (&h)[A + B - LO]) {
+    constexpr int W = A + B - LO;
+    u32 E[W + 1], O[W + 1];
+#pragma unroll
+    for (int k = 0; k <= W; ++k) { E[k] = 0; O[k] = 0; }
+#pragma unroll
+    for (int j = 0; j < B; ++j) {
+        const int i0 = LO - j > 0 ? LO - j : 0;                 // first product of the row, at h word i0 + j - LO
+        const int top = j + A - 1 - LO;                          // h word of its last product
+        if (top < 0) continue;
+        const u32 bj = b[j];
+#pragma unroll
+        for (int odd = 0; odd < 2; ++odd) {
+            u32 (&X)[W + 1] = odd ? O : E;
+            bool first = true;
+#pragma unroll
+            for (int i = i0; i < A; ++i) {
+                const int k = i + j - LO;
+                if ((k & 1) != odd) continue;
+                if (first) wide_mad_cc(X[k], X[k + 1], a[i], bj); else wide_madc_cc(X[k], X[k + 1], a[i], bj);
+                first = false;
+            }
+            if (!first && (top & 1) != odd) X[top + 1] = addc(X[top + 1], 0);
+        }
+    }
+    h[0] = E[0];
+    if constexpr (W > 2) h[1] = add_cc(E[1], O[1]);
+#pragma unroll
+    for (int k = 2; k < W - 1; ++k) h[k] = addc_cc(E[k], O[k]);
+    if constexpr (W > 2) h[W - 1] = addc(E[W - 1], O[W - 1]); else h[1] = E[1] + O[1];
+}
 #endif
 
-// a (A words) * b (B words) = p (A + B words): schoolbook rows with explicit 32-bit carries.
+// a (A words) * b (B words) = p (A + B words).
 template <int A, int B> LFD_FN LFD_INLINE void mul_words(const u32 (&a)[A], const u32 (&b)[B], u32 (&p)[A + B]) {
-LFD_UNROLL
+#ifdef __CUDA_ARCH__
+    mul_rows<A, B, 0>(a, b, p);
+#else
     for (int k = 0; k < A + B; ++k) p[k] = 0;
-LFD_UNROLL
     for (int j = 0; j < B; ++j) {
         u32 c = 0;
-LFD_UNROLL
         for (int i = 0; i < A; ++i) {
             const u64 t = (u64)a[i] * b[j] + p[i + j] + c;
             p[i + j] = (u32)t;
@@ -224,30 +287,9 @@ LFD_UNROLL
         }
         p[j + A] = c;
     }
-}
-
-// p (2N words) = a * b, schoolbook by rows: for row i a low-half carry chain adds
-// lo(a_i b_j) into p[i+j] and a high-half chain adds hi(a_i b_j) into p[i+j+1]; the running
-// sum never exceeds 2^(32(i+N+1)), so the last high-half step cannot carry out.
-template <int N> LFD_FN LFD_INLINE void mant_mul(const u32 (&a)[N], const u32 (&b)[N], u32 (&p)[2 * N]) {
-#ifndef __CUDA_ARCH__
-    mul_words<N, N>(a, b, p);
-#else
-LFD_UNROLL
-    for (int k = 0; k < 2 * N; ++k) p[k] = 0;
-LFD_UNROLL
-    for (int i = 0; i < N; ++i) {
-        p[i] = mad_lo_cc(a[i], b[0], p[i]);
-LFD_UNROLL
-        for (int j = 1; j < N; ++j) p[i + j] = madc_lo_cc(a[i], b[j], p[i + j]);
-        p[i + N] = carry_out();
-        p[i + 1] = mad_hi_cc(a[i], b[0], p[i + 1]);
-LFD_UNROLL
-        for (int j = 1; j < N - 1; ++j) p[i + j + 1] = madc_hi_cc(a[i], b[j], p[i + j + 1]);
-        p[i + N] = madc_hi(a[i], b[N - 1], p[i + N]);
-    }
 #endif
 }
+template <int N> LFD_FN LFD_INLINE void mant_mul(const u32 (&a)[N], const u32 (&b)[N], u32 (&p)[2 * N]) { mul_words<N, N>(a, b, p); }
 // Round a product of two normalized mantissas: its top bit is bit 64N-1 or 64N-2.
 template <int N> LFD_FN LFD_INLINE Num<N> round_product(const u32 (&p)[2 * N], i64 e_sum, int sign, u32 status) {
     const u32 s = (p[2 * N - 1] >> 31) ? 0u : 1u;      // normalizing left shift
@@ -273,51 +315,26 @@ template <int N> LFD_FN LFD_NOINLINE Num<N> mul_exact_call(const Num<N> a, const
 // The same with b read inside the call, so a caller's fast path need not keep b's words live for it.
 template <int N> LFD_FN LFD_NOINLINE Num<N> mul_exact_mem_call(const Num<N> a, const u32* b) { return mul_exact<N>(a, load_plain<N>(b)); }
 
-// The same upper part T as mant_mul_high with b's words read from memory: row j adds b_j times a into
-// the window through an explicit 32-bit carry (64-bit products, no condition code), so successive rows
-// are plain data dependencies that the compiler can overlap, and only a and the window live in
-// registers.  a_i b_j + h + c <= (2^32 - 1)^2 + 2 (2^32 - 1) = 2^64 - 1, so no step overflows.
-template <int N> LFD_FN LFD_INLINE void mant_mul_high_mem(const u32 (&a)[N], const u32* b, u32 (&h)[N + 2]) {
+// Upper part of the product: h = T / 2^(32(N-2)) with T = sum of a_i b_j 2^(32(i+j)) over i + j >= N-2
+// (words N-2 .. 2N-1; about 58% of the word products at N = 32).  The omitted products sum to
+// D = sum_{i+j <= N-3} a_i b_j 2^(32(i+j)) < (N-2) 2^(32(N-1)) (1 + 2^-31), so the full product is T + D
+// with D less than N units of word N-1.  b: an array, or a pointer whose words are read as their rows come up (only a
+// and the accumulators then live in registers).
+template <int N, class Y> LFD_FN LFD_INLINE void mant_mul_high(const u32 (&a)[N], const Y& b, u32 (&h)[N + 2]) {
+#ifdef __CUDA_ARCH__
+    mul_rows<N, N, N - 2>(a, b, h);
+#else
     constexpr int B = N - 2;
-LFD_UNROLL
     for (int k = 0; k < N + 2; ++k) h[k] = 0;
-LFD_UNROLL
     for (int j = 0; j < N; ++j) {
         const u32 bj = b[j];
-        const int i0 = B - j > 0 ? B - j : 0;
         u32 c = 0;
-LFD_UNROLL
-        for (int i = i0; i < N; ++i) {
+        for (int i = B - j > 0 ? B - j : 0; i < N; ++i) {
             const u64 t = (u64)a[i] * bj + h[i + j - B] + c;
             h[i + j - B] = (u32)t;
             c = (u32)(t >> 32);
         }
-        h[j + N - B] = c;        // rows before j end at word j + N - B - 1
-    }
-}
-// Upper part of the product: h = T / 2^(32(N-2)) with T = sum of a_i b_j 2^(32(i+j)) over i + j >= N-2
-// (words N-2 .. 2N-1; about 58% of the word products at N = 32).  The omitted products sum to
-// D = sum_{i+j <= N-3} a_i b_j 2^(32(i+j)) < (N-2) 2^(32(N-1)) (1 + 2^-31), so the full product is T + D
-// with D less than N units of word N-1.  Row carries follow mant_mul: T through row i is at most the
-// full partial product, below 2^(32(i+N+1)), so the last high-half step of a row cannot carry out.
-template <int N> LFD_FN LFD_INLINE void mant_mul_high(const u32 (&a)[N], const u32 (&b)[N], u32 (&h)[N + 2]) {
-#ifndef __CUDA_ARCH__
-    mant_mul_high_mem<N>(a, b, h);                 // the same products, summed with explicit carries
-#else
-    constexpr int B = N - 2;
-LFD_UNROLL
-    for (int k = 0; k < N + 2; ++k) h[k] = 0;
-LFD_UNROLL
-    for (int i = 0; i < N; ++i) {
-        const int j0 = B - i > 0 ? B - i : 0;
-        h[i + j0 - B] = mad_lo_cc(a[i], b[j0], h[i + j0 - B]);
-LFD_UNROLL
-        for (int j = j0 + 1; j < N; ++j) h[i + j - B] = madc_lo_cc(a[i], b[j], h[i + j - B]);
-        h[i + N - B] = carry_out();
-        h[i + j0 + 1 - B] = mad_hi_cc(a[i], b[j0], h[i + j0 + 1 - B]);
-LFD_UNROLL
-        for (int j = j0 + 1; j < N - 1; ++j) h[i + j + 1 - B] = madc_hi_cc(a[i], b[j], h[i + j + 1 - B]);
-        h[i + N - B] = madc_hi(a[i], b[N - 1], h[i + N - B]);
+        h[j + N - B] = c;
     }
 #endif
 }
@@ -361,7 +378,7 @@ template <int N> LFD_FN LFD_INLINE Num<N> mul_mem(const Num<N>& a, const u32* y)
         const u32 st = a.st | y[N + 2];
         if (st || !a.s || !ys) return zero<N>(st);
         u32 h[N + 2];
-        mant_mul_high_mem<N>(a.m, y, h);
+        mant_mul_high<N>(a.m, y, h);
         const u32 s = (h[N + 1] >> 31) ? 0u : 1u;
         const u32 lw = h[1] << s;
         const u32 low = lw & 0x7fffffffu;
@@ -382,6 +399,7 @@ LFD_UNROLL
     for (int b = 0; b < STAGES; ++b) {
         const int s = 1 << b;
         const bool on = (q >> b) & 1u;
+        if (!lf_any(on)) continue;
 LFD_UNROLL
         for (int k = 0; k < (s < W ? s : W); ++k) sticky |= on ? x[k] : 0u;
 LFD_UNROLL
@@ -395,6 +413,18 @@ LFD_UNROLL
     x[W - 1] = x[W - 1] >> r;
 }
 
+// a < b as N-word integers: the borrow of a - b.
+template <int N> LFD_FN LFD_INLINE bool mant_less(const u32 (&a)[N], const u32 (&b)[N]) {
+#ifdef __CUDA_ARCH__
+    add_cc(0xffffffffu, 1u);                                      // a + ~b + 1 carries out exactly when a >= b
+LFD_UNROLL
+    for (int i = 0; i < N; ++i) addc_cc(a[i], ~b[i]);
+    return addc(0, 0) == 0;
+#else
+    for (int i = N - 1; i >= 0; --i) if (a[i] != b[i]) return a[i] < b[i];
+    return false;
+#endif
+}
 // RN(a + b).  x = the larger magnitude, y = the smaller, gap = e_x - e_y.  Window of N + 4 words:
 // x's significand at words [3, N+2] (three words below it, one word of headroom above).  y is aligned
 // by shifting it down gap bits from x's position.  When gap <= 96 all of y stays in the window and the
@@ -408,7 +438,8 @@ template <int N> LFD_FN LFD_INLINE Num<N> add(const Num<N>& a, const Num<N>& b) 
     if (st) return zero<N>(st);
     if (!a.s) return b;
     if (!b.s) return a;
-    const bool swap = mag_cmp<N>(a, b) < 0;
+    bool swap = a.e < b.e;
+    if (lf_any(a.e == b.e)) swap = a.e == b.e ? mant_less<N>(a.m, b.m) : swap;
     const Num<N> x = pick<N>(swap, b, a);
     const Num<N> y = pick<N>(swap, a, b);
     const i64 gap = (i64)x.e - y.e;
@@ -421,17 +452,45 @@ LFD_UNROLL
     shift_down_bits<W>(v, (u32)gap & 31u, lost);
     shift_down_words<W, stages_for<W>()>(v, (u32)gap >> 5, lost);
     const u32 l = lost ? 1u : 0u;
-    if (x.s == y.s) {
-        u64 c = 0;
+    // one chain for both signs: x + y_t, or x - y_t - lost as x + ~y_t + (1 - lost)
+    const bool minus = x.s != y.s;
+    const u32 mask = minus ? 0xffffffffu : 0u;
+#ifdef __CUDA_ARCH__
+    add_cc(mask, minus ? 1u - l : 0u);
 LFD_UNROLL
-        for (int k = 0; k < W; ++k) { u64 t = (u64)w[k] + v[k] + c; w[k] = (u32)t; c = t >> 32; }
-    } else {
-        u32 bo = l;                                         // x - y_t - lost
-LFD_UNROLL
-        for (int k = 0; k < W; ++k) { u64 t = (u64)v[k] + bo; u32 old = w[k]; w[k] = (u32)((u64)old - t); bo = (u64)old < t; }
-    }
+    for (int k = 0; k < W - 1; ++k) w[k] = addc_cc(w[k], v[k] ^ mask);
+    w[W - 1] = addc(w[W - 1], v[W - 1] ^ mask);
+#else
+    u64 c = minus ? 1u - l : 0u;
+    for (int k = 0; k < W; ++k) { const u64 t = (u64)w[k] + (v[k] ^ mask) + c; w[k] = (u32)t; c = t >> 32; }
+#endif
     w[0] |= l;
-    return round_general<N, W>(w, (i64)x.e - (32 * N - 1) - 96, x.s, 0);
+    // The top bit is in word N + 3 after a carry, and in word N + 2 unless the difference cancelled 32 bits or more:
+    // one word step covers both, and only a warp that holds a deeper cancellation (or an exact zero) shifts further.
+    i64 e = (i64)x.e - (32 * N - 1) - 96 + 32 * (W - 1) + 31;
+    if (!w[W - 1]) {
+LFD_UNROLL
+        for (int k = W - 1; k > 0; --k) w[k] = w[k - 1];
+        w[0] = 0; e -= 32;
+    }
+    if (lf_any(w[W - 1] == 0)) {
+        int t = -1;
+LFD_UNROLL
+        for (int k = 0; k < W; ++k) t = w[k] ? k : t;
+        if (t < 0) return zero<N>();
+        shift_up_words<W, stages_for<W>()>(w, (u32)(W - 1 - t));
+        e -= 32 * (i64)(W - 1 - t);
+    }
+    const int lz = lf_clz(w[W - 1]);
+    shift_up_bits<W>(w, (u32)lz);
+    u32 m[N];
+LFD_UNROLL
+    for (int i = 0; i < N; ++i) m[i] = w[W - N + i];
+    const u32 below = w[W - N - 1];
+    u32 sticky = below & 0x7fffffffu;
+LFD_UNROLL
+    for (int k = 0; k < W - N - 1; ++k) sticky |= w[k];
+    return finish<N>(m, e - lz, x.s, (below >> 31) && (sticky || (m[0] & 1u)), 0);
 }
 template <int N> LFD_FN LFD_INLINE Num<N> sub(const Num<N>& a, const Num<N>& b) { return add<N>(a, negate<N>(b)); }
 
@@ -449,67 +508,101 @@ LFD_FN LFD_INLINE u32 div2by1(u32 u1, u32 u0, u32 d, u32 v, u32& rem) {
     rem = r;
     return q1;
 }
+// Three-by-two word division with a reused reciprocal (the same paper, algorithms 5 and 6).  (d1, d0) normalized; v = floor((2^96 - 1) / (d1, d0))
+// - 2^32; the quotient floor((u2, u1, u0) / (d1, d0)) for (u2, u1) < (d1, d0).
+LFD_FN LFD_INLINE u32 reciprocal3by2(u32 d1, u32 d0) {
+    u32 v = (u32)(0xffffffffffffffffull / d1 - 0x100000000ull);
+    u32 p = d1 * v + d0;
+    if (p < d0) { --v; if (p >= d1) { --v; p -= d1; } p -= d1; }
+    const u64 t = (u64)v * d0;
+    const u32 t1 = (u32)(t >> 32), t0 = (u32)t;
+    p += t1;
+    if (p < t1) { --v; if ((((u64)p << 32) | t0) >= (((u64)d1 << 32) | d0)) --v; }
+    return v;
+}
+LFD_FN LFD_INLINE u32 div3by2(u32 u2, u32 u1, u32 u0, u32 d1, u32 d0, u32 v) {
+    const u64 d = ((u64)d1 << 32) | d0;
+    const u64 q = (u64)v * u2 + (((u64)u2 << 32) | u1);
+    u32 q1 = (u32)(q >> 32);
+    const u32 q0 = (u32)q;
+    u64 r = ((((u64)(u1 - q1 * d1)) << 32) | u0) - (u64)d0 * q1 - d;
+    ++q1;
+    if ((u32)(r >> 32) >= q0) { --q1; r += d; }
+    if (r >= d) ++q1;
+    return q1;
+}
 // Quotient Q = floor(A * 2^(32N-1+c) / B), c = (A < B), has exactly 32N bits; schoolbook long
 // division by 32-bit digits (Knuth, TAOCP vol. 2, 4.3.1 algorithm D) with the digit estimate
-// above; RNE from the remainder: 2R > B rounds up, 2R == B is a tie.
+// above, which is the digit or one more; RNE from the remainder: 2R > B rounds up, 2R == B is a tie.
+// The remainder is kept complemented, so that subtracting q B adds word products: those that start at an
+// even word go straight into it by one carry chain, the others are formed as pairs and added by a second.  That is
+// two instructions a word product, where a product, two splits and a compare for the borrow took five.
 template <int N> LFD_FN LFD_INLINE Num<N> div(const Num<N>& a, const Num<N>& b) {
     const u32 st = a.st | b.st;
     if (st) return zero<N>(st);
     if (!b.s) return zero<N>(kDivZero);
     if (!a.s) return zero<N>();
-    int cmp = 0;
-LFD_UNROLL
-    for (int i = 0; i < N; ++i) cmp = (a.m[i] != b.m[i]) ? (a.m[i] > b.m[i] ? 1 : -1) : cmp;
-    const int c = cmp < 0 ? 1 : 0;
+    const int c = mant_less<N>(a.m, b.m) ? 1 : 0;
     const i64 e = (i64)a.e - b.e - c;
     if (e > kEmax || e < -kEmax - 1) return zero<N>(kOverflow);
-    u32 u[2 * N + 1];
+    u32 nu[2 * N + 2];                                   // the complement of the remainder
 LFD_UNROLL
-    for (int k = 0; k <= 2 * N; ++k) u[k] = 0;
-    if (c) {
+    for (int k = 0; k < 2 * N + 2; ++k) nu[k] = 0xffffffffu;
+    nu[N - 1] = c ? 0xffffffffu : ~(a.m[0] << 31);
 LFD_UNROLL
-        for (int i = 0; i < N; ++i) u[N + i] = a.m[i];
-    } else {
-        u[N - 1] = a.m[0] << 31;
-LFD_UNROLL
-        for (int i = 0; i < N; ++i) u[N + i] = (a.m[i] >> 1) | (i + 1 < N ? a.m[i + 1] << 31 : 0u);
-    }
-    const u32 d = b.m[N - 1], d2 = b.m[N - 2];
-    const u32 v = (u32)(0xffffffffffffffffull / d - 0x100000000ull);
+    for (int i = 0; i < N; ++i) nu[N + i] = ~(c ? a.m[i] : (a.m[i] >> 1) | (i + 1 < N ? a.m[i + 1] << 31 : 0u));
+    const u32 d1 = b.m[N - 1], d0 = b.m[N - 2];
+    const u32 v = reciprocal3by2(d1, d0);
     u32 q[N];
 LFD_UNROLL
     for (int j = N - 1; j >= 0; --j) {
-        const u32 u1 = u[j + N], u0 = u[j + N - 1];
-        u32 qh, rh;
-        bool rbig;                                   // r-hat >= 2^32: the refinement cannot trigger
-        if (u1 >= d) { qh = 0xffffffffu; u64 r = ((u64)u1 << 32 | u0) - (u64)qh * d; rbig = (r >> 32) != 0; rh = (u32)r; }
-        else { qh = div2by1(u1, u0, d, v, rh); rbig = false; }
-        const u32 u2 = u[j + N - 2];
-LFD_NOUNROLL
-        for (int it = 0; it < 2 && !rbig; ++it) {
-            if ((u64)qh * d2 > (((u64)rh << 32) | u2)) { --qh; u64 nr = (u64)rh + d; rbig = (nr >> 32) != 0; rh = (u32)nr; }
-            else break;
-        }
-        // u[j .. j+N] -= qh * B
-        u64 borrow = 0;
+        const u32 u2 = ~nu[j + N], u1 = ~nu[j + N - 1], u0 = ~nu[j + N - 2];
+        // the remainder is below B 2^(32j), so (u2, u1) <= (d1, d0); equality gives the largest digit
+        u32 qh = (u2 == d1 && u1 == d0) ? 0xffffffffu : div3by2(u2, u1, u0, d1, d0, v);
+        // nu[j .. j+N] += qh * B; a carry out means that qh was one too large
+        u32 over;
+#ifdef __CUDA_ARCH__
+        {
+            bool first = true;
 LFD_UNROLL
-        for (int i = 0; i < N; ++i) {
-            u64 p = (u64)qh * b.m[i] + borrow;
-            u32 lo = (u32)p, old = u[j + i];
-            u[j + i] = old - lo;
-            borrow = (p >> 32) + (old < lo ? 1u : 0u);
+            for (int i = j & 1; i < N; i += 2) {
+                if (first) wide_mad_cc(nu[j + i], nu[j + i + 1], qh, b.m[i]); else wide_madc_cc(nu[j + i], nu[j + i + 1], qh, b.m[i]);
+                first = false;
+            }
+            if ((j + N) % 2 == 0) nu[j + N] = addc_cc(nu[j + N], 0);         // the chain ended below word j + N
+            over = addc(0, 0);
+            first = true;
+LFD_UNROLL
+            for (int i = (j & 1) ^ 1; i < N; i += 2) {
+                const u64 t = (u64)qh * b.m[i];
+                nu[j + i] = first ? add_cc(nu[j + i], (u32)t) : addc_cc(nu[j + i], (u32)t);
+                nu[j + i + 1] = addc_cc(nu[j + i + 1], (u32)(t >> 32));
+                first = false;
+            }
+            if ((j + N) % 2) nu[j + N] = addc_cc(nu[j + N], 0);
+            over |= addc(0, 0);
         }
-        const bool under = (u64)u[j + N] < borrow;
-        u[j + N] = (u32)((u64)u[j + N] - borrow);
-        if (under) {
-            --qh;
+#else
+        {
             u64 cy = 0;
+            for (int i = 0; i < N; ++i) { const u64 t = (u64)qh * b.m[i] + nu[j + i] + cy; nu[j + i] = (u32)t; cy = t >> 32; }
+            const u64 t = (u64)nu[j + N] + cy;
+            nu[j + N] = (u32)t;
+            over = (u32)(t >> 32);
+        }
+#endif
+        if (over) {                                      // add B back: nu -= B
+            --qh;
+            u32 bo = 0;
 LFD_UNROLL
-            for (int i = 0; i < N; ++i) { u64 t = (u64)u[j + i] + b.m[i] + cy; u[j + i] = (u32)t; cy = t >> 32; }
-            u[j + N] += (u32)cy;
+            for (int i = 0; i < N; ++i) { const u64 t = (u64)nu[j + i] - b.m[i] - bo; nu[j + i] = (u32)t; bo = (u32)(t >> 32) & 1u; }
+            nu[j + N] -= bo;
         }
         q[j] = qh;
     }
+    u32 u[N];
+LFD_UNROLL
+    for (int i = 0; i < N; ++i) u[i] = ~nu[i];
     // remainder u[0..N-1]; compare 2R with B
     int half = 0;
     const bool topbit = u[N - 1] >> 31;
@@ -882,13 +975,18 @@ LFD_UNROLL
     shift_up_bits<W>(v, (u32)(offset & 31));
     shift_up_words<W, stages_for<W>()>(v, (u32)(offset >> 5));
 }
+// acc += t, or acc -= t (mod 2^(32W)): one chain of adds, with t complemented and one carried in to subtract.
 template <int W> LFD_FN LFD_INLINE void accumulate(u32 (&acc)[W], const u32 (&t)[W], bool negative) {
-    if (!negative) { u64 cy = 0;
+    const u32 mask = negative ? 0xffffffffu : 0u;
+#ifdef __CUDA_ARCH__
+    add_cc(mask, mask);
 LFD_UNROLL
-        for (int k = 0; k < W; ++k) { u64 x = (u64)acc[k] + t[k] + cy; acc[k] = (u32)x; cy = x >> 32; } }
-    else { u32 bo = 0;
-LFD_UNROLL
-        for (int k = 0; k < W; ++k) { u64 x = (u64)t[k] + bo; u32 old = acc[k]; acc[k] = (u32)((u64)old - x); bo = (u64)old < x; } }
+    for (int k = 0; k < W - 1; ++k) acc[k] = addc_cc(acc[k], t[k] ^ mask);
+    acc[W - 1] = addc(acc[W - 1], t[W - 1] ^ mask);
+#else
+    u64 cy = mask & 1u;
+    for (int k = 0; k < W; ++k) { const u64 x = (u64)acc[k] + (t[k] ^ mask) + cy; acc[k] = (u32)x; cy = x >> 32; }
+#endif
 }
 template <int N> LFD_FN LFD_INLINE Num<N> fma(const Num<N>& a, const Num<N>& b, const Num<N>& c) {
     const u32 st = a.st | b.st | c.st;
