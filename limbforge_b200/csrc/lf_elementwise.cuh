@@ -1,4 +1,4 @@
-// Element-wise kernels: one value per thread, the reference's element layout (AoS) in HBM.
+// Element-wise kernels: one value per thread (one component of a complex value), the reference's element layout (AoS) in HBM.
 // Broadcast operands are read at (i / stride) % period (kernels.metal:7).  Op codes follow
 // limbforge::Operation (engine.hpp:13).  The mul-chain kernel keeps the running value in
 // registers across every step (the fused form of a resident CommandBatch chain).
@@ -24,40 +24,79 @@ __device__ __forceinline__ u64 bidx(u64 i, u64 s, u64 p) { u64 j = s > 1 ? i / s
 
 constexpr int kEwThreads = 128;
 
+constexpr bool ew_complex(int op) { return op == 4 || op == 5 || op == 6 || op == 11 || op == 12; }
+
 template <int N, int OP> __global__ void __launch_bounds__(kEwThreads) ew_kernel(EwParams p) {
     const u64 i = (u64)blockIdx.x * kEwThreads + threadIdx.x;
     if (i >= p.count) return;
     constexpr u64 E = N + 3;
-    if constexpr (OP == 4 || OP == 5 || OP == 6 || OP == 11 || OP == 12) {
-        const Cpx<N> x = cload<N>(p.a + 2 * E * i);
-        const Cpx<N> y = cload<N>(p.b + 2 * E * bidx(i, p.bs, p.bp));
-        Cpx<N> z;
-        if constexpr (OP == 4) z = cadd<N>(x, y);
-        else if constexpr (OP == 5) z = cmul<N>(x, y);
-        else if constexpr (OP == 6) z = cdiv<N>(x, y);
+    const Num<N> x = load<N>(p.a + E * i);
+    Num<N> z;
+    if constexpr (OP == 7) z = mul<N>(x, x);
+    else if constexpr (OP == 8) z = lfd::sqrt<N>(x);
+    else {
+        const Num<N> y = load<N>(p.b + E * bidx(i, p.bs, p.bp));
+        if constexpr (OP == 0) z = add<N>(x, y);
+        else if constexpr (OP == 1) z = sub<N>(x, y);
+        else if constexpr (OP == 2) z = mul<N>(x, y);
+        else if constexpr (OP == 3) z = div<N>(x, y);
         else {
-            const Cpx<N> w = cload<N>(p.c + 2 * E * bidx(i, p.cs, p.cp));
-            z = OP == 11 ? cfma<N>(x, y, w) : cfms<N>(x, y, w);
+            const Num<N> w = load<N>(p.c + E * bidx(i, p.cs, p.cp));
+            z = OP == 9 ? fma<N>(x, y, w) : fms<N>(x, y, w);
         }
-        cstore<N>(p.out + 2 * E * i, z);
-    } else {
-        const Num<N> x = load<N>(p.a + E * i);
-        Num<N> z;
-        if constexpr (OP == 7) z = mul<N>(x, x);
-        else if constexpr (OP == 8) z = lfd::sqrt<N>(x);
-        else {
-            const Num<N> y = load<N>(p.b + E * bidx(i, p.bs, p.bp));
-            if constexpr (OP == 0) z = add<N>(x, y);
-            else if constexpr (OP == 1) z = sub<N>(x, y);
-            else if constexpr (OP == 2) z = mul<N>(x, y);
-            else if constexpr (OP == 3) z = div<N>(x, y);
-            else {
-                const Num<N> w = load<N>(p.c + E * bidx(i, p.cs, p.cp));
-                z = OP == 9 ? fma<N>(x, y, w) : fms<N>(x, y, w);
-            }
-        }
-        store<N>(p.out + E * i, z);
     }
+    store<N>(p.out + E * i, z);
+}
+
+// Complex operations: two lanes per value, one component each (lane 2q real, 2q + 1 imaginary).  The components are
+// independent rounding sequences but for the quotient's denominator |b|^2, whose two squares the lanes form and
+// exchange.  A thread then holds one running sum beside a product instead of two whole complex values, and the serial
+// chain of a quotient is three products and one division instead of six and two: at 1024 bits, where 65,536 pairs are
+// few warps, the operation is bound by that chain's latency.  The products run as one rolled loop whose second factors
+// are read from memory, so the code of one product is fetched once.  Both lanes have read all their operands before
+// either stores (the output may be an input).
+template <int N, int OP> __global__ void __launch_bounds__(kEwThreads, (N > 16 && OP <= 6 ? 3 : 1)) ew_pair_kernel(EwParams p) {
+    constexpr u64 E = N + 3;
+    const u64 t = (u64)blockIdx.x * kEwThreads + threadIdx.x, i = t >> 1;
+    if (i >= p.count) return;                                     // both lanes of a pair leave together
+    const int im = (int)(t & 1);
+    const u32 pair = 3u << (threadIdx.x & 30u);
+    const u32* a = p.a + 2 * E * i;
+    const u32* b = p.b + 2 * E * bidx(i, p.bs, p.bp);
+    Num<N> z;
+    if constexpr (OP == 4) {
+        z = add<N>(load<N>(a + im * E), load<N>(b + im * E));
+    } else if constexpr (OP == 5 || OP == 6) {
+        // product:  re = a.re b.re - a.im b.im          im = a.re b.im + a.im b.re
+        // quotient: re = (a.re b.re + a.im b.im) / d    im = (a.im b.re - a.re b.im) / d
+        z = zero<N>();
+        Num<N> first = z;
+#pragma unroll 1
+        for (int s = 0; s < (OP == 6 ? 3 : 2); ++s) {
+            const u32* x; const u32* y;
+            if constexpr (OP == 5) { x = a + s * E; y = b + (s ^ im) * E; }
+            else { x = s == 2 ? b + im * E : a + (s ^ im) * E; y = s == 2 ? x : b + s * E; }
+            Num<N> q = mul_mem<N>(load<N>(x), y);
+            if (s == 0) { first = q; continue; }
+            if (s == 1) { if (OP == 5 ? !im : im) q.s = -q.s; }
+            else {
+                z = first;                                        // the numerator waits for the denominator
+#pragma unroll
+                for (int w = 0; w < N; ++w) first.m[w] = __shfl_xor_sync(pair, q.m[w], 1);
+                first.e = __shfl_xor_sync(pair, q.e, 1);
+                first.s = __shfl_xor_sync(pair, q.s, 1);
+                first.st = __shfl_xor_sync(pair, q.st, 1);
+            }
+            first = add<N>(first, q);
+        }
+        if constexpr (OP == 6) z = div<N>(z, first); else z = first;
+    } else {
+        const u32* c = p.c + 2 * E * bidx(i, p.cs, p.cp) + im * E;
+        const Num<N> ai = load<N>(a + E), w = load<N>(c);
+        z = dot2_add<N>(load<N>(a), load<N>(b + im * E), im ? ai : negate<N>(ai), load<N>(b + (im ^ 1) * E), OP == 12 ? negate<N>(w) : w);
+    }
+    __syncwarp(pair);
+    store<N>(p.out + 2 * E * i + im * E, z);
 }
 
 // v <- op_s(v, b_s[...]) for every step; out_s written where non-null.  Steps are uniform across
@@ -131,7 +170,7 @@ template <int N> __global__ void __launch_bounds__(kStagedThreads) chain_staged_
     }
 }
 // ---- Lane pairs: one value over two lanes (N even, N >= 12).  Both lanes hold the running value a.  Lane p forms
-// the rows j = 2m + p of the upper part T of a * y (the products a_i y_j with i + j >= N - 2, as mant_mul_high_mem),
+// the rows j = 2m + p of the upper part T of a * y (the products a_i y_j with i + j >= N - 2, as mant_mul_high),
 // each row a carry chain, into its own window; lane p's window index w'' stands for word w'' - 1 + p of T, which
 // keeps every index static.  Lane 1's row 2m + 1 starts one product earlier than lane 0's row 2m; lane 0 takes that
 // product with a zero operand.  One exchange of the windows (a shuffle per word) gives both lanes T, and both round
@@ -237,21 +276,21 @@ inline bool chain_can_stage(const ChainParams& p, u64 E) {
 
 template <int N> int launch_ew(int op, const EwParams& p, cudaStream_t s) {
     if (!p.count) return 0;
-    const unsigned blocks = (unsigned)((p.count + kEwThreads - 1) / kEwThreads);
+    const unsigned blocks = (unsigned)(((ew_complex(op) ? 2 * p.count : p.count) + kEwThreads - 1) / kEwThreads);
     switch (op) {
     case 0: ew_kernel<N, 0><<<blocks, kEwThreads, 0, s>>>(p); break;
     case 1: ew_kernel<N, 1><<<blocks, kEwThreads, 0, s>>>(p); break;
     case 2: ew_kernel<N, 2><<<blocks, kEwThreads, 0, s>>>(p); break;
     case 3: ew_kernel<N, 3><<<blocks, kEwThreads, 0, s>>>(p); break;
-    case 4: ew_kernel<N, 4><<<blocks, kEwThreads, 0, s>>>(p); break;
-    case 5: ew_kernel<N, 5><<<blocks, kEwThreads, 0, s>>>(p); break;
-    case 6: ew_kernel<N, 6><<<blocks, kEwThreads, 0, s>>>(p); break;
+    case 4: ew_pair_kernel<N, 4><<<blocks, kEwThreads, 0, s>>>(p); break;
+    case 5: ew_pair_kernel<N, 5><<<blocks, kEwThreads, 0, s>>>(p); break;
+    case 6: ew_pair_kernel<N, 6><<<blocks, kEwThreads, 0, s>>>(p); break;
     case 7: ew_kernel<N, 7><<<blocks, kEwThreads, 0, s>>>(p); break;
     case 8: ew_kernel<N, 8><<<blocks, kEwThreads, 0, s>>>(p); break;
     case 9: ew_kernel<N, 9><<<blocks, kEwThreads, 0, s>>>(p); break;
     case 10: ew_kernel<N, 10><<<blocks, kEwThreads, 0, s>>>(p); break;
-    case 11: ew_kernel<N, 11><<<blocks, kEwThreads, 0, s>>>(p); break;
-    case 12: ew_kernel<N, 12><<<blocks, kEwThreads, 0, s>>>(p); break;
+    case 11: ew_pair_kernel<N, 11><<<blocks, kEwThreads, 0, s>>>(p); break;
+    case 12: ew_pair_kernel<N, 12><<<blocks, kEwThreads, 0, s>>>(p); break;
     default: return 1;
     }
     return 0;
@@ -284,15 +323,15 @@ template <int N> int ew_attributes(int op, cudaFuncAttributes* a) {
     case 1: return cudaFuncGetAttributes(a, ew_kernel<N, 1>);
     case 2: return cudaFuncGetAttributes(a, ew_kernel<N, 2>);
     case 3: return cudaFuncGetAttributes(a, ew_kernel<N, 3>);
-    case 4: return cudaFuncGetAttributes(a, ew_kernel<N, 4>);
-    case 5: return cudaFuncGetAttributes(a, ew_kernel<N, 5>);
-    case 6: return cudaFuncGetAttributes(a, ew_kernel<N, 6>);
+    case 4: return cudaFuncGetAttributes(a, ew_pair_kernel<N, 4>);
+    case 5: return cudaFuncGetAttributes(a, ew_pair_kernel<N, 5>);
+    case 6: return cudaFuncGetAttributes(a, ew_pair_kernel<N, 6>);
     case 7: return cudaFuncGetAttributes(a, ew_kernel<N, 7>);
     case 8: return cudaFuncGetAttributes(a, ew_kernel<N, 8>);
     case 9: return cudaFuncGetAttributes(a, ew_kernel<N, 9>);
     case 10: return cudaFuncGetAttributes(a, ew_kernel<N, 10>);
-    case 11: return cudaFuncGetAttributes(a, ew_kernel<N, 11>);
-    case 12: return cudaFuncGetAttributes(a, ew_kernel<N, 12>);
+    case 11: return cudaFuncGetAttributes(a, ew_pair_kernel<N, 11>);
+    case 12: return cudaFuncGetAttributes(a, ew_pair_kernel<N, 12>);
     default: return (int)cudaErrorInvalidValue;
     }
 }
