@@ -12,6 +12,7 @@ namespace lfd {
 struct EwParams {
     const u32* a; const u32* b; const u32* c; u32* out;
     u64 count, bs, bp, cs, cp;
+    int aligned;                          // every operand and the output start on 16-byte boundaries
 };
 struct ChainStep { const u32* b; u32* out; u64 bs, bp; int op; int pad; };
 constexpr int kMaxChain = 32;
@@ -24,28 +25,95 @@ __device__ __forceinline__ u64 bidx(u64 i, u64 s, u64 p) { u64 j = s > 1 ? i / s
 
 constexpr int kEwThreads = 128;
 
-constexpr bool ew_complex(int op) { return op == 4 || op == 5 || op == 6 || op == 11 || op == 12; }
+__device__ __forceinline__ void cp_async16(void* smem, const void* gmem) {
+    const unsigned a = (unsigned)__cvta_generic_to_shared(smem);
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" :: "r"(a), "l"(gmem) : "memory");
+}
+__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+template <int G> __device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;" :: "n"(G) : "memory"); }
+__device__ __forceinline__ void cp_async4(void* smem, const void* gmem) {
+    const unsigned a = (unsigned)__cvta_generic_to_shared(smem);
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" :: "r"(a), "l"(gmem) : "memory");
+}
 
-template <int N, int OP> __global__ void __launch_bounds__(kEwThreads) ew_kernel(EwParams p) {
-    const u64 i = (u64)blockIdx.x * kEwThreads + threadIdx.x;
-    if (i >= p.count) return;
-    constexpr u64 E = N + 3;
-    const Num<N> x = load<N>(p.a + E * i);
-    Num<N> z;
-    if constexpr (OP == 7) z = mul<N>(x, x);
-    else if constexpr (OP == 8) z = lfd::sqrt<N>(x);
-    else {
-        const Num<N> y = load<N>(p.b + E * bidx(i, p.bs, p.bp));
-        if constexpr (OP == 0) z = add<N>(x, y);
-        else if constexpr (OP == 1) z = sub<N>(x, y);
-        else if constexpr (OP == 2) z = mul<N>(x, y);
-        else if constexpr (OP == 3) z = div<N>(x, y);
-        else {
-            const Num<N> w = load<N>(p.c + E * bidx(i, p.cs, p.cp));
-            z = OP == 9 ? fma<N>(x, y, w) : fms<N>(x, y, w);
+// A block's rows (elements, or components of complex values) pass through shared memory: a thread's own N + 3 words lie
+// (N + 3) words from its neighbour's, so a load of one word by a warp touches some N + 3 cache lines, and the element-wise
+// kernels were bound by those (300,000 512-bit sums: 35 us, 1.9 TB/s).  Tiles are copied with cp.async, in
+// 16-byte pieces where the block is whole and the arrays are aligned, word by word otherwise (a last block, a broadcast
+// operand, an even row length: those rows are padded to an odd stride, free of bank conflicts).
+template <int N> constexpr int ew_stride() { return (N + 3) | 1; }
+template <int N> __device__ __forceinline__ void ew_fetch(u32* tile, const u32* src, u64 row0, int rows, u64 bs, u64 bp, int parts, bool wide) {
+    constexpr int E = N + 3, S = ew_stride<N>();
+    if (bs == 1 && !bp) {
+        src += row0 * E;
+        if (S == E && wide) {
+            for (int c = threadIdx.x; c < kEwThreads * E / 4; c += kEwThreads) cp_async16(tile + 4 * c, src + 4 * c);
+        } else {
+            for (int w = threadIdx.x; w < rows * E; w += kEwThreads) cp_async4(tile + w + (w / E) * (S - E), src + w);
+        }
+    } else {
+        for (int w = threadIdx.x; w < rows * E; w += kEwThreads) {
+            const int e = w / E;
+            const u64 row = row0 + e, j = parts == 2 ? 2 * bidx(row >> 1, bs, bp) + (row & 1) : bidx(row, bs, bp);
+            cp_async4(tile + w + e * (S - E), src + j * E + (w - e * E));
         }
     }
-    store<N>(p.out + E * i, z);
+}
+template <int N> __device__ __forceinline__ void ew_put(const u32* tile, u32* dst, u64 row0, int rows, bool wide) {
+    constexpr int E = N + 3, S = ew_stride<N>();
+    dst += row0 * E;
+    if (S == E && wide) {
+        for (int c = threadIdx.x; c < kEwThreads * E / 4; c += kEwThreads)
+            reinterpret_cast<uint4*>(dst)[c] = reinterpret_cast<const uint4*>(tile)[c];
+    } else {
+        for (int w = threadIdx.x; w < rows * E; w += kEwThreads) dst[w] = tile[w + (w / E) * (S - E)];
+    }
+}
+constexpr bool ew_complex(int op) { return op == 4 || op == 5 || op == 6 || op == 11 || op == 12; }
+constexpr int ew_inputs(int op) { return op == 7 || op == 8 ? 1 : op >= 9 ? 3 : 2; }
+template <int N> constexpr size_t ew_smem_bytes(int op) { return (size_t)ew_inputs(op) * kEwThreads * ew_stride<N>() * 4; }
+// The block's rows of every operand, in tiles of kEwThreads rows; returns how many rows the block has.
+template <int N, int OP> __device__ __forceinline__ int ew_load_tiles(const EwParams& p, u32* tile, u64 row0, bool& wide) {
+    constexpr int parts = ew_complex(OP) ? 2 : 1, T = kEwThreads * ew_stride<N>();
+    const u64 left = parts * p.count - row0;
+    const int rows = left < (u64)kEwThreads ? (int)left : kEwThreads;
+    wide = p.aligned && rows == kEwThreads;
+    ew_fetch<N>(tile, p.a, row0, rows, 1, 0, parts, wide);
+    if constexpr (ew_inputs(OP) > 1) ew_fetch<N>(tile + T, p.b, row0, rows, p.bs, p.bp, parts, wide);
+    if constexpr (ew_inputs(OP) > 2) ew_fetch<N>(tile + 2 * T, p.c, row0, rows, p.cs, p.cp, parts, wide);
+    cp_async_commit();
+    cp_async_wait<0>();
+    __syncthreads();
+    return rows;
+}
+
+template <int N, int OP> __global__ void __launch_bounds__(kEwThreads) ew_kernel(EwParams p) {
+    constexpr int S = ew_stride<N>(), T = kEwThreads * S;
+    extern __shared__ __align__(16) u32 ew_tiles[];
+    const u64 row0 = (u64)blockIdx.x * kEwThreads;
+    bool wide;
+    const int rows = ew_load_tiles<N, OP>(p, ew_tiles, row0, wide);
+    u32* const mine = ew_tiles + threadIdx.x * S;
+    if ((int)threadIdx.x < rows) {
+        const Num<N> x = load_plain<N>(mine);
+        Num<N> z;
+        if constexpr (OP == 7) z = mul_mem<N>(x, mine);
+        else if constexpr (OP == 8) z = lfd::sqrt<N>(x);
+        else if constexpr (OP == 2) z = mul_mem<N>(x, mine + T);
+        else {
+            const Num<N> y = load_plain<N>(mine + T);
+            if constexpr (OP == 0) z = add<N>(x, y);
+            else if constexpr (OP == 1) z = sub<N>(x, y);
+            else if constexpr (OP == 3) z = div<N>(x, y);
+            else {
+                const Num<N> w = load_plain<N>(mine + 2 * T);
+                z = OP == 9 ? fma<N>(x, y, w) : fms<N>(x, y, w);
+            }
+        }
+        store<N>(mine, z);
+    }
+    __syncthreads();
+    ew_put<N>(ew_tiles, p.out, row0, rows, wide);
 }
 
 // Complex operations: two lanes per value, one component each (lane 2q real, 2q + 1 imaginary).  The components are
@@ -54,49 +122,54 @@ template <int N, int OP> __global__ void __launch_bounds__(kEwThreads) ew_kernel
 // chain of a quotient is three products and one division instead of six and two: at 1024 bits, where 65,536 pairs are
 // few warps, the operation is bound by that chain's latency.  The products run as one rolled loop whose second factors
 // are read from memory, so the code of one product is fetched once.  Both lanes have read all their operands before
-// either stores (the output may be an input).
+// either writes its result over the first operand's row.
 template <int N, int OP> __global__ void __launch_bounds__(kEwThreads, (N > 16 && OP <= 6 ? 3 : 1)) ew_pair_kernel(EwParams p) {
-    constexpr u64 E = N + 3;
-    const u64 t = (u64)blockIdx.x * kEwThreads + threadIdx.x, i = t >> 1;
-    if (i >= p.count) return;                                     // both lanes of a pair leave together
-    const int im = (int)(t & 1);
-    const u32 pair = 3u << (threadIdx.x & 30u);
-    const u32* a = p.a + 2 * E * i;
-    const u32* b = p.b + 2 * E * bidx(i, p.bs, p.bp);
-    Num<N> z;
-    if constexpr (OP == 4) {
-        z = add<N>(load<N>(a + im * E), load<N>(b + im * E));
-    } else if constexpr (OP == 5 || OP == 6) {
-        // product:  re = a.re b.re - a.im b.im          im = a.re b.im + a.im b.re
-        // quotient: re = (a.re b.re + a.im b.im) / d    im = (a.im b.re - a.re b.im) / d
-        z = zero<N>();
-        Num<N> first = z;
+    constexpr int S = ew_stride<N>(), T = kEwThreads * S;
+    extern __shared__ __align__(16) u32 ew_tiles[];
+    const u64 row0 = (u64)blockIdx.x * kEwThreads;
+    bool wide;
+    const int rows = ew_load_tiles<N, OP>(p, ew_tiles, row0, wide);
+    const int im = (int)(threadIdx.x & 1);
+    u32* const a = ew_tiles + (threadIdx.x & ~1u) * S;            // the value's real row; its imaginary row follows
+    const u32* const b = a + T;
+    if ((int)threadIdx.x < rows) {                                // rows is even: both lanes of a pair, or neither
+        const u32 pair = 3u << (threadIdx.x & 30u);
+        Num<N> z;
+        if constexpr (OP == 4) {
+            z = add<N>(load_plain<N>(a + im * S), load_plain<N>(b + im * S));
+        } else if constexpr (OP == 5 || OP == 6) {
+            // product:  re = a.re b.re - a.im b.im          im = a.re b.im + a.im b.re
+            // quotient: re = (a.re b.re + a.im b.im) / d    im = (a.im b.re - a.re b.im) / d
+            z = zero<N>();
+            Num<N> first = z;
 #pragma unroll 1
-        for (int s = 0; s < (OP == 6 ? 3 : 2); ++s) {
-            const u32* x; const u32* y;
-            if constexpr (OP == 5) { x = a + s * E; y = b + (s ^ im) * E; }
-            else { x = s == 2 ? b + im * E : a + (s ^ im) * E; y = s == 2 ? x : b + s * E; }
-            Num<N> q = mul_mem<N>(load<N>(x), y);
-            if (s == 0) { first = q; continue; }
-            if (s == 1) { if (OP == 5 ? !im : im) q.s = -q.s; }
-            else {
-                z = first;                                        // the numerator waits for the denominator
+            for (int s = 0; s < (OP == 6 ? 3 : 2); ++s) {
+                const u32* x; const u32* y;
+                if constexpr (OP == 5) { x = a + s * S; y = b + (s ^ im) * S; }
+                else { x = s == 2 ? b + im * S : a + (s ^ im) * S; y = s == 2 ? x : b + s * S; }
+                Num<N> q = mul_mem<N>(load_plain<N>(x), y);
+                if (s == 0) { first = q; continue; }
+                if (s == 1) { if (OP == 5 ? !im : im) q.s = -q.s; }
+                else {
+                    z = first;                                        // the numerator waits for the denominator
 #pragma unroll
-                for (int w = 0; w < N; ++w) first.m[w] = __shfl_xor_sync(pair, q.m[w], 1);
-                first.e = __shfl_xor_sync(pair, q.e, 1);
-                first.s = __shfl_xor_sync(pair, q.s, 1);
-                first.st = __shfl_xor_sync(pair, q.st, 1);
+                    for (int w = 0; w < N; ++w) first.m[w] = __shfl_xor_sync(pair, q.m[w], 1);
+                    first.e = __shfl_xor_sync(pair, q.e, 1);
+                    first.s = __shfl_xor_sync(pair, q.s, 1);
+                    first.st = __shfl_xor_sync(pair, q.st, 1);
+                }
+                first = add<N>(first, q);
             }
-            first = add<N>(first, q);
+            if constexpr (OP == 6) z = div<N>(z, first); else z = first;
+        } else {
+            const Num<N> ai = load_plain<N>(a + S), w = load_plain<N>(a + 2 * T + im * S);
+            z = dot2_add<N>(load_plain<N>(a), load_plain<N>(b + im * S), im ? ai : negate<N>(ai), load_plain<N>(b + (im ^ 1) * S), OP == 12 ? negate<N>(w) : w);
         }
-        if constexpr (OP == 6) z = div<N>(z, first); else z = first;
-    } else {
-        const u32* c = p.c + 2 * E * bidx(i, p.cs, p.cp) + im * E;
-        const Num<N> ai = load<N>(a + E), w = load<N>(c);
-        z = dot2_add<N>(load<N>(a), load<N>(b + im * E), im ? ai : negate<N>(ai), load<N>(b + (im ^ 1) * E), OP == 12 ? negate<N>(w) : w);
+        __syncwarp(pair);
+        store<N>(a + im * S, z);
     }
-    __syncwarp(pair);
-    store<N>(p.out + 2 * E * i + im * E, z);
+    __syncthreads();
+    ew_put<N>(ew_tiles, p.out, row0, rows, wide);
 }
 
 // v <- op_s(v, b_s[...]) for every step; out_s written where non-null.  Steps are uniform across
@@ -129,14 +202,7 @@ template <int N, bool MUL_ONLY> __global__ void __launch_bounds__(kChainThreads)
 // multiple of 16 bytes) into shared memory with cp.async while the current products run, so the product
 // reads its factor words from shared memory.  A partial last block reads its factors directly.
 constexpr int kStagedThreads = 32;
-__device__ __forceinline__ void cp_async16(void* smem, const void* gmem) {
-    const unsigned a = (unsigned)__cvta_generic_to_shared(smem);
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" :: "r"(a), "l"(gmem) : "memory");
-}
-__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
-template <int G> __device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;" :: "n"(G) : "memory"); }
-
-template <int N> __global__ void __launch_bounds__(kStagedThreads) chain_staged_kernel(const __grid_constant__ ChainParams p) {
+template <int N> __global__ void __launch_bounds__(kStagedThreads, (N > 24 ? 14 : 1)) chain_staged_kernel(const __grid_constant__ ChainParams p) {
     constexpr u64 E = N + 3;
     constexpr int T = kStagedThreads, TILE = T * (int)E, CH = TILE / 4;
     static_assert(TILE % 4 == 0, "tiles of whole 16-byte chunks");
@@ -274,23 +340,35 @@ inline bool chain_can_stage(const ChainParams& p, u64 E) {
     return true;
 }
 
-template <int N> int launch_ew(int op, const EwParams& p, cudaStream_t s) {
-    if (!p.count) return 0;
-    const unsigned blocks = (unsigned)(((ew_complex(op) ? 2 * p.count : p.count) + kEwThreads - 1) / kEwThreads);
+template <int N, int OP> void launch_ew_op(const EwParams& p, cudaStream_t s) {
+    constexpr size_t smem = ew_smem_bytes<N>(OP);
+    const unsigned blocks = (unsigned)(((ew_complex(OP) ? 2 * p.count : p.count) + kEwThreads - 1) / kEwThreads);
+    if constexpr (ew_complex(OP)) {
+        if constexpr (smem > 48 * 1024) cudaFuncSetAttribute(ew_pair_kernel<N, OP>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        ew_pair_kernel<N, OP><<<blocks, kEwThreads, smem, s>>>(p);
+    } else {
+        if constexpr (smem > 48 * 1024) cudaFuncSetAttribute(ew_kernel<N, OP>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        ew_kernel<N, OP><<<blocks, kEwThreads, smem, s>>>(p);
+    }
+}
+template <int N> int launch_ew(int op, const EwParams& pin, cudaStream_t s) {
+    if (!pin.count) return 0;
+    EwParams p = pin;
+    p.aligned = !(((uintptr_t)p.a | (uintptr_t)p.b | (uintptr_t)p.c | (uintptr_t)p.out) & 15);
     switch (op) {
-    case 0: ew_kernel<N, 0><<<blocks, kEwThreads, 0, s>>>(p); break;
-    case 1: ew_kernel<N, 1><<<blocks, kEwThreads, 0, s>>>(p); break;
-    case 2: ew_kernel<N, 2><<<blocks, kEwThreads, 0, s>>>(p); break;
-    case 3: ew_kernel<N, 3><<<blocks, kEwThreads, 0, s>>>(p); break;
-    case 4: ew_pair_kernel<N, 4><<<blocks, kEwThreads, 0, s>>>(p); break;
-    case 5: ew_pair_kernel<N, 5><<<blocks, kEwThreads, 0, s>>>(p); break;
-    case 6: ew_pair_kernel<N, 6><<<blocks, kEwThreads, 0, s>>>(p); break;
-    case 7: ew_kernel<N, 7><<<blocks, kEwThreads, 0, s>>>(p); break;
-    case 8: ew_kernel<N, 8><<<blocks, kEwThreads, 0, s>>>(p); break;
-    case 9: ew_kernel<N, 9><<<blocks, kEwThreads, 0, s>>>(p); break;
-    case 10: ew_kernel<N, 10><<<blocks, kEwThreads, 0, s>>>(p); break;
-    case 11: ew_pair_kernel<N, 11><<<blocks, kEwThreads, 0, s>>>(p); break;
-    case 12: ew_pair_kernel<N, 12><<<blocks, kEwThreads, 0, s>>>(p); break;
+    case 0: launch_ew_op<N, 0>(p, s); break;
+    case 1: launch_ew_op<N, 1>(p, s); break;
+    case 2: launch_ew_op<N, 2>(p, s); break;
+    case 3: launch_ew_op<N, 3>(p, s); break;
+    case 4: launch_ew_op<N, 4>(p, s); break;
+    case 5: launch_ew_op<N, 5>(p, s); break;
+    case 6: launch_ew_op<N, 6>(p, s); break;
+    case 7: launch_ew_op<N, 7>(p, s); break;
+    case 8: launch_ew_op<N, 8>(p, s); break;
+    case 9: launch_ew_op<N, 9>(p, s); break;
+    case 10: launch_ew_op<N, 10>(p, s); break;
+    case 11: launch_ew_op<N, 11>(p, s); break;
+    case 12: launch_ew_op<N, 12>(p, s); break;
     default: return 1;
     }
     return 0;
