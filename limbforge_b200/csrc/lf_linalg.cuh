@@ -50,8 +50,7 @@ template <int N> __global__ void analyze_kernel(LineView v, u64 lines, u64 K, Li
 struct ResPlan {
     int mode, G;
     int L, qwords, NB, Kp, NS; u32 tmem_cols;        // CRT operand of L
-    int dNB; u32 dtmem;                               // digit operand of L
-    const void* tab; const unsigned char* crt_bimg; const unsigned char* dig_bimg;
+    const void* tab; const unsigned char* crt_bimg; const unsigned char* dig_bimg;   // dig_bimg: digit operand of L
 };
 
 struct DotParams {

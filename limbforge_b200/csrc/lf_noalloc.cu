@@ -136,7 +136,7 @@ extern "C" int lf_dev_exact_product_static(int bits, const void* left, size_t le
     uint64_t Kp = 0, Mp = 0, Np = 0, aplane = 0, bplane = 0;
     size_t res_off = 0;
     if (residue) {                                      // planes and residues must fit the array
-        Kp = up(K, lfd::kTileK); Mp = up(M, lfd::kTileM); Np = up(N, lfd::kTileN);
+        Kp = up(K, lfd::kKAlign); Mp = up(M, lfd::kTileM); Np = up(N, lfd::kTileM);
         aplane = (uint64_t)L * Mp * Kp; bplane = (uint64_t)L * Np * Kp;
         res_off = up(planes_off + 2 * (aplane + bplane), 256);
         residue = res_off + sizeof(uint16_t) * (uint64_t)L * M * N <= kScratchBytes;
@@ -162,10 +162,9 @@ extern "C" int lf_dev_exact_product_static(int bits, const void* left, size_t le
         rk->digits(lfd::DigitParams{lv, M, K, Kp, Mp, L, xwords, linfo, tables, a1, a0}, s);
         rk->digits(lfd::DigitParams{rv, N, K, Kp, Np, L, xwords, linfo + M, tables, b1, b0}, s);
         cuda_check(cudaGetLastError(), "digit planes");
-        const CUtensorMap ta1 = residue_plane_map(a1, Kp, Mp, L), ta0 = residue_plane_map(a0, Kp, Mp, L);
-        const CUtensorMap tb1 = residue_plane_map(b1, Kp, Np, L), tb0 = residue_plane_map(b0, Kp, Np, L);
         lfd::MmaParams mp{res, tables, M, N, Kp, lower ? 1 : 0, err};
-        residue_mma_launch(dim3((unsigned)(Np / lfd::kTileN), (unsigned)(Mp / lfd::kTileM), (unsigned)L), ta1, ta0, tb1, tb0, mp, s);
+        residue_mma_launch(residue_plane_map(a1, Kp, Mp, L, true), residue_plane_map(a0, Kp, Mp, L, true),
+                           residue_plane_map(b1, Kp, Np, L, false), residue_plane_map(b0, Kp, Np, L, false), L, mp, s);
         rk->rec(lfd::RecParams{res, tables, L, qwords, linfo, linfo + M, out, ldc, M, N, subtract ? 1 : 0, lower ? 1 : 0}, s);
         cuda_check(cudaGetLastError(), "reconstruction");
     }

@@ -122,8 +122,9 @@ TableSet tables_for(int device, int L) {
     return t;
 }
 
-// Digit-plane operand of one (L, xwords): B[2l + h][b] = byte h of 2^(8b) mod m_l, as the swizzled image.
-struct DigitTable { unsigned char* bimg = nullptr; int NB = 0, KB = 0; unsigned tmem_cols = 0; };
+// Digit-plane operand of one (L, xwords): byte h of 2^(8b) mod m_l in row l of the tile (l / 128, h), repeated down the 128
+// rows as digit_copies says, as the swizzled image.
+struct DigitTable { unsigned char* bimg = nullptr; int KB = 0; };
 std::map<std::tuple<int, int, int>, DigitTable> g_digit_tables;     // (device, L, xwords)
 DigitTable digit_table_for(int device, int L, int xwords) {
     std::lock_guard<std::mutex> lock(g_table_mutex);
@@ -131,27 +132,29 @@ DigitTable digit_table_for(int device, int L, int xwords) {
     auto it = g_digit_tables.find(key);
     if (it != g_digit_tables.end()) return it->second;
     DigitTable t;
-    t.NB = (2 * L + 15) / 16 * 16;
     t.KB = (4 * xwords + 31) / 32 * 32;
-    t.tmem_cols = 32;
-    while ((int)t.tmem_cols < t.NB) t.tmem_cols *= 2;
-    const int kblocks = (t.KB + 127) / 128;
-    std::vector<unsigned char> img((size_t)kblocks * t.NB * 128, 0);
+    const int kblocks = (t.KB + 127) / 128, tiles = lfd::digit_row_tiles(L), rows = 128 / lfd::digit_copies(L);
+    std::vector<unsigned char> img((size_t)2 * tiles * kblocks * 16384, 0);
     const auto& m = primes();
-    for (int l = 0; l < L; ++l) {
-        uint64_t pw = 1 % m[l];
-        for (int b = 0; b < 4 * xwords; ++b) {
-            for (int h = 0; h < 2; ++h)
-                img[(size_t)(b / 128) * t.NB * 128 + lfd::sw128_offset((uint32_t)(2 * l + h), (uint32_t)(b % 128))] = (unsigned char)(pw >> (8 * h));
-            pw = (pw << 8) % m[l];
+    for (int tile = 0; tile < tiles; ++tile)
+        for (int row = 0; row < 128; ++row) {
+            const int l = tile * 128 + row % rows;
+            if (l >= L) continue;
+            uint64_t pw = 1 % m[l];
+            for (int b = 0; b < 4 * xwords; ++b) {
+                for (int h = 0; h < 2; ++h)
+                    img[(size_t)((2 * tile + h) * kblocks + b / 128) * 16384 + lfd::sw128_offset((uint32_t)row, (uint32_t)(b % 128))] =
+                        (unsigned char)(pw >> (8 * h));
+                pw = (pw << 8) % m[l];
+            }
         }
-    }
     cuda_check(cudaMalloc(&t.bimg, img.size()), "digit operand");
     cuda_check(cudaMemcpy(t.bimg, img.data(), img.size(), cudaMemcpyHostToDevice), "digit operand");
     cuda_check(cudaStreamSynchronize(0), "digit operand");
     g_digit_tables[key] = t;
     return t;
 }
+uint64_t round_up(uint64_t x, uint64_t to) { return (x + to - 1) / to * to; }
 // Persistent launch shape of the tcgen05 kernels that hold `tmem_cols` TMEM columns per CTA: as many
 // CTAs per SM as TMEM allows (512 columns), shared memory sized so that no more are resident.
 void tmem_launch_shape(unsigned tmem_cols, size_t smem_need, int sms, uint64_t tiles, unsigned& grid, size_t& smem) {
@@ -176,12 +179,12 @@ EncodeTiled encoder() {
     if (!fn) throw runtime_error("cuTensorMapEncodeTiled unavailable");
     return fn;
 }
-// [L][rows_pad][Kp] int8 planes, 128 x 128 boxes with the 128-byte swizzle.
-CUtensorMap plane_map(void* base, uint64_t Kp, uint64_t rows_pad, int L) {
+// [L][rows_pad][Kp] int8 planes, boxes of 128 bytes by `rows` rows with the 128-byte swizzle (a box beyond Kp reads zeros).
+CUtensorMap plane_map(void* base, uint64_t Kp, uint64_t rows_pad, int L, int rows) {
     CUtensorMap map;
     const cuuint64_t dims[3] = {Kp, rows_pad, (cuuint64_t)L};
     const cuuint64_t strides[2] = {Kp, rows_pad * Kp};
-    const cuuint32_t box[3] = {lfd::kTileK, lfd::kTileM, 1};
+    const cuuint32_t box[3] = {lfd::kTileK, (cuuint32_t)rows, 1};
     const cuuint32_t estr[3] = {1, 1, 1};
     CUresult r = encoder()(&map, CU_TENSOR_MAP_DATA_TYPE_UINT8, 3, base, dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
                            CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
@@ -189,6 +192,16 @@ CUtensorMap plane_map(void* base, uint64_t Kp, uint64_t rows_pad, int L) {
     return map;
 }
 }  // namespace
+
+// The residue products of `moduli` moduli: one CTA per output tile and modulus.
+void residue_mma_launch(const CUtensorMap& ta1, const CUtensorMap& ta0, const CUtensorMap& tb1, const CUtensorMap& tb0, int moduli,
+                        const lfd::MmaParams& p, cudaStream_t s) {
+    const size_t smem = lfd::kStages * lfd::kStageBytes + 1024;
+    cuda_check(cudaFuncSetAttribute(lfd::residue_mma_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem), "smem");
+    const dim3 grid((unsigned)((p.Nc + lfd::kTileN - 1) / lfd::kTileN), (unsigned)((p.M + lfd::kTileM - 1) / lfd::kTileM), (unsigned)moduli);
+    lfd::residue_mma_kernel<<<grid, lfd::kMmaThreads, smem, s>>>(ta1, ta0, tb1, tb0, p);
+    cuda_check(cudaGetLastError(), "residue products");
+}
 
 bool ResidueEngine::run(int bits, lfd::LineView left, lfd::LineView right, uint64_t M, uint64_t Nc, uint64_t K, uint32_t* C,
                         uint64_t ldc, bool subtract, bool lower, uint32_t* error, cudaStream_t s, bool forced,
@@ -235,8 +248,7 @@ bool ResidueEngine::run(int bits, lfd::LineView left, lfd::LineView right, uint6
     int dev = 0;
     cudaGetDevice(&dev);
     TableSet tab = tables_for(dev, L);
-    const uint64_t Kp = (K + lfd::kTileK - 1) / lfd::kTileK * lfd::kTileK;
-    const uint64_t Mp = (M + lfd::kTileM - 1) / lfd::kTileM * lfd::kTileM, Np = (Nc + lfd::kTileN - 1) / lfd::kTileN * lfd::kTileN;
+    const uint64_t Kp = round_up(K, lfd::kKAlign), Mp = round_up(M, lfd::kTileM), Np = round_up(Nc, lfd::kTileM);
     const uint64_t aplane = (uint64_t)L * Mp * Kp, bplane = same ? 0 : (uint64_t)L * Np * Kp;
     auto* pl = static_cast<signed char*>(planes.get(2 * (aplane + bplane) + 256));
     signed char *a1 = pl, *a0 = pl + aplane, *b1 = same ? a1 : pl + 2 * aplane, *b0 = same ? a0 : pl + 2 * aplane + bplane;
@@ -246,25 +258,20 @@ bool ResidueEngine::run(int bits, lfd::LineView left, lfd::LineView right, uint6
     cuda_check(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev), "SM count");
     {
         const DigitTable dt = digit_table_for(dev, L, xwords);
-        const int kblocks = (dt.KB + 127) / 128;
         auto planes_of = [&](lfd::LineView v, uint64_t lines, uint64_t rows_pad, const lfd::LineInfo* info, signed char* d1, signed char* d0) {
             unsigned grid = 0; size_t smem = 0;
-            tmem_launch_shape(dt.tmem_cols, 1024 + (size_t)kblocks * 16384 + (size_t)kblocks * dt.NB * 128, sms, rows_pad * Kp / 128, grid, smem);
-            rk->digits_mma(lfd::DigitMmaParams{v, lines, K, Kp, rows_pad, L, xwords, info, tab.dev, dt.bimg, dt.NB, dt.KB, dt.tmem_cols,
-                                               d1, d0, error}, grid, smem, s);
+            tmem_launch_shape(lfd::digit_tmem_cols(L), lfd::digit_smem_bytes(lfd::digit_row_tiles(L), dt.KB), sms,
+                              rows_pad * Kp / lfd::kDigitCols, grid, smem);
+            rk->digits_mma(lfd::DigitMmaParams{v, lines, K, Kp, rows_pad, L, xwords, info, tab.dev, dt.bimg, dt.KB, d1, d0, error}, grid,
+                           smem, s);
         };
         planes_of(left, M, Mp, linfo, a1, a0);
         if (!same) planes_of(right, Nc, Np, rinfo, b1, b0);
         cuda_check(cudaGetLastError(), "digit planes");
     }
-    const CUtensorMap ta1 = plane_map(a1, Kp, Mp, L), ta0 = plane_map(a0, Kp, Mp, L);
-    const CUtensorMap tb1 = plane_map(b1, Kp, same ? Mp : Np, L), tb0 = plane_map(b0, Kp, same ? Mp : Np, L);
-    const size_t smem = lfd::kStages * lfd::kStageBytes + 1024;
-    cuda_check(cudaFuncSetAttribute(lfd::residue_mma_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem), "smem");
-    lfd::MmaParams mp{res, tab.dev, M, Nc, Kp, lower ? 1 : 0, error};
-    dim3 grid((unsigned)(Np / lfd::kTileN), (unsigned)(Mp / lfd::kTileM), (unsigned)L);
-    lfd::residue_mma_kernel<<<grid, lfd::kMmaThreads, smem, s>>>(ta1, ta0, tb1, tb0, mp);
-    cuda_check(cudaGetLastError(), "residue products");
+    lfd::MmaParams mp{res, tab.dev, M, Nc, Kp, lower ? 1 : 0, error, nullptr, 0, 0, 1};
+    residue_mma_launch(plane_map(a1, Kp, Mp, L, lfd::kTileM), plane_map(a0, Kp, Mp, L, lfd::kTileM),
+                       plane_map(b1, Kp, same ? Mp : Np, L, lfd::kTileN), plane_map(b0, Kp, same ? Mp : Np, L, lfd::kTileN), L, mp, s);
     {
         // persistent CRT: as many CTAs per SM as TMEM holds (512 columns per SM), shared memory sized
         // so that no more than that are resident
@@ -272,7 +279,7 @@ bool ResidueEngine::run(int bits, lfd::LineView left, lfd::LineView right, uint6
         unsigned grid = 0; size_t smem = 0;
         tmem_launch_shape(tab.tmem_cols, 1024 + (size_t)kblocks * 16384 + (size_t)kblocks * tab.NB * 128, sms, (M * Nc + 127) / 128,
                           grid, smem);
-        auto* sf = static_cast<uint32_t*>(misc.get(sizeof(uint32_t) * (uint64_t)(tab.qwords + 4) * M * Nc + 64));
+        auto* sf = static_cast<uint32_t*>(misc.get(sizeof(uint32_t) * (uint64_t)(tab.qwords + lfd::kCrtExtraWords) * M * Nc + 64));
         lfd::CrtParams cp{res, tab.dev, tab.bimg, L, tab.qwords, tab.NB, tab.Kp, tab.NS, tab.tmem_cols, linfo, rinfo, C, ldc, M, Nc,
                           subtract ? 1 : 0, lower ? 1 : 0, error, nullptr, sf};
         rk->crt(cp, grid, smem, s);
@@ -329,14 +336,8 @@ void residue_tables_host(int L, lfd::ResTables& h, int& qwords_out) {
     qwords_out = std::max(qwords, (int)M.size() - 1);
 }
 
-CUtensorMap residue_plane_map(void* base, uint64_t Kp, uint64_t rows_pad, int L) { return plane_map(base, Kp, rows_pad, L); }
-
-void residue_mma_launch(dim3 grid, const CUtensorMap& ta1, const CUtensorMap& ta0, const CUtensorMap& tb1, const CUtensorMap& tb0,
-                        const lfd::MmaParams& p, cudaStream_t s) {
-    const size_t smem = lfd::kStages * lfd::kStageBytes + 1024;
-    cuda_check(cudaFuncSetAttribute(lfd::residue_mma_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem), "smem");
-    lfd::residue_mma_kernel<<<grid, lfd::kMmaThreads, smem, s>>>(ta1, ta0, tb1, tb0, p);
-    cuda_check(cudaGetLastError(), "residue products");
+CUtensorMap residue_plane_map(void* base, uint64_t Kp, uint64_t rows_pad, int L, bool left) {
+    return plane_map(base, Kp, rows_pad, L, left ? lfd::kTileM : lfd::kTileN);
 }
 
 }  // namespace lfr
@@ -353,7 +354,7 @@ struct ResidentProduct {
     int device = 0, sms = 0, Lmin = 0, Lmax = 0, xwords = 0;
     DevBuf lines, planes, res, plan, cands, cum, error, sf;
     uint64_t Kp = 0, Mp = 0, Np = 0;
-    int maxNB = 0, maxKp = 0, maxDNB = 0, KB = 0; unsigned maxTmem = 0, maxDTmem = 0;
+    int maxNB = 0, maxKp = 0, KB = 0; unsigned maxTmem = 0;
     CUtensorMap ta1{}, ta0{}, tb1{}, tb0{};
     cudaEvent_t done = nullptr;
     bool launched = false;
@@ -405,28 +406,27 @@ std::shared_ptr<ResidentProduct> resident_product_create(int bits, lfd::LineView
         const DigitTable d = digit_table_for(r->device, L, r->xwords);
         lfd::ResPlan& c = cand[i];
         c.mode = 1; c.L = L; c.qwords = t.qwords; c.NB = t.NB; c.Kp = t.Kp; c.NS = t.NS; c.tmem_cols = t.tmem_cols;
-        c.dNB = d.NB; c.dtmem = d.tmem_cols; c.tab = t.dev; c.crt_bimg = t.bimg; c.dig_bimg = d.bimg;
+        c.tab = t.dev; c.crt_bimg = t.bimg; c.dig_bimg = d.bimg;
         double have = 0;
         for (int l = 0; l < L; ++l) have += std::log2((double)primes()[l]);
         cum[i] = have;
         r->maxNB = std::max(r->maxNB, t.NB); r->maxKp = std::max(r->maxKp, t.Kp); r->maxTmem = std::max(r->maxTmem, t.tmem_cols);
-        r->maxDNB = std::max(r->maxDNB, d.NB); r->maxDTmem = std::max(r->maxDTmem, d.tmem_cols); r->KB = d.KB;
+        r->KB = d.KB;
     }
     cuda_check(cudaMemcpy(r->cands.get(sizeof(lfd::ResPlan) * count), cand.data(), sizeof(lfd::ResPlan) * count, cudaMemcpyHostToDevice), "plan candidates");
     cuda_check(cudaMemcpy(r->cum.get(sizeof(double) * count), cum.data(), sizeof(double) * count, cudaMemcpyHostToDevice), "plan candidates");
     cuda_check(cudaStreamSynchronize(0), "plan candidates");
-    r->Kp = (K + lfd::kTileK - 1) / lfd::kTileK * lfd::kTileK;
-    r->Mp = (M + lfd::kTileM - 1) / lfd::kTileM * lfd::kTileM;
-    r->Np = (Nc + lfd::kTileN - 1) / lfd::kTileN * lfd::kTileN;
+    r->Kp = round_up(K, lfd::kKAlign); r->Mp = round_up(M, lfd::kTileM); r->Np = round_up(Nc, lfd::kTileM);
     const uint64_t aplane = (uint64_t)r->Lmax * r->Mp * r->Kp, bplane = r->same ? 0 : (uint64_t)r->Lmax * r->Np * r->Kp;
     auto* pl = static_cast<signed char*>(r->planes.get(2 * (aplane + bplane) + 256));
     signed char *a1 = pl, *a0 = pl + aplane, *b1 = r->same ? a1 : pl + 2 * aplane, *b0 = r->same ? a0 : pl + 2 * aplane + bplane;
     r->res.get(sizeof(uint16_t) * (uint64_t)r->Lmax * M * Nc + 64);
     int maxq = 0;
     for (const auto& c : cand) maxq = std::max(maxq, c.qwords);
-    r->sf.get(sizeof(uint32_t) * (uint64_t)(maxq + 4) * M * Nc + 64);
-    r->ta1 = plane_map(a1, r->Kp, r->Mp, r->Lmax); r->ta0 = plane_map(a0, r->Kp, r->Mp, r->Lmax);
-    r->tb1 = plane_map(b1, r->Kp, r->same ? r->Mp : r->Np, r->Lmax); r->tb0 = plane_map(b0, r->Kp, r->same ? r->Mp : r->Np, r->Lmax);
+    r->sf.get(sizeof(uint32_t) * (uint64_t)(maxq + lfd::kCrtExtraWords) * M * Nc + 64);
+    r->ta1 = plane_map(a1, r->Kp, r->Mp, r->Lmax, lfd::kTileM); r->ta0 = plane_map(a0, r->Kp, r->Mp, r->Lmax, lfd::kTileM);
+    r->tb1 = plane_map(b1, r->Kp, r->same ? r->Mp : r->Np, r->Lmax, lfd::kTileN);
+    r->tb0 = plane_map(b0, r->Kp, r->same ? r->Mp : r->Np, r->Lmax, lfd::kTileN);
     return r;
 }
 
@@ -452,22 +452,18 @@ void resident_product_launch(ResidentProduct& r, cudaStream_t s) {
         auto* pl = static_cast<signed char*>(r.planes.p);
         signed char *a1 = pl, *a0 = pl + aplane, *b1 = r.same ? a1 : pl + 2 * aplane, *b0 = r.same ? a0 : pl + 2 * aplane + bplane;
         auto* res = static_cast<uint16_t*>(r.res.p);
-        const int kblocks = (r.KB + 127) / 128;
         auto planes_of = [&](lfd::LineView v, uint64_t lines, uint64_t rows_pad, const lfd::LineInfo* info, signed char* d1, signed char* d0) {
             unsigned grid = 0; size_t smem = 0;
-            tmem_launch_shape(r.maxDTmem, 1024 + (size_t)kblocks * 16384 + (size_t)kblocks * r.maxDNB * 128, r.sms, rows_pad * r.Kp / 128,
-                              grid, smem);
-            lfd::DigitMmaParams dp{v, lines, r.K, r.Kp, rows_pad, 0, r.xwords, info, nullptr, nullptr, 0, r.KB, 0, d1, d0, err, plan};
+            tmem_launch_shape(lfd::digit_tmem_cols(r.Lmax), lfd::digit_smem_bytes(lfd::digit_row_tiles(r.Lmax), r.KB), r.sms,
+                              rows_pad * r.Kp / lfd::kDigitCols, grid, smem);
+            lfd::DigitMmaParams dp{v, lines, r.K, r.Kp, rows_pad, 0, r.xwords, info, nullptr, nullptr, r.KB, d1, d0, err, plan};
             rk->digits_mma(dp, grid, smem, s);
         };
         planes_of(r.left, r.M, r.Mp, linfo, a1, a0);
         if (!r.same) planes_of(r.right, r.Nc, r.Np, rinfo, b1, b0);
         cuda_check(cudaGetLastError(), "digit planes");
-        const size_t smem = lfd::kStages * lfd::kStageBytes + 1024;
-        cuda_check(cudaFuncSetAttribute(lfd::residue_mma_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem), "smem");
-        lfd::MmaParams mp{res, nullptr, r.M, r.Nc, r.Kp, r.lower ? 1 : 0, err, plan};
-        dim3 grid((unsigned)(r.Np / lfd::kTileN), (unsigned)(r.Mp / lfd::kTileM), (unsigned)r.Lmax);
-        lfd::residue_mma_kernel<<<grid, lfd::kMmaThreads, smem, s>>>(r.ta1, r.ta0, r.tb1, r.tb0, mp);
+        lfd::MmaParams mp{res, nullptr, r.M, r.Nc, r.Kp, r.lower ? 1 : 0, err, plan, 0, 0, 1};
+        residue_mma_launch(r.ta1, r.ta0, r.tb1, r.tb0, r.Lmax, mp, s);
         cuda_check(cudaGetLastError(), "residue products");
         const int ckb = (r.maxKp + 127) / 128;
         unsigned cgrid = 0; size_t csmem = 0;
@@ -539,7 +535,7 @@ bool resident_product_report(ResidentProduct& r, lf_linalg_report& rep) {
 }  // namespace lfr
 
 // ---------------------------------------------------------------- failure detection test hook
-// One 128 x 128 tile of the residue products with the producer's loads left out, so the MMA issuer's first
+// One tile of the residue products with the producer's loads left out, so the MMA issuer's first
 // barrier wait never completes and gives up after `polls` polls: the kernel records error 2, frees its TMEM and
 // returns, and the context stays usable.  The value of the error word comes back in *error_word.
 extern "C" int lf_test_residue_wait_limit(unsigned polls, uint32_t* error_word) {
@@ -556,13 +552,9 @@ extern "C" int lf_test_residue_wait_limit(unsigned polls, uint32_t* error_word) 
     auto* r16 = static_cast<uint16_t*>(res.get(64));
     auto* e = static_cast<uint32_t*>(err.get(16));
     cuda_check(cudaMemset(e, 0, 16), "error word");
-    const CUtensorMap t1 = plane_map(pl, Kp, Mp, 1), t0 = plane_map(pl + Mp * Kp, Kp, Mp, 1);
-    const CUtensorMap u1 = plane_map(pl + 2 * Mp * Kp, Kp, Mp, 1), u0 = plane_map(pl + 3 * Mp * Kp, Kp, Mp, 1);
     lfd::MmaParams mp{r16, tab.dev, 1, 1, Kp, 0, e, nullptr, polls, 1};
-    const size_t smem = lfd::kStages * lfd::kStageBytes + 1024;
-    cuda_check(cudaFuncSetAttribute(lfd::residue_mma_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem), "smem");
-    lfd::residue_mma_kernel<<<dim3(1, 1, 1), lfd::kMmaThreads, smem, nullptr>>>(t1, t0, u1, u0, mp);
-    cuda_check(cudaGetLastError(), "launch");
+    residue_mma_launch(plane_map(pl, Kp, Mp, 1, lfd::kTileM), plane_map(pl + Mp * Kp, Kp, Mp, 1, lfd::kTileM),
+                       plane_map(pl + 2 * Mp * Kp, Kp, Mp, 1, lfd::kTileN), plane_map(pl + 3 * Mp * Kp, Kp, Mp, 1, lfd::kTileN), 1, mp, nullptr);
     cuda_check(cudaDeviceSynchronize(), "bounded wait");
     cuda_check(cudaMemcpy(error_word, e, 4, cudaMemcpyDeviceToHost), "error word");
     LF_API_END

@@ -82,17 +82,22 @@ template <int N> __global__ void __launch_bounds__(128) digits_kernel(DigitParam
 }
 
 // ---------------------------------------------------------------- 2. tcgen05 residue products
-constexpr int kTileM = 128, kTileN = 128, kTileK = 128;      // K tile in int8 elements = one 128-byte row
-constexpr int kStages = 3;                                    // 3 x 64 KB of operand tiles (of 227 KB shared)
-constexpr int kTileBytes = kTileM * kTileK;                   // 16 KB per operand tile
-constexpr int kStageBytes = 4 * kTileBytes;                   // D1a, D0a, D1b, D0b
+// Output tiles of 128 x 64: the three accumulators take 192 of 256 allocated TMEM columns and two stages 96 KB, so two
+// CTAs share an SM and one's epilogue runs under the other's loads and MMAs (a 128 x 128 tile fills TMEM and leaves
+// the tensor pipe idle during its epilogue: 33% active).
+constexpr int kTileM = 128, kTileN = 64, kTileK = 128;       // K tile in int8 elements = one 128-byte row
+constexpr int kKAlign = 32;                                   // planes hold K rounded up to one MMA step, not a whole tile
+constexpr int kStages = 2;
+constexpr int kTileABytes = kTileM * kTileK, kTileBBytes = kTileN * kTileK;
+constexpr int kStageBytes = 2 * (kTileABytes + kTileBBytes);  // D1a, D0a, D1b, D0b
+constexpr u32 kMmaTmem = 256;
 constexpr u32 kSpinLimit = 1u << 28;                          // bounded mbarrier waits
 constexpr int kMmaThreads = 256;                              // warps w and w + 4 share TMEM lanes 32 (w % 4) ..
 constexpr int kDigitThreads = 256;                            // digit planes: the same lane sharing
 constexpr int kCrtThreads = 256;                              // CRT column sums: the same lane sharing
 
 struct MmaParams {
-    u16* res;                               // [L][M][Nc] residues (0 <= r < m)
+    u16* res;                               // [L][M][Nc] residues (0 <= r < m), times w_l mod m_l when weighted
     const ResTables* tab;
     u64 M, Nc, Kp;
     int lower;                              // skip tiles strictly above the diagonal (SYRK)
@@ -100,6 +105,7 @@ struct MmaParams {
     const ResPlan* plan;                    // planned on the GPU: moduli at or above plan->L have no work
     u32 poll_limit;                         // polls of a barrier wait before it gives up (0: kSpinLimit)
     int no_loads;                           // failure test only: the producer issues no loads, so the first wait runs out
+    int weighted;                           // store t_l = r w_l mod m_l, the operand of the tensor-core CRT
 };
 
 __device__ __forceinline__ u32 smem_u32(const void* p) { return (u32)__cvta_generic_to_shared(p); }
@@ -131,7 +137,7 @@ __device__ __forceinline__ u64 smem_desc(const void* p) {
     const u64 start = (smem_u32(p) >> 4) & 0x3FFFu;
     return start | (1ull << 16) | (64ull << 32) | (1ull << 46) | (2ull << 61);
 }
-// kind::i8: D s32, A s8, B s8, both K-major, M = 128, N = 128.
+// kind::i8: D s32, A s8, B s8, both K-major, M = 128, N = kTileN.
 constexpr u32 kIdesc = (2u << 4) | (1u << 7) | (1u << 10) | ((u32)(kTileN >> 3) << 17) | ((u32)(kTileM >> 4) << 24);
 
 __device__ __forceinline__ void mma_i8(u32 d_tmem, u64 a, u64 b, bool accumulate) {
@@ -153,11 +159,14 @@ __device__ __forceinline__ void tmem_ld32(u32 taddr, u32 (&r)[32]) {
 }
 
 #ifdef LF_RESIDUE_MMA_KERNEL
-// One CTA = one 128 x 128 output tile of one modulus (grid z).  Warp 0 lane 0 issues TMA loads,
+// x mod m in [0, 2m) for any 32-bit x, rr = floor(2^32 / m).
+__device__ __forceinline__ u32 mod_lazy(u32 x, u32 m, u32 rr) { return x - __umulhi(x, rr) * m; }
+// One CTA = one 128 x 64 output tile of one modulus (grid z).  Warp 0 lane 0 issues TMA loads,
 // warp 1 lane 0 issues the MMAs; then all eight warps reduce the accumulators: warp w reads TMEM lanes
 // 32 (w % 4) .. + 31 (rows) for the columns of half w / 4 and stores 32 residues of a row with four
-// 16-byte stores when the row stride allows.
-__global__ void __launch_bounds__(kMmaThreads, 1) residue_mma_kernel(const __grid_constant__ CUtensorMap ta1, const __grid_constant__ CUtensorMap ta0,
+// 16-byte stores when the row stride allows.  The planes end at K rounded up to one MMA step of 32; the last
+// K tile's rows beyond it are zeros that the TMA load fills in, and no MMA reads them.
+__global__ void __launch_bounds__(kMmaThreads, 2) residue_mma_kernel(const __grid_constant__ CUtensorMap ta1, const __grid_constant__ CUtensorMap ta0,
                                                               const __grid_constant__ CUtensorMap tb1, const __grid_constant__ CUtensorMap tb0,
                                                               MmaParams p) {
     extern __shared__ __align__(1024) unsigned char smem_raw[];
@@ -178,7 +187,7 @@ __global__ void __launch_bounds__(kMmaThreads, 1) residue_mma_kernel(const __gri
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     if (warp == 0) {
-        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], 512;" :: "r"(smem_u32(&tmem_slot)));
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" :: "r"(smem_u32(&tmem_slot)), "r"(kMmaTmem));
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
     }
     asm volatile("tcgen05.fence::before_thread_sync;");
@@ -186,7 +195,7 @@ __global__ void __launch_bounds__(kMmaThreads, 1) residue_mma_kernel(const __gri
     asm volatile("tcgen05.fence::after_thread_sync;");
     const u32 tmem = tmem_slot;
     const u32 acc11 = tmem, acc00 = tmem + kTileN, accm = tmem + 2 * kTileN;
-    const int kblocks = (int)(p.Kp / kTileK);
+    const int kblocks = (int)((p.Kp + kTileK - 1) / kTileK);
     const u32 polls = p.poll_limit ? p.poll_limit : kSpinLimit;
     __shared__ int abort_flag, issued, consumed;          // stages loaded by the producer / read by the MMA issuer
     if (threadIdx.x == 0) { abort_flag = 0; issued = 0; consumed = kblocks; }
@@ -201,9 +210,9 @@ __global__ void __launch_bounds__(kMmaThreads, 1) residue_mma_kernel(const __gri
             unsigned char* st = smem + s * kStageBytes;
             mbar_expect_tx(&full[s], kStageBytes);
             tma_load_3d(st, &ta1, &full[s], kb * kTileK, tm * kTileM, l);
-            tma_load_3d(st + kTileBytes, &ta0, &full[s], kb * kTileK, tm * kTileM, l);
-            tma_load_3d(st + 2 * kTileBytes, &tb1, &full[s], kb * kTileK, tn * kTileN, l);
-            tma_load_3d(st + 3 * kTileBytes, &tb0, &full[s], kb * kTileK, tn * kTileN, l);
+            tma_load_3d(st + kTileABytes, &ta0, &full[s], kb * kTileK, tm * kTileM, l);
+            tma_load_3d(st + 2 * kTileABytes, &tb1, &full[s], kb * kTileK, tn * kTileN, l);
+            tma_load_3d(st + 2 * kTileABytes + kTileBBytes, &tb0, &full[s], kb * kTileK, tn * kTileN, l);
             issued = kb + 1;
         }
     } else if (warp == 1 && lane == 0) {
@@ -215,10 +224,10 @@ __global__ void __launch_bounds__(kMmaThreads, 1) residue_mma_kernel(const __gri
             if (!mbar_wait(&full[s], ph, p.error, polls)) { ok = false; consumed = kb; *(volatile int*)&abort_flag = 1; break; }
             asm volatile("tcgen05.fence::after_thread_sync;");
             unsigned char* st = smem + s * kStageBytes;
-            const u64 a1 = smem_desc(st), a0 = smem_desc(st + kTileBytes), b1 = smem_desc(st + 2 * kTileBytes),
-                      b0 = smem_desc(st + 3 * kTileBytes);
-#pragma unroll
-            for (int kk = 0; kk < kTileK / 32; ++kk) {
+            const u64 a1 = smem_desc(st), a0 = smem_desc(st + kTileABytes), b1 = smem_desc(st + 2 * kTileABytes),
+                      b0 = smem_desc(st + 2 * kTileABytes + kTileBBytes);
+            const int left = (int)(p.Kp - (u64)kb * kTileK) / 32, steps = left < kTileK / 32 ? left : kTileK / 32;
+            for (int kk = 0; kk < steps; ++kk) {
                 const u64 off = (u64)(kk * 32) >> 4;           // 32 bytes along K inside the swizzled row
                 const bool acc = kb > 0 || kk > 0;
                 mma_i8(acc11, a1 + off, b1 + off, acc);
@@ -240,8 +249,10 @@ __global__ void __launch_bounds__(kMmaThreads, 1) residue_mma_kernel(const __gri
     asm volatile("tcgen05.fence::after_thread_sync;");
     if (fine) {
         const u32 m = tab->m[l];
-        const u64 br = tab->barrett[l];
-        const u32 moff = m - mod_barrett(1ull << 49, m, br);  // m - (2^49 mod m), in (0, m]
+        const u32 rr = (u32)(tab->barrett[l] >> 32);          // floor(2^64 / m) >> 32 = floor(2^32 / m)
+        const u32 w = p.weighted ? tab->w[l] : 1u;
+        // multiples of m that make the sums nonnegative: |S11|, |S00| < 2^30 and |Smid| < 2^31 for K <= kMaxK
+        const u32 off30 = ((1u << 30) / m + 1) * m, off31 = ((1u << 31) / m) * m;
         const int q = warp & 3, half = warp >> 2;
         const u64 row = (u64)tm * kTileM + q * 32 + lane;
         const u32 lane_base = (u32)(q * 32) << 16;
@@ -258,10 +269,13 @@ __global__ void __launch_bounds__(kMmaThreads, 1) residue_mma_kernel(const __gri
                 u32 r[32];
 #pragma unroll
                 for (int c = 0; c < 32; ++c) {
-                    // 65536 S11 + 256 Smid + S00 (|.| < 2^48), made nonnegative by 2^49 and reduced
-                    const long long v = (long long)(int)s11[c] * 65536 + (long long)(int)sm[c] * 256 + (long long)(int)s00[c];
-                    const u32 t = mod_barrett((u64)(v + (1ll << 49)), m, br) + moff;     // in (0, 2m)
-                    r[c] = t >= m ? t - m : t;
+                    // 65536 S11 + 256 Smid + S00 by Horner's rule in 32-bit words: every mod_lazy leaves [0, 2m), 2m < 2^17
+                    const u32 hi = mod_lazy(s11[c] + off30, m, rr) * 256u + mod_lazy(sm[c] + off31, m, rr);
+                    const u32 x = mod_lazy(hi, m, rr) * 256u + (s00[c] + off30);
+                    u32 t = mod_lazy(x, m, rr);
+                    t = min(t, t - m);                         // [0, m)
+                    t = mod_lazy(t * w, m, rr);
+                    r[c] = min(t, t - m);
                 }
                 if (vec && col0 + 32 <= p.Nc) {
                     uint4* o = reinterpret_cast<uint4*>(out);
@@ -279,7 +293,7 @@ __global__ void __launch_bounds__(kMmaThreads, 1) residue_mma_kernel(const __gri
     }
     asm volatile("tcgen05.fence::before_thread_sync;");
     __syncthreads();
-    if (warp == 0) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, 512;" :: "r"(tmem));
+    if (warp == 0) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" :: "r"(tmem), "r"(kMmaTmem));
 }
 
 // Plans a product on the GPU from its line analysis (the rule of the host driver): the residue engine
@@ -570,12 +584,12 @@ template <int N> __global__ void __launch_bounds__(128) reconstruct_kernel(RecPa
 // (shifted) bytes, uploaded once per modulus count already in the 128-byte-swizzled K-major layout
 // of shared memory.  Each P[b] is below 2L * 255^2 < 2^25, so the int32 accumulators are exact.  One
 // CTA computes 128 outputs per tile and is persistent over the tiles:
-//   - eight warps build the rows of A from the residues (r -> t = r w_l mod m_l), warps q and q + 4
-//     taking alternate groups of 16 moduli of the same rows;
+//   - eight warps copy the rows of A from the t_l that the residue products stored, two moduli a shared store,
+//     warps q and q + 4 taking alternate groups of 16 moduli of the same rows;
 //   - one thread issues tcgen05.mma kind::i8 (u8 x u8 -> s32, M = 128, N <= 256 per instruction)
 //     into TMEM;
-//   - each thread of warps 0-3 reads its TMEM lane and carries the byte columns into S and F, which
-//     go to memory for crt_round_kernel (or are rounded here with crt_tail).
+//   - warps q and q + 4 read the same TMEM lanes and carry the byte columns of the lower and of the upper words into
+//     S and F, which go to memory for crt_round_kernel; the lower words' last carry goes to a word of its own.
 struct CrtParams {
     const u16* res; const ResTables* tab; const unsigned char* bimg;
     int L, qwords, NB, Kp, NS;             // B rows (multiple of 16), K bytes (multiple of 32), S byte columns
@@ -585,9 +599,16 @@ struct CrtParams {
     int subtract, lower;
     u32* error;
     const ResPlan* plan;                   // planned on the GPU: L and its operand come from the plan
-    u32* sf;                               // not null: S (qwords + 2 words) and F (2 words) go here, word-major
-                                           // (word w of output o at sf[w * M * Nc + o]), and crt_round_kernel rounds
+    u32* sf;                               // S (qwords + 2 words), F (2 words) and the carry into word crt_split_word of
+                                           // S, word-major (word w of output o at sf[w * M * Nc + o])
 };
+constexpr int kCrtExtraWords = 5;          // words of an output in sf beyond qwords
+// S words below this one are carried by warps 0-3, the others by warps 4-7: whole 32-column chunks, the larger part below
+// (the chunk with F and the last words costs more).
+__host__ __device__ __forceinline__ int crt_split_word(int qwords) {
+    const int chunks = qwords / 8;
+    return 8 * (chunks < 2 ? chunks : (chunks + 2) / 2);
+}
 __device__ __forceinline__ void mma_i8_u(u32 d_tmem, u64 a, u64 b, u32 idesc, bool accumulate) {
     asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
                  "tcgen05.mma.cta_group::1.kind::i8 [%0], %1, %2, %3, {%5, %5, %5, %5}, p;\n\t}"
@@ -615,17 +636,12 @@ template <int N> __global__ void __launch_bounds__(kCrtThreads, 2) crt_mma_kerne
     unsigned char* sB = smem + kblocks * 16384;                // kblocks x [NB rows][128 B]
     __shared__ __align__(8) u64 done;
     __shared__ u32 tmem_slot;
-    __shared__ u32 s_m[kResMaxModuli], s_w[kResMaxModuli], s_r[kResMaxModuli];   // m_l, (M/m_l)^-1, floor(2^32/m_l)
-    __shared__ unsigned char s_any[2][128];                    // some residue of the row is nonzero, per half
     const int warp = threadIdx.x >> 5;
     const u64 bbytes = (u64)kblocks * p.NB * 128;
     for (u64 o = (u64)threadIdx.x * 16; o < bbytes; o += (u64)blockDim.x * 16)
         *reinterpret_cast<uint4*>(sB + o) = *reinterpret_cast<const uint4*>(p.bimg + o);
-    for (int l = threadIdx.x; l < p.L; l += blockDim.x) {
-        s_m[l] = p.tab->m[l];
-        s_w[l] = p.tab->w[l];
-        s_r[l] = (u32)(p.tab->barrett[l] >> 32);               // floor(2^64 / m) >> 32 = floor(2^32 / m)
-    }
+    for (u32 o = threadIdx.x * 16u; o < (u32)kblocks * 16384u; o += blockDim.x * 16u)      // bytes beyond 2 L stay zero
+        *reinterpret_cast<uint4*>(sA + o) = make_uint4(0, 0, 0, 0);
     if (threadIdx.x == 0) {
         mbar_init(&done, 1);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -655,27 +671,19 @@ template <int N> __global__ void __launch_bounds__(kCrtThreads, 2) crt_mma_kerne
         }
         const u64 o = tile * 128 + row;
         const bool valid = o < outputs;
-        bool any = false;
+        const u16* src = p.res + o;
         for (int l0 = half * 16; l0 < p.L; l0 += 32) {          // row of A: t_l as two bytes; 16 loads in flight
-            u32 r[16];
+            u32 t[16];
 #pragma unroll
-            for (int q = 0; q < 16; ++q) r[q] = (valid && l0 + q < p.L) ? p.res[(u64)(l0 + q) * outputs + o] : 0u;
+            for (int q = 0; q < 16; ++q) t[q] = (valid && l0 + q < p.L) ? __ldg(src + (u64)(l0 + q) * outputs) : 0u;
+            unsigned char* base = sA + (l0 >> 6) * 16384u;
+            const u32 k0 = 2u * (l0 & 63);
 #pragma unroll
-            for (int q = 0; q < 16; ++q) {
-                const int l = l0 + q;
-                if (l >= p.L) break;
-                any |= r[q] != 0;
-                // t = r w mod m: r < m and w < m, so r w < 2^32 and one 32-bit Barrett step leaves [0, 2m)
-                const u32 m = s_m[l], x = r[q] * s_w[l];
-                u32 t = x - __umulhi(x, s_r[l]) * m;
-                if (t >= m) t -= m;
-                const u32 k = 2u * l;
-                *reinterpret_cast<u16*>(sA + (k >> 7) * 16384u + sw128_offset(row, k & 127u)) = (u16)t;
+            for (int q = 0; q < 16; q += 2) {
+                if (l0 + q >= p.L) break;
+                *reinterpret_cast<u32*>(base + sw128_offset(row, k0 + 2u * q)) = t[q] | (t[q + 1] << 16);
             }
         }
-        for (u32 k = 2u * p.L + 2u * half; k < (u32)kblocks * 128u; k += 4)
-            *reinterpret_cast<u16*>(sA + (k >> 7) * 16384u + sw128_offset(row, k & 127u)) = 0;
-        s_any[half][row] = any ? 1 : 0;
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");   // generic writes -> tensor core reads
         __syncthreads();
         if (threadIdx.x == 0) {
@@ -694,13 +702,28 @@ template <int N> __global__ void __launch_bounds__(kCrtThreads, 2) crt_mma_kerne
         phase ^= 1u;
         asm volatile("tcgen05.fence::after_thread_sync;");
         if (!fine) break;
-        any = (s_any[0][row] | s_any[1][row]) != 0;
-        // S and F from the byte columns of this row (every thread of warps 0-3 reads its lane: .sync.aligned)
-        if (half == 0 && p.sf) {                                // S and F to global memory, word-major
-            int sw = 0;
-            u64 acc = 0, F = 0;
-            u32* dst = p.sf + o;
-            for (int c0 = 0; c0 < p.NB; c0 += 32) {
+        // word w of S is the sum of its four byte columns and the carry from below (every thread of the warp reads its lane:
+        // .sync.aligned); each column is below 2^25, so a word's sum stays below 2^50
+        const int split = crt_split_word(p.qwords), chunks = p.qwords / 8;     // 8-word chunks wholly inside S
+        u32* dst = p.sf + o;
+        u64 acc = 0;
+        for (int ch = half ? split / 8 : 0; ch < (half ? chunks : split / 8); ++ch) {
+            u32 P[32];
+            tmem_ld32(tmem + lane_base + (u32)ch * 32u, P);
+            asm volatile("tcgen05.wait::ld.sync.aligned;");
+#pragma unroll
+            for (int w = 0; w < 8; ++w) {
+                acc += ((u64)P[4 * w + 1] << 8) + P[4 * w] + (((u64)P[4 * w + 3] << 24) + ((u64)P[4 * w + 2] << 16));
+                if (valid) dst[(u64)(8 * ch + w) * outputs] = (u32)acc;
+                acc >>= 32;
+            }
+        }
+        if (half == 0) {
+            if (valid) dst[(u64)(p.qwords + 4) * outputs] = (u32)acc;
+        } else {
+            int sw = 8 * chunks;
+            u64 F = 0;
+            for (int c0 = 4 * sw; c0 < p.NB; c0 += 32) {
                 u32 P[32];
                 tmem_ld32(tmem + lane_base + (u32)c0, P);
                 asm volatile("tcgen05.wait::ld.sync.aligned;");
@@ -720,42 +743,6 @@ template <int N> __global__ void __launch_bounds__(kCrtThreads, 2) crt_mma_kerne
                 dst[(u64)(p.qwords + 2) * outputs] = (u32)F;
                 dst[(u64)(p.qwords + 3) * outputs] = (u32)(F >> 32);
             }
-        } else if (half == 0) {                                 // S and F in registers, rounded here
-        u32 S[kResMaxQWords + 2];
-        int sw = 0;
-        u64 acc = 0, F = 0;
-        for (int c0 = 0; c0 < p.NB; c0 += 32) {
-            u32 P[32];
-            tmem_ld32(tmem + lane_base + (u32)c0, P);
-            asm volatile("tcgen05.wait::ld.sync.aligned;");
-#pragma unroll
-            for (int c = 0; c < 32; ++c) {
-                const int col = c0 + c;
-                if (col < p.NS) {
-                    acc += (u64)P[c] << (8 * (col & 3));
-                    if ((col & 3) == 3) { S[sw++] = (u32)acc; acc >>= 32; }
-                } else if (col < p.NS + 6) {
-                    F += (u64)P[c] << (8 * (col - p.NS));
-                }
-            }
-        }
-        while (sw < p.qwords + 2) { S[sw++] = (u32)acc; acc >>= 32; }
-        if (valid) {
-            const u64 i = o / p.Nc, j = o % p.Nc;
-            if (!(p.lower && j > i)) {
-                constexpr u64 E = N + 3;
-                u32* out = p.C + (i * p.ldc + j) * E;
-                const Num<N> c = p.subtract ? load_plain<N>(out) : zero<N>();
-                const LineInfo li = p.linfo[i], ri = p.rinfo[j];
-                const u32 st = (p.subtract ? c.st : 0u) | li.status | ri.status;
-                if (st) store<N>(out, zero<N>(st));
-                else if (!li.nonzero || !ri.nonzero || !any) store<N>(out, p.subtract ? c : zero<N>());
-                else {
-                    u32 scratch[round_sum2_words<N>(kResMaxQWords + 2)];
-                    store<N>(out, crt_tail<N>(S, p.qwords, F, p.tab, (i64)li.bottom + ri.bottom - 2 * (32 * N - 1), p.subtract != 0, c, scratch));
-                }
-            }
-        }
         }
         asm volatile("tcgen05.fence::before_thread_sync;");
         __syncthreads();                                        // TMEM and A are free for the next tile
@@ -766,51 +753,60 @@ template <int N> __global__ void __launch_bounds__(kCrtThreads, 2) crt_mma_kerne
 }
 
 // ---------------------------------------------------------------- 1b. digit planes on the tensor cores
-// X mod m_l for all L moduli as one unsigned int8 GEMM: with x_b the bytes of X (4 xwords of them) and
-// T_l[b] = 2^(8b) mod m_l = 256 th + tl, the columns 2l, 2l+1 of P = [x bytes] x [tl; th] give
-// X == P_2l + 256 P_2l+1 (mod m_l), each P below 160 * 255^2 < 2^24.  Rows are the padded entries
-// (line, k) in plane order, 128 per tile; B is the constant [2L][4 xwords] byte table, uploaded per
-// (L, xwords) as its swizzled shared-memory image.  The epilogue reduces, negates for negative
-// entries, balances and splits each residue into the two int8 digits, and writes them to the planes
-// (consecutive rows are consecutive plane bytes).
+// X mod m_l for all L moduli as two unsigned int8 GEMMs: with x_b the bytes of X (4 xwords of them) and
+// 2^(8b) mod m_l = 256 th + tl, P0 = [tl] x [x bytes] and P1 = [th] x [x bytes] give
+// X == P0 + 256 P1 (mod m_l), each P below 160 * 255^2 < 2^24.  The moduli are the rows (TMEM lanes) and 128 padded
+// entries (line, k) in plane order the columns: a thread then has its modulus in registers and 32 consecutive entries
+// of one plane, whose digits it packs and stores as 32 bytes.  With entries as rows every digit was a store of
+// its own byte and every residue two shared loads of its modulus (0.21 ms for 1024^2 512-bit entries).  Up to 64 (32)
+// moduli the table's rows repeat two (four) times down the lanes, and each copy takes its share of the columns.
+// B is the constant byte table, uploaded per (L, xwords) as its swizzled shared-memory image.  The epilogue reduces,
+// balances, negates for negative entries and splits each residue into the two int8 digits.
 struct DigitMmaParams {
     LineView v; u64 lines, K, Kp, rows_pad; int L; int xwords;
     const LineInfo* info; const ResTables* tab;
-    const unsigned char* bimg; int NB, KB; u32 tmem_cols;
+    const unsigned char* bimg; int KB;
     signed char* d1; signed char* d0;
     u32* error;
     const ResPlan* plan;                   // planned on the GPU: L and its operand come from the plan
 };
-template <int N> __global__ void __launch_bounds__(kDigitThreads, 1) digits_mma_kernel(const DigitMmaParams pin) {
+constexpr int kDigitCols = 128;                                // entries per tile
+__host__ __device__ constexpr int digit_row_tiles(int L) { return L > 128 ? 2 : 1; }
+__host__ __device__ constexpr int digit_copies(int L) { return L <= 32 ? 4 : L <= 64 ? 2 : 1; }
+__host__ __device__ constexpr u32 digit_tmem_cols(int L) { return 2u * kDigitCols * digit_row_tiles(L); }
+__host__ __device__ constexpr size_t digit_smem_bytes(int row_tiles, int KB) {
+    return 1024 + (size_t)(2 * row_tiles + 1) * ((KB + 127) / 128) * 16384;
+}
+__device__ __forceinline__ void store_bytes32(signed char* p, const u32 (&w)[8]) {
+    asm volatile("st.global.v8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" :: "l"(p), "r"(w[0]), "r"(w[1]), "r"(w[2]), "r"(w[3]),
+                 "r"(w[4]), "r"(w[5]), "r"(w[6]), "r"(w[7]) : "memory");
+}
+template <int N> __global__ void __launch_bounds__(kDigitThreads, 2) digits_mma_kernel(const DigitMmaParams pin) {
     DigitMmaParams p = pin;
     if (pin.plan) {
         const ResPlan& r = *pin.plan;
         if (r.mode != 1) return;
-        p.tab = static_cast<const ResTables*>(r.tab); p.bimg = r.dig_bimg; p.L = r.L; p.NB = r.dNB; p.tmem_cols = r.dtmem;
+        p.tab = static_cast<const ResTables*>(r.tab); p.bimg = r.dig_bimg; p.L = r.L;
     }
     extern __shared__ __align__(1024) unsigned char dig_raw[];
     unsigned char* smem = (unsigned char*)(((uintptr_t)dig_raw + 1023) & ~(uintptr_t)1023);
-    const int kblocks = p.KB / 128 + (p.KB % 128 ? 1 : 0);
-    unsigned char* sA = smem;
-    unsigned char* sB = smem + kblocks * 16384;
+    const int kblocks = p.KB / 128 + (p.KB % 128 ? 1 : 0), row_tiles = digit_row_tiles(p.L);
+    unsigned char* sX = smem;                                  // kblocks x [128 entries][128 B]
+    unsigned char* sT = smem + kblocks * 16384;                // row tiles x (tl, th) x kblocks x [128 moduli][128 B]
     __shared__ __align__(8) u64 done;
     __shared__ u32 tmem_slot;
-    __shared__ u32 s_m[kResMaxModuli], s_r[kResMaxModuli];     // m_l and floor(2^32 / m_l)
-    __shared__ unsigned char s_neg[128];                       // row holds a negative entry
-    const int warp = threadIdx.x >> 5;
-    const u64 bbytes = (u64)kblocks * p.NB * 128;
-    for (u64 o = (u64)threadIdx.x * 16; o < bbytes; o += (u64)blockDim.x * 16)
-        *reinterpret_cast<uint4*>(sB + o) = *reinterpret_cast<const uint4*>(p.bimg + o);
-    for (int l = threadIdx.x; l < p.L; l += blockDim.x) {
-        s_m[l] = p.tab->m[l];
-        s_r[l] = (u32)(p.tab->barrett[l] >> 32);               // floor(2^64 / m) >> 32 = floor(2^32 / m)
-    }
+    __shared__ u32 s_neg[kDigitCols / 32];                     // negative entries of the tile, one bit each
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const u32 tbytes = 2u * row_tiles * kblocks * 16384u;
+    for (u32 o = threadIdx.x * 16u; o < tbytes; o += blockDim.x * 16u)
+        *reinterpret_cast<uint4*>(sT + o) = *reinterpret_cast<const uint4*>(p.bimg + o);
     if (threadIdx.x == 0) {
         mbar_init(&done, 1);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
+    const u32 tmem_cols = digit_tmem_cols(p.L);
     if (warp == 0) {
-        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" :: "r"(smem_u32(&tmem_slot)), "r"(p.tmem_cols));
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" :: "r"(smem_u32(&tmem_slot)), "r"(tmem_cols));
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
     }
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
@@ -818,19 +814,20 @@ template <int N> __global__ void __launch_bounds__(kDigitThreads, 1) digits_mma_
     __syncthreads();
     asm volatile("tcgen05.fence::after_thread_sync;");
     const u32 tmem = tmem_slot;
-    const int N1 = p.NB < 256 ? p.NB : 256, N2 = p.NB - N1;
-    const u32 id1 = (2u << 4) | ((u32)(N1 >> 3) << 17) | ((u32)(128 >> 4) << 24);
-    const u32 id2 = (2u << 4) | ((u32)(N2 >> 3) << 17) | ((u32)(128 >> 4) << 24);
-    const u64 plane = p.rows_pad * p.Kp, tiles = plane / 128;     // Kp is a multiple of 128
+    constexpr u32 idesc = (2u << 4) | ((u32)(kDigitCols >> 3) << 17) | ((u32)(128 >> 4) << 24);
+    const u64 plane = p.rows_pad * p.Kp, tiles = plane / kDigitCols;      // rows_pad is a multiple of 128
     const int q = warp & 3, half = warp >> 2;                  // warps q and q + 4 share TMEM lanes 32 q ..
-    const u32 row = (u32)(q * 32 + (threadIdx.x & 31)), lane_base = (u32)(q * 32) << 16;
-    // The first four warps stage the entries of a tile (one row each); the entry of the next tile is
+    const u32 lane_base = (u32)(q * 32) << 16;
+    const int copies = digit_copies(p.L), rows = 128 / copies, span = kDigitCols / copies;
+    const int group = (q * 32) / rows;                         // the copy of the table this warp's lanes belong to
+    // The first four warps stage the entries of a tile (one each a thread); the entry of the next tile is
     // loaded before the current tile's epilogue so that its latency hides behind the digit work.
+    const u32 entry = (u32)(q * 32 + lane);
     Num<N> a = zero<N>();
     u64 aline = 0;
     auto fetch = [&](u64 t) {
         a = zero<N>();
-        const u64 e = t * 128 + row;
+        const u64 e = t * kDigitCols + entry;
         aline = e / p.Kp;
         const u64 k = e % p.Kp;
         if (t < tiles && k < p.K && aline < p.lines) a = load<N>(p.v.base + (aline * p.v.ls + k * p.v.ks) * (u64)(N + 3));
@@ -838,13 +835,12 @@ template <int N> __global__ void __launch_bounds__(kDigitThreads, 1) digits_mma_
     if (half == 0) fetch(blockIdx.x);
     u32 phase = 0;
     for (u64 tile = blockIdx.x; tile < tiles; tile += gridDim.x) {
-        const u64 e = tile * 128 + row;
         if (half == 0) {
-            // row of A: the bytes of X = |entry| 2^(e - bottom) (0 <= shift <= G), zero beyond its words
+            // column of B: the bytes of X = |entry| 2^(e - bottom) (0 <= shift <= G), zero beyond its words
 #pragma unroll
             for (int c = 0; c < 16; ++c) {                      // up to 2 K blocks of 8 chunks
                 if (c >= kblocks * 8) break;
-                *reinterpret_cast<uint4*>(sA + (c >> 3) * 16384u + sw128_offset(row, (u32)(c & 7) * 16u)) = make_uint4(0, 0, 0, 0);
+                *reinterpret_cast<uint4*>(sX + (c >> 3) * 16384u + sw128_offset(entry, (u32)(c & 7) * 16u)) = make_uint4(0, 0, 0, 0);
             }
             bool negative = false;
             if (!a.st && a.s) {
@@ -856,52 +852,63 @@ template <int N> __global__ void __launch_bounds__(kDigitThreads, 1) digits_mma_
                     u32 v = i < N ? a.m[i] << bs : 0u;
                     if (bs && i > 0) v |= a.m[i - 1] >> (32 - bs);
                     const u32 byte = (u32)(i + ws) * 4u;      // word i + ws < xwords <= KB / 4
-                    *reinterpret_cast<u32*>(sA + (byte >> 7) * 16384u + sw128_offset(row, byte & 127u)) = v;
+                    *reinterpret_cast<u32*>(sX + (byte >> 7) * 16384u + sw128_offset(entry, byte & 127u)) = v;
                 }
             }
-            s_neg[row] = negative ? 1 : 0;
+            const u32 neg = __ballot_sync(0xffffffffu, negative);
+            if (lane == 0) s_neg[q] = neg;
         }
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
         __syncthreads();
         if (threadIdx.x == 0) {
             asm volatile("tcgen05.fence::after_thread_sync;");
-            for (int ks = 0; ks < p.KB / 32; ++ks) {
-                const int kb = ks >> 2;
-                const u64 koff = (u64)((ks & 3) * 32) >> 4;
-                const u64 ad = crt_desc(smem_u32(sA + kb * 16384)) + koff;
-                const u32 bbase = smem_u32(sB + (u64)kb * p.NB * 128);
-                mma_i8_u(tmem, ad, crt_desc(bbase) + koff, id1, ks > 0);
-                if (N2) mma_i8_u(tmem + 256, ad, crt_desc(bbase + 256 * 128) + koff, id2, ks > 0);
-            }
+            for (int g = 0; g < 2 * row_tiles; ++g)
+                for (int ks = 0; ks < p.KB / 32; ++ks) {
+                    const u64 koff = (u64)((ks & 3) * 32) >> 4;
+                    mma_i8_u(tmem + (u32)(g * kDigitCols), crt_desc(smem_u32(sT + (g * kblocks + (ks >> 2)) * 16384)) + koff,
+                             crt_desc(smem_u32(sX + (ks >> 2) * 16384)) + koff, idesc, ks > 0);
+                }
             mma_commit(&done);
         }
         const bool fine = __syncthreads_and(mbar_wait(&done, phase, p.error));
         phase ^= 1u;
         asm volatile("tcgen05.fence::after_thread_sync;");
         if (!fine) break;
-        if (half == 0) fetch(tile + gridDim.x);                // sA is rewritten only after the barrier below
-        const bool negative = s_neg[row] != 0;
-        signed char* d1 = p.d1 + e;
-        signed char* d0 = p.d0 + e;
-        // X == P_2l + 256 P_2l+1 (mod m_l) with both P below 160 * 255^2, so the sum stays below 2^32 and one
-        // 32-bit Barrett step with floor(2^32 / m) leaves it in [0, 2m).
-        for (int c0 = half * 32; c0 < 2 * p.L; c0 += 64) {
-            u32 P[32];
-            tmem_ld32(tmem + lane_base + (u32)c0, P);
-            asm volatile("tcgen05.wait::ld.sync.aligned;");
+        if (half == 0) fetch(tile + gridDim.x);                // sX is rewritten only after the barrier below
+        for (int t = 0; t < row_tiles; ++t) {
+            const int l = t * 128 + (int)entry - group * rows;
+            const bool live = l < p.L;
+            const u32 m = live ? p.tab->m[l] : 3u, rr = live ? (u32)(p.tab->barrett[l] >> 32) : 0u, h = m >> 1;
+            const u64 at = (u64)(live ? l : 0) * plane + tile * kDigitCols;
+            for (int ch = half; ch < span / 32; ch += 2) {
+                const u32 c0 = (u32)(group * span + ch * 32);
+                u32 P0[32], P1[32];
+                tmem_ld32(tmem + lane_base + (u32)(2 * t * kDigitCols) + c0, P0);
+                tmem_ld32(tmem + lane_base + (u32)((2 * t + 1) * kDigitCols) + c0, P1);
+                asm volatile("tcgen05.wait::ld.sync.aligned;");
+                if (live) {
+                    const u32 neg = s_neg[c0 >> 5];
+                    u32 w0[8], w1[8];
 #pragma unroll
-            for (int c = 0; c < 32; c += 2) {
-                const int l = (c0 + c) >> 1;
-                if (l >= p.L) break;
-                const u32 m = s_m[l];
-                const u32 x = P[c] + (P[c + 1] << 8);
-                u32 u = x - __umulhi(x, s_r[l]) * m;
-                if (u >= m) u -= m;
-                if (negative && u) u = m - u;                   // residue of -X
-                const int r = (int)u - (u > (m >> 1) ? (int)m : 0);   // balanced: |r| <= 32639
-                const int lo = (int)(signed char)(r & 0xff);
-                d1[(u64)l * plane] = (signed char)((r - lo) >> 8);
-                d0[(u64)l * plane] = (signed char)lo;
+                    for (int g = 0; g < 8; ++g) {
+                        int r[4];
+#pragma unroll
+                        for (int b = 0; b < 4; ++b) {
+                            const int c = 4 * g + b;
+                            const u32 x = P0[c] + (P1[c] << 8);     // below 2^32: one Barrett step leaves [0, 2m)
+                            u32 u = x - __umulhi(x, rr) * m;
+                            u = min(u, u - m);
+                            const int v = (int)u - (u > h ? (int)m : 0);       // balanced (m is odd): |v| <= 32639
+                            r[b] = (neg >> c) & 1u ? -v : v;
+                        }
+                        // low digit: the byte of r; high digit: (r - low) >> 8 = byte 1 of r + 128
+                        w0[g] = __byte_perm(__byte_perm(r[0], r[1], 0x0040), __byte_perm(r[2], r[3], 0x0040), 0x5410);
+                        w1[g] = __byte_perm(__byte_perm(r[0] + 128, r[1] + 128, 0x0051), __byte_perm(r[2] + 128, r[3] + 128, 0x0051), 0x5410);
+                    }
+                    store_bytes32(p.d1 + at + c0, w1);
+                    store_bytes32(p.d0 + at + c0, w0);
+                }
+                __syncwarp();
             }
         }
         asm volatile("tcgen05.fence::before_thread_sync;");
@@ -909,17 +916,23 @@ template <int N> __global__ void __launch_bounds__(kDigitThreads, 1) digits_mma_
     }
     asm volatile("tcgen05.fence::before_thread_sync;");
     __syncthreads();
-    if (warp == 0) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" :: "r"(tmem), "r"(p.tmem_cols));
+    if (warp == 0) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" :: "r"(tmem), "r"(tmem_cols));
 }
 
-// The rounding half of the CRT when crt_mma_kernel wrote S and F: one thread per output.  Each thread's S and
-// rounding window live in shared memory (crt_round_words words per thread, an odd stride so that the 32 lanes of a
-// warp touching the same word index hit 32 banks), so the data-dependent word indexing of crt_tail costs no local-
-// memory traffic to L2 and DRAM.  An output whose residues were all zero has S = F = 0, which crt_tail turns into
-// c itself (or zero), as the fused path does.
-constexpr int kCrtRoundThreads = 64;
-template <int N> __host__ __device__ constexpr int crt_round_words(int qwords) {
-    return ((qwords + 2) + round_sum2_words<N>(qwords + 2)) | 1;
+// The rounding half of the CRT: one thread per output, RN(c - X 2^scale) or RN(X 2^scale) with X = S - round(F) M.
+// One pass over the words subtracts q M and adds the old entry in place (T = X - c at X's scale, negated when it is rounded),
+// leaving T's words in shared memory (an odd stride: the lanes of a warp touch 32 banks); the rounding reads the N + 2 words
+// under T's top and learns the sticky bit from the lowest nonzero word, which the pass recorded.  That needs the old
+// entry's bits to lie inside X's words; an entry that reaches outside takes the two-window form (crt_tail, in thread-
+// local memory).  The two-window form for every output took 0.32 ms for 1024^2 outputs at 512 bits, four passes over
+// 82-word windows.
+constexpr int kCrtRoundThreads = 128;
+__host__ __device__ constexpr int crt_round_words(int qwords) { return (qwords + 2) | 1; }
+template <int N> __device__ __noinline__ Num<N> crt_tail_call(const u32* S, int qwords, u64 F, const ResTables* tab, i64 scale,
+                                                              bool subtract, const Num<N> c) {
+    u32 X[kResMaxQWords + 2], scratch[round_sum2_words<N>(kResMaxQWords + 2)];
+    for (int w = 0; w < qwords + 2; ++w) X[w] = S[w];
+    return crt_tail<N>(X, qwords, F, tab, scale, subtract, c, scratch);
 }
 template <int N> __global__ void __launch_bounds__(kCrtRoundThreads) crt_round_kernel(const CrtParams pin) {
     CrtParams p = pin;
@@ -928,21 +941,86 @@ template <int N> __global__ void __launch_bounds__(kCrtRoundThreads) crt_round_k
         p.tab = static_cast<const ResTables*>(pin.plan->tab); p.qwords = pin.plan->qwords;
     }
     extern __shared__ u32 crt_round_park[];
+    __shared__ u32 s_M[kResMaxQWords + 2];
+    const int xw = p.qwords + 2;
+    for (int w = threadIdx.x; w < xw; w += kCrtRoundThreads) s_M[w] = w <= p.qwords ? p.tab->M[w] : 0u;
+    __syncthreads();
     const u64 outputs = p.M * p.Nc, o = (u64)blockIdx.x * kCrtRoundThreads + threadIdx.x;
     if (o >= outputs) return;
     const u64 i = o / p.Nc, j = o % p.Nc;
     if (p.lower && j > i) return;
     constexpr u64 E = N + 3;
     u32* out = p.C + (i * p.ldc + j) * E;
-    const Num<N> c = p.subtract ? load_plain<N>(out) : zero<N>();
     const LineInfo li = p.linfo[i], ri = p.rinfo[j];
-    const u32 st = (p.subtract ? c.st : 0u) | li.status | ri.status;
+    int ce = 0, cs = 0;
+    u32 cst = 0;
+    if (p.subtract) { ce = (int)out[N]; cs = (int)out[N + 1]; cst = out[N + 2]; }
+    const u32 st = cst | li.status | ri.status;
     if (st) { store<N>(out, zero<N>(st)); return; }
-    if (!li.nonzero || !ri.nonzero) { store<N>(out, p.subtract ? c : zero<N>()); return; }
-    u32* S = crt_round_park + threadIdx.x * crt_round_words<N>(p.qwords);
-    for (int w = 0; w < p.qwords + 2; ++w) S[w] = p.sf[(u64)w * outputs + o];
-    const u64 F = (u64)p.sf[(u64)(p.qwords + 2) * outputs + o] | ((u64)p.sf[(u64)(p.qwords + 3) * outputs + o] << 32);
-    store<N>(out, crt_tail<N>(S, p.qwords, F, p.tab, (i64)li.bottom + ri.bottom - 2 * (32 * N - 1), p.subtract != 0, c, S + p.qwords + 2));
+    if (!li.nonzero || !ri.nonzero) { if (!p.subtract) store<N>(out, zero<N>()); return; }      // C stays
+    u32* T = crt_round_park + threadIdx.x * crt_round_words(p.qwords);
+    const u32* sf = p.sf + o;
+    const u64 F = (u64)sf[(u64)(p.qwords + 2) * outputs] | ((u64)sf[(u64)(p.qwords + 3) * outputs] << 32);
+    const int split = crt_split_word(p.qwords);
+    const u32 up = sf[(u64)(p.qwords + 4) * outputs];            // carry of the lower words' columns
+    const i64 scale = (i64)li.bottom + ri.bottom - 2 * (32 * N - 1);
+    const i64 off = (i64)ce - (32 * N - 1) - scale;              // bit of T that the old entry's lowest bit falls on
+    if (cs && (off < 0 || off + 32 * N > 32 * (i64)xw - 2)) {
+        u64 cy = 0;
+        for (int w = 0; w < xw; ++w) {
+            const u64 v = (u64)sf[(u64)w * outputs] + (w == split ? up : 0u) + cy;
+            T[w] = (u32)v; cy = v >> 32;
+        }
+        store<N>(out, crt_tail_call<N>(T, p.qwords, F, p.tab, scale, true, load_plain<N>(out)));
+        return;
+    }
+    // T = S - q M - c (two's complement); without an old entry T = X
+    const u32 q = (u32)((F + (1ull << 47)) >> 48);              // round(F) <= L: X = S - q M
+    const int ws = cs ? (int)(off >> 5) : xw, bs = cs ? (int)(off & 31) : 0;
+    const u32 mask = cs > 0 ? 0xffffffffu : 0u;                   // c > 0 is subtracted
+    u64 cy = 0, qm = 0, ca = mask & 1u;
+    u32 prev = 0, low = 0xffffffffu;                              // lowest nonzero word of T
+    int borrow = 0;
+    for (int w = 0; w < xw; ++w) {
+        const u64 sv = (u64)sf[(u64)w * outputs] + (w == split ? up : 0u) + cy;
+        cy = sv >> 32;
+        qm += (u64)s_M[w] * q;
+        const i64 d = (i64)(sv & 0xffffffffull) - (i64)(qm & 0xffffffffull) - borrow;
+        qm >>= 32;
+        borrow = d < 0;
+        u32 cur = 0, add = 0;
+        const int k = w - ws;
+        if (k >= 0 && k <= N) {
+            if (k < N) cur = out[k];
+            add = __funnelshift_l(prev, cur, bs);
+            prev = cur;
+        }
+        const u64 v = (u64)(u32)d + (add ^ mask) + ca;
+        ca = v >> 32;
+        T[w] = (u32)v;
+        if ((u32)v && low == 0xffffffffu) low = (u32)w;
+    }
+    if (low == 0xffffffffu) { store<N>(out, zero<N>()); return; }
+    const bool neg = T[xw - 1] >> 31;
+    auto mag = [&](int w) -> u32 {                                // word w of |T|
+        if (w < (int)low) return 0u;
+        return neg ? (w == (int)low ? 0u - T[w] : ~T[w]) : T[w];
+    };
+    int t = xw - 1;
+    while (!mag(t)) --t;
+    u32 hi = mag(t);
+    const int lz = __clz(hi);
+    u32 m[N];
+#pragma unroll
+    for (int x = N - 1; x >= 0; --x) {
+        const u32 below = mag(t - N + x);
+        m[x] = __funnelshift_l(below, hi, lz);
+        hi = below;
+    }
+    const u32 next = mag(t - N - 1), g = __funnelshift_l(next, hi, lz);
+    const bool sticky = (g & 0x7fffffffu) || (next << lz) || (int)low < t - N - 1;
+    // subtract: the result is c - X = -T
+    store<N>(out, finish<N>(m, scale + 32 * (i64)t + 31 - lz, neg != (p.subtract != 0) ? -1 : 1, (g >> 31) && (sticky || (m[0] & 1u)), 0));
 }
 
 typedef void (*DigitFn)(const DigitParams&, cudaStream_t);
@@ -962,13 +1040,10 @@ template <int N> void crt_launch(const CrtParams& p, unsigned grid, size_t smem,
     if (!p.M || !p.Nc) return;
     cudaFuncSetAttribute(crt_mma_kernel<N>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     crt_mma_kernel<N><<<grid, kCrtThreads, smem, s>>>(p);
-    if (p.sf) {
-        // the planned form learns qwords on the GPU: size the rounding scratch for the largest table
-        const int qw = p.plan ? kResMaxQWords : p.qwords;
-        const size_t rsmem = (size_t)kCrtRoundThreads * crt_round_words<N>(qw) * 4;
-        if (rsmem > 48 * 1024) cudaFuncSetAttribute(crt_round_kernel<N>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)rsmem);
-        crt_round_kernel<N><<<(unsigned)((p.M * p.Nc + kCrtRoundThreads - 1) / kCrtRoundThreads), kCrtRoundThreads, rsmem, s>>>(p);
-    }
+    // the planned form learns qwords on the GPU: size the words of T for the largest table
+    const size_t rsmem = (size_t)kCrtRoundThreads * crt_round_words(p.plan ? kResMaxQWords : p.qwords) * 4;
+    if (rsmem > 48 * 1024) cudaFuncSetAttribute(crt_round_kernel<N>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)rsmem);
+    crt_round_kernel<N><<<(unsigned)((p.M * p.Nc + kCrtRoundThreads - 1) / kCrtRoundThreads), kCrtRoundThreads, rsmem, s>>>(p);
 }
 template <int N> void digits_mma_launch(const DigitMmaParams& p, unsigned grid, size_t smem, cudaStream_t s) {
     if (!p.rows_pad || !p.Kp) return;

@@ -26,8 +26,8 @@ int residue_moduli_for(int bits, int G, uint64_t K);      // modulus count L, 0 
 int residue_max_band();
 uint64_t residue_max_k();
 void residue_tables_host(int L, lfd::ResTables& tables, int& qwords);
-CUtensorMap residue_plane_map(void* base, uint64_t Kp, uint64_t rows_pad, int L);
-void residue_mma_launch(dim3 grid, const CUtensorMap& ta1, const CUtensorMap& ta0, const CUtensorMap& tb1, const CUtensorMap& tb0,
+CUtensorMap residue_plane_map(void* base, uint64_t Kp, uint64_t rows_pad, int L, bool left);     // boxes of a left or right tile
+void residue_mma_launch(const CUtensorMap& ta1, const CUtensorMap& ta0, const CUtensorMap& tb1, const CUtensorMap& tb0, int moduli,
                         const lfd::MmaParams& p, cudaStream_t s);
 }  // namespace lfr
 
