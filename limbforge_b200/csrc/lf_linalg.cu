@@ -59,7 +59,8 @@ static ProductLane side_lane(Linalg& la) {
 
 // C (M x Nc at ldc) <- RN(C - L R^T) (subtract) or RN(L R^T), L/R given as line views; lower: only j <= i.  On `lane`
 // and stream s; with `check`, the call waits for the product and raises a cluster overflow, otherwise the caller reads
-// the lane's error word later (its word is not cleared here then).
+// the lane's error word later (its word is not cleared here then).  Without `check` these are the products between a
+// factorization's blocks, and short ones take the four-lane kernel.
 void exact_product_on(Linalg& la, const ProductLane& lane, int bits, lfd::LineView left, lfd::LineView right, uint64_t M,
                       uint64_t Nc, uint64_t K, uint32_t* C, uint64_t ldc, bool subtract, bool lower, cudaStream_t s,
                       int* method_used, bool check) {
@@ -68,6 +69,14 @@ void exact_product_on(Linalg& la, const ProductLane& lane, int bits, lfd::LineVi
     uint32_t* err = lane.err;
     if (check) cuda_check(cudaMemsetAsync(err, 0, 4, s), "memset");
     int method = la.options.method;                    // 0 auto, 1 limb kernel, 2 residue engine
+    if (!check && !method && !la.options.force_fallback && lfd::short_product_fits(n, M, Nc, K)) {
+        lfd::DotParams p{};
+        p.left = left; p.right = right; p.C = C; p.ldc = ldc; p.M = M; p.Nc = Nc; p.K = K;
+        p.subtract = subtract; p.lower = lower; p.error = err;
+        lfd::linalg_kernels(n)->short_product(p, s);
+        cuda_check(cudaGetLastError(), "short product launch");
+        return;
+    }
     bool used_residue = false;
     if (method != 1 && !la.options.force_fallback)
         used_residue = lane.residue->run(bits, left, right, M, Nc, K, C, ldc, subtract, lower, err, s, method == 2, la.report);

@@ -148,10 +148,107 @@ template <int N> __global__ void mirror_kernel(u32* C, u64 n, u64 ldc) {
     for (int w = 0; w < (int)E; ++w) dst[w] = src[w];
 }
 
+// exact_dot_add by a group of four lanes, eight outputs a warp: for sums of a few dozen terms, where a warp per output spends
+// itself on the reduction of 32 windows and one rounding.  Each lane sums every fourth term in its window, two exchanges add
+// the windows, and the roundings of the eight groups run side by side.  Every lane of the group returns the result; all lanes
+// of a group call together.
+template <int N, bool RO> __device__ __forceinline__ Num<N> quad_exact_dot(const u32* cp, bool subtract, const u32* x, i64 sx, const u32* y, i64 sy,
+                                                                          u64 K, u32* error) {
+    constexpr int W = 2 * N + 10;
+    constexpr i64 E = N + 3;
+    const int q = threadIdx.x & 3;
+    const u32 group = 0xFu << (threadIdx.x & 28);
+    const Num<N> c = cp ? ldn<N, RO>(cp) : zero<N>();
+    u32 st = 0; int cnt = 0;
+    i64 lo = INT64_MAX, hi = INT64_MIN;
+    for (u64 k = q; k < K; k += 4) {
+        const u32* a = x + (i64)k * sx * E; const u32* b = y + (i64)k * sy * E;
+        st |= ldw<RO>(a + N + 2) | ldw<RO>(b + N + 2);
+        if ((int)ldw<RO>(a + N + 1) && (int)ldw<RO>(b + N + 1)) {
+            const i64 s = (i64)(int)ldw<RO>(a + N) + (int)ldw<RO>(b + N) - 2 * (32 * N - 1);
+            lo = s < lo ? s : lo; hi = s + 64 * N > hi ? s + 64 * N : hi; ++cnt;
+        }
+    }
+#pragma unroll
+    for (int o = 1; o < 4; o <<= 1) {
+        st |= __shfl_xor_sync(group, st, o);
+        cnt += __shfl_xor_sync(group, cnt, o);
+        const i64 l2 = __shfl_xor_sync(group, lo, o), h2 = __shfl_xor_sync(group, hi, o);
+        lo = l2 < lo ? l2 : lo; hi = h2 > hi ? h2 : hi;
+    }
+    st |= c.st;
+    if (st) return zero<N>(st);
+    if (!cnt) return cp ? c : zero<N>();
+    if (c.s) {
+        const i64 sc = (i64)c.e - (32 * N - 1);
+        lo = sc < lo ? sc : lo; hi = (i64)c.e + 1 > hi ? (i64)c.e + 1 : hi;
+    }
+    int logc = 0;
+    while ((1 << logc) < cnt + 2) ++logc;
+    Num<N> r = zero<N>();
+    if (hi - lo + logc + 1 >= 32 * (i64)W) {
+        if (q == 0) r = exact_dot_add_dev<N, RO>(cp, subtract, x, sx, y, sy, K, error);
+        const int first = threadIdx.x & 28;
+#pragma unroll
+        for (int w = 0; w < N; ++w) r.m[w] = __shfl_sync(group, r.m[w], first);
+        r.e = __shfl_sync(group, r.e, first); r.s = __shfl_sync(group, r.s, first); r.st = __shfl_sync(group, r.st, first);
+        return r;
+    }
+    u32 acc[W], t[W];
+#pragma unroll
+    for (int w = 0; w < W; ++w) acc[w] = 0;
+    if (q == 3 && c.s) {                                          // the lane with the fewest terms
+        place_words<W, N>(t, c.m, (i64)c.e - (32 * N - 1) - lo);
+        accumulate<W>(acc, t, c.s < 0);
+    }
+    for (u64 k = q; k < K; k += 4) {
+        const Num<N> a = ldn<N, RO>(x + (i64)k * sx * E), b = ldn<N, RO>(y + (i64)k * sy * E);
+        if (!a.s || !b.s) continue;
+        u32 p[2 * N];
+        mant_mul<N>(a.m, b.m, p);
+        place_words<W, 2 * N>(t, p, (i64)a.e + b.e - 2 * (32 * N - 1) - lo);
+        accumulate<W>(acc, t, (subtract ? -a.s * b.s : a.s * b.s) < 0);
+    }
+    __syncwarp(group);
+#pragma unroll 1
+    for (int o = 1; o < 4; o <<= 1) {
+#pragma unroll
+        for (int w = 0; w < W; ++w) t[w] = __shfl_xor_sync(group, acc[w], o);
+        accumulate<W>(acc, t, false);
+    }
+    const bool neg = acc[W - 1] >> 31;
+#pragma unroll
+    for (int w = 0; w < W; ++w) t[w] = 0;
+    accumulate<W>(t, acc, neg);                                   // the magnitude
+    return round_general<N, W>(t, lo, neg ? -1 : 1, 0);
+}
+
+// Products whose every output sums a few dozen terms, as the factorizations make between their blocks: four lanes an output, no line
+// analysis and so no round trip to the host before the launch.  short_product_fits says where that is the faster way: the
+// residue engine takes some 80 us in latency whatever the size (analysis, host decision, digits, products, CRT,
+// rounding), this kernel outputs (K c + 6000) / 32 warp cycles with c about 4 N^2 + 18 N + 200 for a product and its
+// addition; the line is drawn where that reaches 50 us on the whole chip, and at 64 terms, 16 in sequence a lane.
+constexpr int kShortThreads = 64;
+constexpr u64 kShortMaxK = 64;
+inline bool short_product_fits(int limbs, u64 M, u64 Nc, u64 K) {
+    const double c = 4.0 * limbs * limbs + 18.0 * limbs + 200.0;
+    return K <= kShortMaxK && (double)M * (double)Nc * ((double)K * c + 6000.0) <= 1.86e9;
+}
+template <int N> __global__ void __launch_bounds__(kShortThreads) short_product_kernel(DotParams p) {
+    constexpr u64 E = N + 3;
+    const u64 o = ((u64)blockIdx.x * kShortThreads + threadIdx.x) >> 2, i = o / p.Nc, j = o % p.Nc;
+    if (i >= p.M || (p.lower && j > i)) return;                    // a group of four leaves together
+    u32* out = p.C + (i * p.ldc + j) * E;
+    const Num<N> v = quad_exact_dot<N, true>(p.subtract ? out : nullptr, p.subtract, p.left.base + i * p.left.ls * E, (i64)p.left.ks,
+                                             p.right.base + j * p.right.ls * E, (i64)p.right.ks, p.K, p.error);
+    __syncwarp(0xFu << (threadIdx.x & 28));                        // every lane has read the old entry
+    if ((threadIdx.x & 3) == 0) store<N>(out, v);
+}
+
 typedef void (*AnalyzeFn)(LineView, u64, u64, LineInfo*, cudaStream_t);
 typedef void (*DotFn)(const DotParams&, cudaStream_t);
 typedef void (*MirrorFn)(u32*, u64, u64, cudaStream_t);
-struct LinalgKernels { AnalyzeFn analyze; DotFn dot; MirrorFn mirror; };
+struct LinalgKernels { AnalyzeFn analyze; DotFn dot; MirrorFn mirror; DotFn short_product; };
 const LinalgKernels* linalg_kernels(int limbs);
 
 template <int N> void analyze_launch(LineView v, u64 lines, u64 K, LineInfo* out, cudaStream_t s) {
@@ -163,6 +260,10 @@ template <int N> void dot_launch(const DotParams& p, cudaStream_t s) {
     dim3 block(32, 4), grid((unsigned)((p.Nc + 31) / 32), (unsigned)((p.M + 3) / 4));
     exact_dot_kernel<N><<<grid, block, 0, s>>>(p);
 }
+template <int N> void short_product_launch(const DotParams& p, cudaStream_t s) {
+    if (!p.M || !p.Nc) return;
+    short_product_kernel<N><<<(unsigned)((4 * p.M * p.Nc + kShortThreads - 1) / kShortThreads), kShortThreads, 0, s>>>(p);
+}
 template <int N> void mirror_launch(u32* C, u64 n, u64 ldc, cudaStream_t s) {
     if (n < 2) return;
     dim3 block(32, 4), grid((unsigned)((n + 31) / 32), (unsigned)((n + 3) / 4));
@@ -173,7 +274,7 @@ template <int N> void mirror_launch(u32* C, u64 n, u64 ldc, cudaStream_t s) {
 
 #define LF_LINALG_INSTANTIATE(N)                                                                      \
     namespace lfd {                                                                                   \
-    extern const LinalgKernels linalg_kernels_##N; const LinalgKernels linalg_kernels_##N = {analyze_launch<N>, dot_launch<N>, mirror_launch<N>};    \
+    extern const LinalgKernels linalg_kernels_##N; const LinalgKernels linalg_kernels_##N = {analyze_launch<N>, dot_launch<N>, mirror_launch<N>, short_product_launch<N>}; \
     }
 
 namespace lfd {
@@ -401,6 +502,131 @@ template <int N, bool RO> __device__ __noinline__ Num<N> warp_exact_dot(const u3
     return warp_broadcast<N>(r);
 }
 
+// ---------------------------------------------------------------- running exact sums
+// c - sum x_k y_k of one entry, kept exactly while its terms arrive one at a time: a two's-complement window of 2N + 10
+// words anchored at 2^lo, in a thread's registers.  A column step of a triangular recurrence then costs an entry one product and
+// one addition, and a rounding only when its own turn comes, where forming every entry's dot product afresh (warp_exact_dot)
+// costs a warp-wide reduction and a rounding an entry.  The anchor is a guess made before the terms are known: a term
+// that does not fit the window sets `bad`, and the entry is then formed afresh, so the bits never depend on the guess.
+constexpr u64 kTriBlock = 32;     // widest block of the running-sum kernels: one lane per column
+template <int N> struct RunningSum {
+    static constexpr int W = 2 * N + 10;
+    u32 acc[W];
+    i64 lo;
+    u32 st;
+    bool bad;
+    // Terms and partial sums of up to kTriBlock terms below 2^top fit.
+    __device__ __forceinline__ static i64 anchor(i64 top) { return top + 8 - 32 * (i64)W; }
+    __device__ __forceinline__ void start(const Num<N>& c, i64 anchor_lo) {
+        lo = anchor_lo; st = c.st; bad = false;
+#pragma unroll
+        for (int w = 0; w < W; ++w) acc[w] = 0;
+        if (!c.s) return;
+        const i64 off = (i64)c.e - (32 * N - 1) - lo;
+        if (off < 0 || off > 32 * (W - N) - 8) { bad = true; return; }
+        u32 t[W];
+        place_words<W, N>(t, c.m, off);
+        accumulate<W>(acc, t, c.s < 0);
+    }
+    __device__ __forceinline__ void subtract(const Num<N>& a, const Num<N>& b) {
+        st |= a.st | b.st;
+        if (!a.s || !b.s) return;
+        const i64 off = (i64)a.e + b.e - 2 * (32 * N - 1) - lo;
+        if (off < 0 || off > 32 * (W - 2 * N) - 8) { bad = true; return; }
+        u32 p[2 * N], t[W];
+        mant_mul<N>(a.m, b.m, p);
+        place_words<W, 2 * N>(t, p, off);
+        accumulate<W>(acc, t, a.s * b.s > 0);
+    }
+    __device__ __forceinline__ Num<N> round() const {              // meaningful unless bad
+        if (st) return zero<N>(st);
+        u32 x[W];
+        const bool neg = acc[W - 1] >> 31;
+#pragma unroll
+        for (int w = 0; w < W; ++w) x[w] = 0;
+        accumulate<W>(x, acc, neg);                                 // the magnitude
+        return round_general<N, W>(x, lo, neg ? -1 : 1, 0);
+    }
+};
+
+// Triangular recurrences over one block of kb <= kTriBlock positions, one warp per line (a row below a Cholesky diagonal
+// block, a right-hand side): x_t = RN(D(x_t; coef(t, 0..t), x_0..t) / coef(t, t)), t in solve order.  Position t is index
+// first + t * dir; x_t lies at X + (line * xl + index * xs) elements and coef(t, k) at C + (index_t * ct + index_k * ck).
+// Lane t keeps x_t's running sum; at step k lane k rounds and divides, and the lanes behind it subtract coef(t, k) x_k.
+struct TriParams {
+    const u32* C; u64 ct, ck; u32* X; u64 xl, xs;
+    i64 first; int dir, kb;
+    u64 line0, lines;
+    u32* error;
+};
+constexpr int kTriThreads = 128;
+// Shared memory: the coefficients below the diagonal by steps (step k: coef(k + 1 .. kb, k), rows an odd number of words
+// apart), the diagonal and its reciprocals.
+template <int N> __host__ __device__ constexpr int tri_row() { return (N + 3) | 1; }
+template <int N> __host__ __device__ constexpr int tri_recip_row() { return (N + 4) | 1; }
+__host__ __device__ constexpr int tri_step(int k, int kb) { return k * (2 * kb - k - 1) / 2; }   // first row of step k
+template <int N> __host__ __device__ constexpr size_t tri_smem_bytes(int kb) {
+    return 4 * ((size_t)(tri_step(kb, kb) + kb) * tri_row<N>() + (size_t)kb * tri_recip_row<N>());
+}
+template <int N> __global__ void __launch_bounds__(kTriThreads) tri_kernel(const TriParams p) {
+    constexpr int E = N + 3, S = tri_row<N>(), RS = tri_recip_row<N>();
+    constexpr u32 FULL = 0xffffffffu;
+    extern __shared__ u32 tri_park[];
+    const int kb = p.kb, lane = threadIdx.x & 31;
+    u32* const coef = tri_park;
+    u32* const diag = coef + tri_step(kb, kb) * S;
+    u32* const recip = diag + kb * S;
+    for (int x = threadIdx.x; x < kb * kb * E; x += kTriThreads) {          // coef(t, k), k <= t
+        const int e = x / E, w = x - e * E, t = e / kb, k = e - t * kb;
+        if (k > t) continue;
+        const u32 v = ldw<false>(p.C + ((u64)(p.first + t * p.dir) * p.ct + (u64)(p.first + k * p.dir) * p.ck) * E + w);
+        (k == t ? diag + t * S : coef + (tri_step(k, kb) + t - k - 1) * S)[w] = v;
+    }
+    __syncthreads();
+    if ((int)threadIdx.x < kb) store<N + 1>(recip + threadIdx.x * RS, reciprocal<N>(load_plain<N>(diag + threadIdx.x * S)));
+    __syncthreads();
+    const u64 line = p.line0 + ((u64)blockIdx.x * kTriThreads + threadIdx.x) / 32;
+    if (line >= p.lines) return;
+    const bool mine = lane < kb;
+    u32* const x = p.X + (line * p.xl + (u64)(p.first + lane * p.dir) * p.xs) * E;
+    Num<N> c = zero<N>();
+    if (mine) c = ldn<N, false>(x);
+    // anchor: x_k is guessed as c_k / coef(k, k), with 96 bits of room above the largest term so guessed
+    constexpr int kNone = INT_MIN / 2;
+    const int guess = mine && c.s ? c.e - (int)diag[lane * S + N] + 1 : kNone;
+    int top = mine && c.s ? c.e : kNone;
+    for (int k = 0; k < kb; ++k) {
+        const int g = __shfl_sync(FULL, guess, k);
+        if (mine && lane > k && g != kNone) {
+            const u32* f = coef + (tri_step(k, kb) + lane - k - 1) * S;
+            if (f[N + 1]) { const int h = (int)f[N] + g; top = h > top ? h : top; }
+        }
+    }
+    RunningSum<N> sum;
+    sum.start(c, RunningSum<N>::anchor((i64)top + 97));
+    for (int k = 0; k < kb; ++k) {
+        Num<N> v = zero<N>();
+        const bool redo = __shfl_sync(FULL, (int)sum.bad, k) != 0 && !__shfl_sync(FULL, sum.st, k);
+        if (redo) {
+            const u32* ck = p.C + ((u64)(p.first + k * p.dir) * p.ct + (u64)p.first * p.ck) * E;
+            u32* xk = p.X + (line * p.xl + (u64)p.first * p.xs) * E;
+            v = warp_exact_dot<N, false>(xk + (i64)k * p.dir * (i64)p.xs * E, true, xk, (i64)p.dir * (i64)p.xs, ck, (i64)p.dir * (i64)p.ck,
+                                         (u64)k, p.error);
+        }
+        if (lane == k) {
+            if (!redo) v = sum.round();
+            v = div_by<N>(v, load_plain<N>(diag + k * S), load_plain<N + 1>(recip + k * RS));
+            store<N>(x, v);
+        }
+        __syncwarp();
+        if (k + 1 == kb) break;
+#pragma unroll
+        for (int w = 0; w < N; ++w) v.m[w] = __shfl_sync(FULL, v.m[w], k);
+        v.e = __shfl_sync(FULL, v.e, k); v.s = __shfl_sync(FULL, v.s, k); v.st = __shfl_sync(FULL, v.st, k);
+        if (mine && lane > k) sum.subtract(load_plain<N>(coef + (tri_step(k, kb) + lane - k - 1) * S), v);
+    }
+}
+
 // ---------------------------------------------------------------- blocked Cholesky pieces
 // W: n x n row-major work matrix (element stride E).  D(c; x, y; K) = RN(c - sum x_k y_k), one rounding.
 struct CholParams { u32* W; u64 n, k0, k1; long long* info; u32* error; };
@@ -442,6 +668,112 @@ template <int N> __global__ void __launch_bounds__(diag_threads<N>()) chol_diag_
             store<N>(wij, div<N>(ldn<N, false>(wij), ldn<N, false>(wjj)));
         }
         __syncthreads();
+    }
+}
+// The same for blocks of at most kTriBlock columns and widths up to kDiagLimbs, with running sums (in shared memory, one
+// per entry below the second column).  The first warp carries the serial chain on its own, lane i for row i: subtract step k from column k + 1,
+// round it, take the root and reciprocal of its pivot, divide the rows below.  The other warps meanwhile subtract step k from the later
+// columns; one barrier a step.  One warp per dot product took 13.8 us a column at 256 bits.
+constexpr int kDiagLimbs = 24;    // the sums and the block fit shared memory up to here
+constexpr int kDiagThreads = 256;
+template <int N> __host__ __device__ constexpr int diag_sum_row() { return (2 * N + 10 + 2) | 1; }      // window, status, bad
+template <int N> __host__ __device__ constexpr size_t diag_smem_bytes(int kb) {
+    const int entries = kb * (kb + 1) / 2;
+    return 4 * ((size_t)entries * (diag_sum_row<N>() + tri_row<N>()) + 32 + tri_recip_row<N>() + tri_row<N>());
+}
+__host__ __device__ constexpr int diag_entry(int i, int j) { return i * (i + 1) / 2 + j; }
+template <int N> __device__ __forceinline__ void diag_load(RunningSum<N>& r, const u32* row, i64 lo) {
+#pragma unroll
+    for (int w = 0; w < RunningSum<N>::W; ++w) r.acc[w] = row[w];
+    r.st = row[RunningSum<N>::W]; r.bad = row[RunningSum<N>::W + 1] != 0; r.lo = lo;
+}
+template <int N> __device__ __forceinline__ void diag_keep(const RunningSum<N>& r, u32* row) {
+#pragma unroll
+    for (int w = 0; w < RunningSum<N>::W; ++w) row[w] = r.acc[w];
+    row[RunningSum<N>::W] = r.st; row[RunningSum<N>::W + 1] = r.bad;
+}
+template <int N> __global__ void __launch_bounds__(kDiagThreads) chol_diag_sums_kernel(CholParams p) {
+    constexpr int E = N + 3, S = tri_row<N>(), SR = diag_sum_row<N>();
+    constexpr u32 FULL = 0xffffffffu;
+    extern __shared__ u32 diag_park[];
+    const int kb = (int)(p.k1 - p.k0), entries = kb * (kb + 1) / 2, lane = threadIdx.x & 31;
+    u32* const sums = diag_park;
+    u32* const L = sums + entries * SR;                             // the block's entries, then of the factor
+    int* const top = reinterpret_cast<int*>(L + entries * S);       // exponents of the block's diagonal
+    u32* const recip = reinterpret_cast<u32*>(top + 32);
+    u32* const pivot = recip + tri_recip_row<N>();
+    __shared__ int failed;
+    if (!threadIdx.x) failed = 0;
+    for (int x = threadIdx.x; x < kb * kb * E; x += kDiagThreads) {
+        const int e = x / E, w = x - e * E, i = e / kb, j = e - i * kb;
+        if (j <= i) L[diag_entry(i, j) * S + w] = ldw<false>(p.W + ((p.k0 + i) * p.n + p.k0 + j) * E + w);
+    }
+    __syncthreads();
+    if ((int)threadIdx.x < kb) top[threadIdx.x] = (int)L[diag_entry(threadIdx.x, threadIdx.x) * S + N];
+    __syncthreads();
+    // a positive definite block has |w_ij| and every |l_ik l_jk| below 2^((e_ii + e_jj) / 2 + 1)
+    const auto anchor = [&](int i, int j) { return RunningSum<N>::anchor((((i64)top[i] + top[j]) >> 1) + 2); };
+    for (int e = threadIdx.x; e < kb * kb; e += kDiagThreads) {
+        const int i = e / kb, j = e - i * kb;
+        if (j > i) continue;
+        RunningSum<N> r;
+        r.start(load_plain<N>(L + diag_entry(i, j) * S), anchor(i, j));
+        diag_keep<N>(r, sums + diag_entry(i, j) * SR);
+    }
+    __syncthreads();
+    for (int j = 0; j < kb; ++j) {
+        // steps before j - 1 are in every sum; the first warp subtracts step j - 1 from column j, the others from columns after j
+        if (threadIdx.x < 32) {
+            const int i = lane;
+            const bool live = i >= j && i < kb;
+            Num<N> v = zero<N>();
+            bool bad = false;
+            if (live) {
+                RunningSum<N> r;
+                diag_load<N>(r, sums + diag_entry(i, j) * SR, anchor(i, j));
+                if (j) r.subtract(load_plain<N>(L + diag_entry(i, j - 1) * S), load_plain<N>(L + diag_entry(j, j - 1) * S));
+                v = r.round();
+                bad = r.bad && !r.st;
+            }
+            for (u32 todo = __ballot_sync(FULL, bad); todo; todo &= todo - 1) {      // formed afresh, row by row
+                const u64 gi = p.k0 + (u64)__ffs(todo) - 1, gj = p.k0 + j;
+                const Num<N> d = warp_exact_dot<N, false>(p.W + (gi * p.n + gj) * E, true, p.W + (gi * p.n + p.k0) * E, 1,
+                                                          p.W + (gj * p.n + p.k0) * E, 1, (u64)j, p.error);
+                if (i == __ffs(todo) - 1) v = d;
+            }
+            if (i == j) {
+                if (v.st || v.s <= 0) {
+                    p.info[0] = (long long)(p.k0 + j); p.info[1] = v.st ? 0 : v.s; p.info[2] = v.st;
+                    failed = 1;
+                } else {
+                    v = lfd::sqrt<N>(v);
+                    store<N>(pivot, v);
+                    store<N + 1>(recip, reciprocal<N>(v));
+                }
+            }
+            __syncwarp();
+            if (!*(volatile int*)&failed && live) {
+                if (i > j) v = div_by<N>(v, load_plain<N>(pivot), load_plain<N + 1>(recip));
+                store<N>(L + diag_entry(i, j) * S, v);
+                store<N>(p.W + ((p.k0 + i) * p.n + p.k0 + j) * E, v);
+            }
+        } else if (j) {
+            // entries (i, c), j < c <= i < kb, flattened over the threads
+            const int m = kb - j - 1, count = m * (m + 1) / 2;
+            for (int e = (int)threadIdx.x - 32; e < count; e += kDiagThreads - 32) {
+                int r = (int)((sqrtf(8.0f * (float)e + 1.0f) - 1.0f) * 0.5f);          // row of the triangle
+                while (r * (r + 1) / 2 > e) --r;
+                while ((r + 1) * (r + 2) / 2 <= e) ++r;
+                const int i = j + 1 + r, c = j + 1 + e - r * (r + 1) / 2;
+                u32* row = sums + diag_entry(i, c) * SR;
+                RunningSum<N> s;
+                diag_load<N>(s, row, anchor(i, c));
+                s.subtract(load_plain<N>(L + diag_entry(i, j - 1) * S), load_plain<N>(L + diag_entry(c, j - 1) * S));
+                diag_keep<N>(s, row);
+            }
+        }
+        __syncthreads();
+        if (failed) return;
     }
 }
 // Rows i in [r0, n) below the diagonal block: l_ij = RN(D(w_ij; row i, row j; [k0,j)) / l_jj) for
@@ -555,13 +887,30 @@ typedef void (*SolveFn)(const SolveParams&, bool, cudaStream_t);
 struct FactorKernels { CholDiagFn diag; CholRowsFn rows; CholPrepFn prep; SolveFn solve; };
 const FactorKernels* factor_kernels(int limbs);
 
+template <int N> void tri_launch(const TriParams& p, cudaStream_t s) {
+    const size_t smem = tri_smem_bytes<N>(p.kb);
+    if (smem > 48 * 1024) cudaFuncSetAttribute(tri_kernel<N>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    tri_kernel<N><<<(unsigned)((p.lines - p.line0 + kTriThreads / 32 - 1) / (kTriThreads / 32)), kTriThreads, smem, s>>>(p);
+}
 template <int N> void chol_diag_launch(const CholParams& p, cudaStream_t s) {
+    if constexpr (N <= kDiagLimbs) {
+        if (p.k1 - p.k0 <= kTriBlock) {
+            const size_t smem = diag_smem_bytes<N>((int)(p.k1 - p.k0));
+            cudaFuncSetAttribute(chol_diag_sums_kernel<N>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+            chol_diag_sums_kernel<N><<<1, kDiagThreads, smem, s>>>(p);
+            return;
+        }
+    }
     const size_t smem = dot_smem_bytes<N>(diag_threads<N>() / 32);
     cudaFuncSetAttribute(chol_diag_kernel<N>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     chol_diag_kernel<N><<<1, diag_threads<N>(), smem, s>>>(p);
 }
 template <int N> void chol_rows_launch(const CholParams& p, u64 r0, u64 jend, cudaStream_t s) {
     if (r0 >= p.n || jend <= p.k0) return;
+    if (jend - p.k0 <= kTriBlock) {
+        tri_launch<N>(TriParams{p.W, p.n, 1, p.W, p.n, 1, (i64)p.k0, 1, (int)(jend - p.k0), r0, p.n, p.error}, s);
+        return;
+    }
     const u64 rows = p.n - r0;
     chol_rows_kernel<N><<<(unsigned)((rows + 3) / 4), 128, dot_smem_bytes<N>(4) + kRecips * (N + 4) * 4, s>>>(p, r0, jend);
 }
@@ -572,6 +921,13 @@ template <int N> void chol_prep_launch(const u32* A, u32* W, u64 n, u64 fail, cu
 }
 template <int N> void solve_launch(const SolveParams& p, bool forward, cudaStream_t s) {
     if (!p.nrhs || p.r1 <= p.r0) return;
+    if (p.r1 - p.r0 <= kTriBlock) {
+        const int kb = (int)(p.r1 - p.r0);
+        const bool rows = forward || p.upper;                         // coef(t, k) along row t of L (of R), else along column t
+        tri_launch<N>(TriParams{p.L, rows ? p.n : 1, rows ? 1 : p.n, p.X, 1, p.nrhs, (i64)(forward ? p.r0 : p.r1 - 1), forward ? 1 : -1, kb,
+                                0, p.nrhs, p.error}, s);
+        return;
+    }
     const unsigned blocks = (unsigned)((p.nrhs + 3) / 4);
     const size_t smem = dot_smem_bytes<N>(4) + kRecips * (N + 4) * 4;
     if (forward) solve_forward_kernel<N><<<blocks, 128, smem, s>>>(p);
