@@ -68,31 +68,28 @@ template <int N> __global__ void cqr_load_kernel(CqrPanel p) {
     for (u64 w = 0; w < C2; ++w) { p.Vt[q * C2 + w] = 0; p.Vi[q * C2 + w] = 0; }
 }
 // Column c by the panel's reflectors so far: x_r = (D(Re x_r; Vr[r][0..q), conj y), D(Im x_r; Vr[r][0..q), i conj y))
-// over 2q real terms each (linalg_complex.mm:188-193).  One warp per row.
-template <int N> __global__ void __launch_bounds__(256) cqr_update_kernel(CqrPanel p, u64 c) {
+// over 2q real terms each (linalg_complex.mm:188-193).  Four lanes per component of a row.
+template <int N> __global__ void __launch_bounds__(kQrUpdateThreads) cqr_update_kernel(CqrPanel p, u64 c) {
     constexpr u64 E = N + 3, C2 = 2 * E;
     const long long rank = p.st->rank, j = (long long)(p.k0 + c);
     const long long q = (rank < j ? rank : j) - (long long)p.k0;
     if (q <= 0) return;
-    const u64 r = ((u64)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    if (r >= p.mr) return;
-    u32* x = p.Pt + (c * p.mr + r) * C2;
-    const u32* vr = p.Vr + r * p.nb * C2;
-    const Num<N> re = warp_exact_dot<N, true>(x, true, vr, 1, p.yc, 1, 2 * (u64)q, p.error);
-    const Num<N> im = warp_exact_dot<N, true>(x + E, true, vr, 1, p.yic, 1, 2 * (u64)q, p.error);
-    if ((threadIdx.x & 31) == 0) cq_store<N>(x, re, im);
+    const u64 t = ((u64)blockIdx.x * kQrUpdateThreads + threadIdx.x) >> 2, r = t >> 1;
+    if (r >= p.mr) return;                                        // a group of four leaves together
+    u32* x = p.Pt + (c * p.mr + r) * C2 + (t & 1) * E;
+    const Num<N> v = quad_exact_dot<N, true>(x, true, p.Vr + r * p.nb * C2, 1, t & 1 ? p.yic : p.yc, 1, 2 * (u64)q, p.error);
+    if ((threadIdx.x & 3) == 0) store<N>(x, v);
 }
 // Reflector of column c (linalg_complex.mm:205-226): s = P(x^H x); a zero or status column, or one failing the rank
 // test, ends the factorization; otherwise, when anything lies below the diagonal or Im alpha != 0, beta =
-// -sgn(Re alpha) sqrt(s), v0 = (RN(Re alpha - beta), Im alpha), v = 2^-e (v0, x_1, ...) with e = exponent(Re v0) and
-// tau = (RN(2 / P(v^H v)), 0) when Im v0 = 0, else with a = P(v^H v) / 2, b = RN(2^-e beta Im v0), d = RN(a^2 + b^2):
-// tau = (RN(a / d), -RN(b / d)); nothing to reflect: tau = 0, v = e_c, r_jj = alpha.  r_jj = (beta, 0), T_cc = tau,
-// and the rows of v and i v from row c (Vt, Vi, Vr).  One block.
+// -sgn(Re alpha) sqrt(s), v0 = (RN(Re alpha - beta), Im alpha), v = 2^-e (v0, x_1, ...) with e = exponent(Re v0) (nothing to
+// reflect: v = e_c, r_jj = alpha).  r_jj = (beta, 0), and the rows of v and i v from row c (Vt, Vi, Vr); tau
+// follows in cqr_tau.  One block.
 template <int N> __global__ void __launch_bounds__(kQrThreads) cqr_reflect_kernel(CqrPanel p, u64 c) {
     __shared__ __align__(16) u32 sm[qr_dot_words<N>()];
     __shared__ u32 s_keep[qr_keep_words<N>()];
     __shared__ long long s_e;
-    __shared__ int s_go, s_needs, s_fast;
+    __shared__ int s_go, s_needs;
     constexpr u64 E = N + 3, C2 = 2 * E;
     QrState* st = p.st;
     if (st->rank < (long long)p.n) return;
@@ -127,38 +124,19 @@ template <int N> __global__ void __launch_bounds__(kQrThreads) cqr_reflect_kerne
     if (!s_go) return;
     const long long e = s_e;
     const bool needs = s_needs;
-    Num<N> tre = zero<N>(), tim = zero<N>();
-    auto tau_of = [&](const Num<N>& sv) {                             // thread 0
-        const Num<N> vim = load_plain<N>(v + E);
-        if (!vim.s && !vim.st) tre = divx<N>(qr_pow2<N>(1), sv);
-        else {
-            const Num<N> a = qr_scaled<N>(sv, 1), b = mulx<N>(qr_scaled<N>(beta, e), vim);
-            const Num<N> d = dot2_add<N>(a, a, b, b, zero<N>());
-            tre = divx<N>(a, d); tim = negate<N>(divx<N>(b, d));
-        }
-    };
-    // Thread 0 forms P(v^H v) from the kept window and tau while warps 1.. scale the rest of the reflector.
-    if (threadIdx.x == 0) {
-        Num<N> sv;
-        const int fast = needs && qr_resum<N>(s_keep, are, v0, e, sv);
-        if (fast) tau_of(sv);
-        s_fast = fast;
-    }
-    if (needs && threadIdx.x >= 32)
-        for (u64 r = 1 + threadIdx.x - 32; r < len; r += kQrThreads - 32)
+    for (int w = threadIdx.x; w < qr_keep_words<N>(); w += kQrThreads) st->keep[w] = s_keep[w];
+    if (needs)
+        for (u64 r = 1 + threadIdx.x; r < len; r += kQrThreads)
             cq_store<N>(v + r * C2, qr_scaled<N>(load_plain<N>(xc + r * C2), e), qr_scaled<N>(load_plain<N>(xc + r * C2 + E), e));
-    __syncthreads();
-    if (needs && !s_fast) {
-        const Num<N> sv = block_exact_dot<N, false>(v, 1, v, 1, 2 * len, sm, p.error);
-        if (threadIdx.x == 0) tau_of(sv);
-    }
     if (threadIdx.x == 0) {
+        store<N>(st->keep + kQrKeepMax, are);
+        store<N>(st->keep + kQrKeepMax + E, v0);
+        st->reflects = needs;
         cq_store<N>(xc, beta, zero<N>());
-        cq_store<N>(p.tau + j * C2, tre, tim);
-        cq_store<N>(p.T + ((p.k0 / p.nb) * p.nb * p.nb + c * p.nb + c) * C2, tre, tim);
         if (!st->have_top || (long long)beta.e > st->top) st->top = beta.e;
         st->have_top = 1;
     }
+    __syncthreads();
     for (u64 r = threadIdx.x; r < len; r += kQrThreads) {
         cq_times_i<N>(iv + r * C2, v + r * C2);
         for (u64 w = 0; w < C2; ++w) p.Vr[((c + r) * p.nb + c) * C2 + w] = v[r * C2 + w];
@@ -168,71 +146,134 @@ template <int N> __global__ void __launch_bounds__(kQrThreads) cqr_reflect_kerne
         }
     }
 }
-// After reflector c: block u < c gives G[u] = P(v_u^H v_c), block u >= c the W row entry Wp[c][u+1] = P(v_c^H a_{u+1})
-// (the block-start column), over rows [c, mr), two real dots each.  kb - 1 blocks.
+// tau_c = (RN(2 / P(v^H v)), 0) when Im v0 = 0, else with a = P(v^H v) / 2, b = RN(2^-e beta Im v0), d = RN(a^2 + b^2):
+// (RN(a / d), -RN(b / d)); zero when nothing was reflected.  Also T_cc; by one block, as qr_tau.
+template <int N> __device__ __noinline__ void cqr_tau(const CqrPanel p, u64 c, u32* sm) {
+    constexpr u64 E = N + 3, C2 = 2 * E;
+    __shared__ int s_done;
+    const QrState* st = p.st;
+    const u32* v = p.Vt + (c * p.mr + c) * C2;
+    Num<N> tre = zero<N>(), tim = zero<N>();
+    auto tau_of = [&](const Num<N>& sv, long long e) {                // thread 0
+        const Num<N> vim = load_plain<N>(v + E);
+        if (!vim.s && !vim.st) tre = divx<N>(qr_pow2<N>(1), sv);
+        else {
+            const Num<N> beta = load_plain<N>(p.Pt + (c * p.mr + c) * C2);
+            const Num<N> a = qr_scaled<N>(sv, 1), b = mulx<N>(qr_scaled<N>(beta, e), vim);
+            const Num<N> d = dot2_add<N>(a, a, b, b, zero<N>());
+            tre = divx<N>(a, d); tim = negate<N>(divx<N>(b, d));
+        }
+    };
+    const Num<N> v0 = load_plain<N>(st->keep + kQrKeepMax + E);
+    if (threadIdx.x == 0) {
+        s_done = 1;
+        if (st->reflects) {
+            Num<N> sv;
+            s_done = qr_resum<N>(st->keep, load_plain<N>(st->keep + kQrKeepMax), v0, v0.e, sv);
+            if (s_done) tau_of(sv, v0.e);
+        }
+    }
+    __syncthreads();
+    if (!s_done) {
+        const Num<N> sv = block_exact_dot<N, true>(v, 1, v, 1, 2 * (p.mr - c), sm, p.error);
+        if (threadIdx.x == 0) tau_of(sv, v0.e);
+    }
+    if (threadIdx.x == 0) {
+        cq_store<N>(p.tau + (p.k0 + c) * C2, tre, tim);
+        cq_store<N>(p.T + ((p.k0 / p.nb) * p.nb * p.nb + c * p.nb + c) * C2, tre, tim);
+    }
+}
+// After reflector c: block pair u < c gives G[u] = P(v_u^H v_c), with its conjugate and i times that for the T column, block
+// pair u >= c the W row entry Wp[c][u+1] = P(v_c^H a_{u+1}) (the block-start column), over rows [c, mr): one block per real
+// dot, 2 (kb - 1) blocks, and one for tau.
 template <int N> __global__ void __launch_bounds__(kQrThreads) cqr_dots_kernel(CqrPanel p, u64 c) {
     __shared__ __align__(16) u32 sm[qr_dot_words<N>()];
     constexpr u64 E = N + 3, C2 = 2 * E;
     const long long rank = p.st->rank;
     const bool reflected = rank == (long long)p.n;
-    const u64 len = p.mr - c, u = blockIdx.x;
+    const u64 len = p.mr - c, u = blockIdx.x >> 1;
+    const int im = blockIdx.x & 1;
     if (reflected && u + 1 < p.kb) {
         const u32* v = p.Vt + (c * p.mr + c) * C2;
         const u32* iv = p.Vi + (c * p.mr + c) * C2;
-        const u32 *a0, *a1, *b0;
-        u32* out;
-        if (u < c) { a0 = p.Vt + (u * p.mr + c) * C2; a1 = p.Vi + (u * p.mr + c) * C2; b0 = v; out = p.G + u * C2; }
-        else { a0 = v; a1 = iv; b0 = p.Pt + ((u + 1) * p.mr + c) * C2; out = p.Wp + (c * p.nb + u + 1) * C2; }
-        const Num<N> re = block_exact_dot<N, true>(a0, 1, b0, 1, 2 * len, sm, p.error);
-        const Num<N> im = block_exact_dot<N, true>(a1, 1, b0, 1, 2 * len, sm, p.error);
-        if (threadIdx.x == 0) cq_store<N>(out, re, im);
+        const u32 *a, *b;
+        if (u < c) { a = (im ? p.Vi : p.Vt) + (u * p.mr + c) * C2; b = v; }
+        else { a = im ? iv : v; b = p.Pt + ((u + 1) * p.mr + c) * C2; }
+        const Num<N> d = block_exact_dot<N, true>(a, 1, b, 1, 2 * len, sm, p.error);
+        if (threadIdx.x == 0) {
+            if (u < c) {
+                store<N>(p.G + u * C2 + im * E, d);
+                store<N>(p.Gc + u * C2 + im * E, im ? negate<N>(d) : d);          // (re, -im)
+                store<N>(p.Gic + u * C2 + (im ^ 1) * E, d);                        // (im, re)
+            } else {
+                store<N>(p.Wp + (c * p.nb + u + 1) * C2 + im * E, d);
+            }
+        }
+    } else if (reflected) {
+        cqr_tau<N>(p, c, sm);
     }
 }
 
 // T column c, T_lc = -(tau * P(T[l][l..c) G[l..c))) with one rounding per component (cfma, linalg_complex.mm:237),
-// then the next column's conj y and i conj y for y_i = P(T[0..i][i]^H Wp[0..i][c+1]) (linalg_complex.mm:186-187): one
-// warp per entry, 16 warps.  One block, after the dots kernel.
-constexpr int kCqrTcolThreads = 512;
+// and the next column's conj y and i conj y for y_i = P(T[0..i][i]^H Wp[0..i][c+1]) (linalg_complex.mm:186-187).  As in the
+// real panel the T entries and the y_i of earlier columns run side by side, a block of two warps each (one per
+// component), and the last block to arrive forms y_c.
+constexpr int kCqrTcolThreads = 64;
 template <int N> __global__ void __launch_bounds__(kCqrTcolThreads) cqr_tcol_kernel(CqrPanel p, u64 c) {
     constexpr u64 E = N + 3, C2 = 2 * E;
+    __shared__ u32 rows[2 * 32 * dot_row_words<N>()];
+    __shared__ u32 s_part[2][N + 3];
+    __shared__ int s_last;
     const long long rank = p.st->rank;
     const bool reflected = rank == (long long)p.n;
-    const u64 j = p.k0 + c;
+    const u64 j = p.k0 + c, b = blockIdx.x;
     u32* Tb = p.T + (p.k0 / p.nb) * p.nb * p.nb * C2;
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    constexpr int WARPS = kCqrTcolThreads / 32;
-    if (reflected) {
-        for (u64 l = threadIdx.x; l < c; l += kCqrTcolThreads) { cq_conj<N>(p.Gc + l * C2, p.G + l * C2); cq_i_conj<N>(p.Gic + l * C2, p.G + l * C2); }
+    const int im = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    u32* srow = rows + im * 32 * dot_row_words<N>();
+    const long long qn = c + 1 < p.kb ? (rank < (long long)j + 1 ? rank : (long long)j + 1) - (long long)p.k0 : 0;   // entries of y
+    const auto y = [&](u64 i) {
+        u32* tcol = p.scr + i * 3 * p.nb * C2;
+        u32* itcol = tcol + p.nb * C2;
+        u32* wl = itcol + p.nb * C2;
+        for (u64 l = threadIdx.x; l <= i; l += kCqrTcolThreads) {
+            const u32* t = Tb + (l * p.nb + i) * C2;
+            for (u64 w = 0; w < C2; ++w) { tcol[l * C2 + w] = ldw<false>(t + w); wl[l * C2 + w] = p.Wp[(l * p.nb + c + 1) * C2 + w]; }
+            cq_times_i<N>(itcol + l * C2, tcol + l * C2);
+        }
         __syncthreads();
-        const Num<N> tre = ldn<N, false>(p.tau + j * C2), tim = ldn<N, false>(p.tau + j * C2 + E);
-        for (u64 l = warp; l < c; l += WARPS) {
-            const u32* trow = Tb + (l * p.nb + l) * C2;
-            const Num<N> pre = warp_exact_dot<N, false>(nullptr, false, trow, 1, p.Gc + l * C2, 1, 2 * (c - l), p.error);
-            const Num<N> pim = warp_exact_dot<N, false>(nullptr, false, trow, 1, p.Gic + l * C2, 1, 2 * (c - l), p.error);
-            if (lane == 0) {
-                const Cpx<N> z = cfma<N>(Cpx<N>{tre, tim}, Cpx<N>{pre, pim}, Cpx<N>{zero<N>(), zero<N>()});
-                cq_store<N>(Tb + (l * p.nb + c) * C2, negate<N>(z.re), negate<N>(z.im));
+        const Num<N> d = warp_exact_dot<N, false>(nullptr, false, im ? itcol : tcol, 1, wl, 1, 2 * (i + 1), p.error, srow);
+        if (lane == 0) {
+            store<N>(p.yc + i * C2 + im * E, im ? negate<N>(d) : d);               // (re, -im)
+            store<N>(p.yic + i * C2 + (im ^ 1) * E, d);                             // (im, re)
+        }
+    };
+    if (b < c) {
+        if (reflected) {
+            const Num<N> d = warp_exact_dot<N, false>(nullptr, false, Tb + (b * p.nb + b) * C2, 1, (im ? p.Gic : p.Gc) + b * C2, 1, 2 * (c - b),
+                                                      p.error, srow);
+            if (lane == 0) store<N>(s_part[im], d);
+            __syncthreads();
+            if (lane == 0) {                                       // the component of cfma(tau, (pre, pim), 0)
+                const Num<N> tre = ldn<N, false>(p.tau + j * C2), tim = ldn<N, false>(p.tau + j * C2 + E);
+                const Num<N> pre = load_plain<N>(s_part[0]), pim = load_plain<N>(s_part[1]);
+                const Num<N> z = dot2_add<N>(tre, im ? pim : pre, im ? tim : negate<N>(tim), im ? pre : pim, zero<N>());
+                store<N>(Tb + (b * p.nb + c) * C2 + im * E, negate<N>(z));
             }
         }
+    } else if (b < 2 * c && (long long)(b - c) < qn) {
+        y(b - c);
+    }
+    __threadfence();
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        const u32 before = atomicAdd(&p.st->arrivals, 1u);
+        s_last = before == gridDim.x - 1;
+        if (s_last) p.st->arrivals = 0;
     }
     __syncthreads();
-    if (c + 1 < p.kb) {
-        const long long qn = (rank < (long long)j + 1 ? rank : (long long)j + 1) - (long long)p.k0;
-        for (long long i = warp; i < qn; i += WARPS) {
-            u32* tcol = p.scr + (u64)i * 3 * p.nb * C2;
-            u32* itcol = tcol + p.nb * C2;
-            u32* wl = itcol + p.nb * C2;
-            for (long long l = lane; l <= i; l += 32) {
-                const u32* t = Tb + ((u64)l * p.nb + (u64)i) * C2;
-                for (u64 w = 0; w < C2; ++w) { tcol[l * C2 + w] = t[w]; wl[l * C2 + w] = p.Wp[((u64)l * p.nb + c + 1) * C2 + w]; }
-                cq_times_i<N>(itcol + l * C2, t);
-            }
-            __syncwarp();
-            const Num<N> yre = warp_exact_dot<N, false>(nullptr, false, tcol, 1, wl, 1, 2 * ((u64)i + 1), p.error);
-            const Num<N> yim = warp_exact_dot<N, false>(nullptr, false, itcol, 1, wl, 1, 2 * ((u64)i + 1), p.error);
-            if (lane == 0) { cq_store<N>(p.yc + i * C2, yre, negate<N>(yim)); cq_store<N>(p.yic + i * C2, yim, yre); }
-        }
-    }
+    if (!s_last || (long long)c >= qn) return;
+    __threadfence();
+    y(c);
 }
 // ---- column pivoting (linalg_complex.mm:136-139, 160-255): the real pivoted sequence on complex columns.  The
 // squared norms are real sums over the 2m split rows (qrp_norms_kernel on the split matrix); conj(v) and i conj(v)
@@ -304,7 +345,7 @@ template <int N> __global__ void __launch_bounds__(256) cqrp_column_kernel(CqrPa
 // trailing column k = j + 1 + (u - c): W[2c][k] = P(v_j . a_k), W[2c + 1][k] = P(i v_j . a_k) over the split rows
 // from 2j (block-start values).  The last block to arrive writes the T column (cfma, linalg_complex.mm:237) and then
 // the column with i times it for the Y rows.
-template <int N> __global__ void __launch_bounds__(kQrThreads) cqrp_gramw_kernel(CqrPanel p, u64 c) {
+template <int N> __global__ void __launch_bounds__(kQrThreads, 2) cqrp_gramw_kernel(CqrPanel p, u64 c) {
     __shared__ __align__(16) u32 sm[qr_dot_words<N>()];
     __shared__ int s_last;
     constexpr u64 E = N + 3, C2 = 2 * E;
@@ -323,6 +364,8 @@ template <int N> __global__ void __launch_bounds__(kQrThreads) cqrp_gramw_kernel
         const Num<N> re = block_exact_dot<N, true>(v, 1, a, (i64)p.n, 2 * len, sm, p.error);
         const Num<N> im = block_exact_dot<N, true>(iv, 1, a, (i64)p.n, 2 * len, sm, p.error);
         if (threadIdx.x == 0) { store<N>(p.Wr + (2 * c * p.n + k) * E, re); store<N>(p.Wr + ((2 * c + 1) * p.n + k) * E, im); }
+    } else {
+        cqr_tau<N>(p, c, sm);
     }
     if (threadIdx.x == 0) {
         __threadfence();
@@ -351,8 +394,8 @@ template <int N> __global__ void __launch_bounds__(kQrThreads) cqrp_gramw_kernel
     __syncthreads();
     for (u64 l = threadIdx.x; l <= c; l += kQrThreads) {
         const u32* t = Tb + (l * p.nb + c) * C2;
-        for (u64 w = 0; w < C2; ++w) p.tc[l * C2 + w] = t[w];
-        cq_times_i<N>(p.tc + (p.nb + l) * C2, t);
+        for (u64 w = 0; w < C2; ++w) p.tc[l * C2 + w] = ldw<false>(t + w);      // T_cc comes from another block
+        cq_times_i<N>(p.tc + (p.nb + l) * C2, p.tc + l * C2);
     }
 }
 // Every trailing column k > j: the Y rows Y[2c][k] = P(T[0..c][c] . W[0..2c+2)[k]), Y[2c + 1][k] = P(i T[0..c][c] .
@@ -486,14 +529,14 @@ template <int N> void cqr_load_launch(const CqrPanel& p, cudaStream_t s) {
     if (p.mr * p.nb) cqr_load_kernel<N><<<qr_grid(p.mr * p.nb, 128), 128, 0, s>>>(p);
 }
 template <int N> void cqr_update_launch(const CqrPanel& p, u64 c, cudaStream_t s) {
-    if (p.mr) cqr_update_kernel<N><<<qr_grid(p.mr * 32, 256), 256, 0, s>>>(p, c);
+    if (p.mr) cqr_update_kernel<N><<<qr_grid(p.mr * 8, kQrUpdateThreads), kQrUpdateThreads, 0, s>>>(p, c);
 }
 template <int N> void cqr_reflect_launch(const CqrPanel& p, u64 c, cudaStream_t s) { cqr_reflect_kernel<N><<<1, kQrThreads, 0, s>>>(p, c); }
 template <int N> void cqr_dots_launch(const CqrPanel& p, u64 c, cudaStream_t s) {
-    if (p.kb > 1) cqr_dots_kernel<N><<<(unsigned)(p.kb - 1), kQrThreads, 0, s>>>(p, c);
+    cqr_dots_kernel<N><<<(unsigned)(2 * (p.kb - 1) + 1), kQrThreads, 0, s>>>(p, c);
 }
 template <int N> void cqr_tcol_launch(const CqrPanel& p, u64 c, cudaStream_t s) {
-    if (p.kb > 1) cqr_tcol_kernel<N><<<1, kCqrTcolThreads, 0, s>>>(p, c);
+    if (p.kb > 1) cqr_tcol_kernel<N><<<(unsigned)(c ? 2 * c : 1), kCqrTcolThreads, 0, s>>>(p, c);
 }
 template <int N> void cqr_store_launch(const CqrPanel& p, cudaStream_t s) {
     const u64 items = p.kb * p.mr > p.kb * p.kb ? p.kb * p.mr : p.kb * p.kb;
@@ -508,8 +551,7 @@ template <int N> void cqrp_column_launch(const CqrPanel& p, u64 c, cudaStream_t 
     if (p.mr) cqrp_column_kernel<N><<<qr_grid(p.mr * 32, 256), 256, 0, s>>>(p, c);
 }
 template <int N> void cqrp_gramw_launch(const CqrPanel& p, u64 c, cudaStream_t s) {
-    const u64 blocks = c + (p.n - (p.k0 + c) - 1);
-    cqrp_gramw_kernel<N><<<(unsigned)(blocks ? blocks : 1), kQrThreads, 0, s>>>(p, c);
+    cqrp_gramw_kernel<N><<<(unsigned)(c + (p.n - (p.k0 + c) - 1) + 1), kQrThreads, 0, s>>>(p, c);
 }
 template <int N> void cqrp_trailing_launch(const CqrPanel& p, u64 c, cudaStream_t s) {
     const u64 trailing = p.n - (p.k0 + c) - 1;

@@ -4,15 +4,16 @@
 //
 // A panel of kb columns starting at column k0 is copied column-contiguous (Pt: entry (c, r) at c * mr + r,
 // mr = m - k0 rows), its reflectors are built in Vt with the same layout, and every column step runs as four
-// launches with no host round trip: the rows of the column reduced by the panel's earlier reflectors (one warp
+// launches with no host round trip: the rows of the column reduced by the panel's earlier reflectors (four lanes
 // per row), the reflector (one block: the squared norm, sqrt, the scaled reflector and tau), the panel W row and
-// Gram column (one block per dot), then one block that writes the T column and the next column's y.  Failures (zero, small or status columns) are recorded in a device-side state that the following launches
+// Gram column (one block per dot), then the T column and the next column's y (one warp an entry).  Failures (zero, small or status columns) are recorded in a device-side state that the following launches
 // and the host read; the trailing matrix is updated by the compact-WY products on the exact GEMM engine.
 #pragma once
 #include "lf_linalg.cuh"
 
 namespace lfd {
 
+constexpr int kQrKeepMax = 88;
 // Progress of one factorization, written by the panel kernels and read by the next launches and the host.
 struct QrState {
     long long rank;      // n while every column so far gave a reflector; the first failing column otherwise
@@ -22,6 +23,9 @@ struct QrState {
     int have_top;
     u32 arrivals;        // blocks of the current dots launch that have finished
     u32 recomputed;      // column pivoting: downdated squared norms recomputed from the reduced column
+    // the current reflector, for its tau: the window of s = P(x, x) (qr_keep_words), then x0 and v0, and whether it reflects
+    u32 keep[kQrKeepMax + 2 * 35];
+    int reflects;
 };
 
 struct QrPanel {
@@ -40,6 +44,7 @@ struct QrPanel {
 };
 
 constexpr int kQrThreads = 256;
+constexpr int kQrUpdateThreads = 64;      // 16 rows a block: a column of a few hundred rows still reaches many SMs
 // Window words of the block-wide exact dot: the product width plus headroom for the spread of the products'
 // exponents (about 800 bits up to 512-bit numbers, 320 bits beyond); wider spreads take the cluster method.
 template <int N> __host__ __device__ constexpr int qr_window() { return 2 * N + 10 + (N <= 16 ? 16 : 4); }
@@ -85,7 +90,10 @@ template <int N, bool RO> struct StridedPair {
 // logc, the two's-complement words) so that it can add terms to the exact sum and round again (qr_resum).
 // The window reductions run as rolled loops: these kernels are latency-bound on one or a few blocks, where the
 // instruction fetch of fully unrolled code, not the arithmetic, sets the time.
-template <int N> __host__ __device__ constexpr int qr_keep_words() { return qr_window<N>() + 6; }
+template <int N> __host__ __device__ constexpr int qr_keep_words() {
+    static_assert(qr_window<N>() + 6 <= kQrKeepMax && N <= 32, "QrState::keep holds the window");
+    return qr_window<N>() + 6;
+}
 template <int N, class Src> __device__ __noinline__ Num<N> block_exact_sum(const Src& src, u64 K, u32* sm, u32* error, u32* keep = nullptr) {
     constexpr int W = qr_window<N>();
     constexpr int WARPS = kQrThreads / 32;
@@ -258,28 +266,28 @@ template <int N> __global__ void qr_store_kernel(QrPanel p) {
 }
 
 // Column c (j = k0 + c) by the panel's reflectors so far: x_r = D(x_r; Vt[0..q)[r], y[0..q)) for every row of the
-// panel, q = min(j, rank) - k0.  One warp per row.
-template <int N> __global__ void __launch_bounds__(256) qr_update_kernel(QrPanel p, u64 c) {
+// panel, q = min(j, rank) - k0.  Four lanes per row.
+template <int N> __global__ void __launch_bounds__(kQrUpdateThreads) qr_update_kernel(QrPanel p, u64 c) {
     constexpr u64 E = N + 3;
     const long long rank = p.st->rank, j = (long long)(p.k0 + c);
     const long long q = (rank < j ? rank : j) - (long long)p.k0;
     if (q <= 0) return;
-    const u64 r = ((u64)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    if (r >= p.mr) return;
+    const u64 r = ((u64)blockIdx.x * kQrUpdateThreads + threadIdx.x) >> 2;
+    if (r >= p.mr) return;                                        // a group of four leaves together
     u32* x = p.Pt + (c * p.mr + r) * E;
-    const Num<N> v = warp_exact_dot<N, true>(x, true, p.Vt + r * E, (i64)p.mr, p.y, 1, (u64)q, p.error);
-    if ((threadIdx.x & 31) == 0) store<N>(x, v);
+    const Num<N> v = quad_exact_dot<N, true>(x, true, p.Vt + r * E, (i64)p.mr, p.y, 1, (u64)q, p.error);
+    if ((threadIdx.x & 3) == 0) store<N>(x, v);
 }
 
 // Reflector of column c from its reduced entries x = Pt[c][c..mr) (linalg.mm:675-690): s = P(x, x); a zero or
 // status column, or one failing the rank test, ends the factorization there; otherwise beta = -sgn(x0) sqrt(s),
-// v0 = RN(x0 - beta), v = 2^-e (v0, x1, ...) with e = exponent(v0) and tau = RN(2 / P(v, v)) (nothing below the
-// diagonal: tau = 0, v = e_c, beta = x0); r_jj = beta, T_cc = tau.  One block.
+// v0 = RN(x0 - beta), v = 2^-e (v0, x1, ...) with e = exponent(v0) (nothing below the diagonal: v = e_c,
+// beta = x0); r_jj = beta.  tau follows in qr_tau.  One block.
 template <int N> __global__ void __launch_bounds__(kQrThreads) qr_reflect_kernel(QrPanel p, u64 c) {
     __shared__ __align__(16) u32 sm[qr_dot_words<N>()];
     __shared__ u32 s_keep[qr_keep_words<N>()];
     __shared__ long long s_e;
-    __shared__ int s_go, s_fast;
+    __shared__ int s_go;
     constexpr u64 E = N + 3;
     QrState* st = p.st;
     if (st->rank < (long long)p.n) return;
@@ -307,33 +315,50 @@ template <int N> __global__ void __launch_bounds__(kQrThreads) qr_reflect_kernel
     __syncthreads();
     if (!s_go) return;
     const long long e = s_e;
-    // Thread 0 forms P(v, v) from the kept window and tau while warps 1.. scale the rest of the reflector.
-    Num<N> tj = zero<N>();
+    for (int w = threadIdx.x; w < qr_keep_words<N>(); w += kQrThreads) st->keep[w] = s_keep[w];
+    if (below)
+        for (u64 r = 1 + threadIdx.x; r < len; r += kQrThreads) store<N>(v + r * E, qr_scaled<N>(load_plain<N>(xc + r * E), e));
     if (threadIdx.x == 0) {
         store<N>(v, below ? qr_scaled<N>(v0, e) : qr_pow2<N>(0));
-        Num<N> pv;
-        const int fast = below && qr_resum<N>(s_keep, x0, v0, e, pv);
-        if (fast) tj = divx<N>(qr_pow2<N>(1), pv);
-        s_fast = fast;
-    }
-    if (below && threadIdx.x >= 32)
-        for (u64 r = 1 + threadIdx.x - 32; r < len; r += kQrThreads - 32) store<N>(v + r * E, qr_scaled<N>(load_plain<N>(xc + r * E), e));
-    __syncthreads();
-    if (below && !s_fast) {
-        const Num<N> pv = block_exact_dot<N, false>(v, 1, v, 1, len, sm, p.error);
-        if (threadIdx.x == 0) tj = divx<N>(qr_pow2<N>(1), pv);
-    }
-    if (threadIdx.x == 0) {
+        store<N>(st->keep + kQrKeepMax, x0);
+        store<N>(st->keep + kQrKeepMax + E, v0);
+        st->reflects = below;
         store<N>(xc, beta);
-        store<N>(p.tau + j * E, tj);
-        store<N>(p.T + ((p.k0 / p.nb) * p.nb * p.nb + c * p.nb + c) * E, tj);
         if (!st->have_top || (long long)beta.e > st->top) st->top = beta.e;
         st->have_top = 1;
     }
 }
+// tau_c = RN(2 / P(v_c, v_c)) (zero when nothing was reflected), also T_cc, by one block: from the window that the reflector kept, or
+// from v itself when that does not serve.  Only the T column needs tau, so this runs beside the dot products instead
+// of at the end of the reflector's serial chain.
+template <int N> __device__ __noinline__ void qr_tau(const QrPanel p, u64 c, u32* sm) {
+    constexpr u64 E = N + 3;
+    __shared__ int s_done;
+    const QrState* st = p.st;
+    Num<N> tj = zero<N>();
+    if (threadIdx.x == 0) {
+        s_done = 1;
+        if (st->reflects) {
+            const Num<N> x0 = load_plain<N>(st->keep + kQrKeepMax), v0 = load_plain<N>(st->keep + kQrKeepMax + E);
+            Num<N> pv;
+            s_done = qr_resum<N>(st->keep, x0, v0, v0.e, pv);
+            if (s_done) tj = divx<N>(qr_pow2<N>(1), pv);
+        }
+    }
+    __syncthreads();
+    if (!s_done) {
+        const u32* v = p.Vt + (c * p.mr + c) * E;
+        const Num<N> pv = block_exact_dot<N, true>(v, 1, v, 1, p.mr - c, sm, p.error);
+        if (threadIdx.x == 0) tj = divx<N>(qr_pow2<N>(1), pv);
+    }
+    if (threadIdx.x == 0) {
+        store<N>(p.tau + (p.k0 + c) * E, tj);
+        store<N>(p.T + ((p.k0 / p.nb) * p.nb * p.nb + c * p.nb + c) * E, tj);
+    }
+}
 
 // After reflector c: block u < c gives G[u] = P(v_u, v_c), block u >= c the W row entry Wp[c][u+1] = P(v_c,
-// a_{u+1}) (the block-start column), both over rows [c, mr) (linalg.mm:636-645).  kb - 1 blocks.
+// a_{u+1}) (the block-start column), both over rows [c, mr) (linalg.mm:636-645).  kb - 1 blocks, and one for tau.
 template <int N> __global__ void __launch_bounds__(kQrThreads) qr_dots_kernel(QrPanel p, u64 c) {
     __shared__ __align__(16) u32 sm[qr_dot_words<N>()];
     constexpr u64 E = N + 3;
@@ -346,36 +371,44 @@ template <int N> __global__ void __launch_bounds__(kQrThreads) qr_dots_kernel(Qr
         const Num<N> d = u < c ? block_exact_dot<N, true>(p.Vt + (u * p.mr + c) * E, 1, v, 1, len, sm, p.error)
                                : block_exact_dot<N, true>(v, 1, p.Pt + ((u + 1) * p.mr + c) * E, 1, len, sm, p.error);
         if (threadIdx.x == 0) store<N>(u < c ? p.G + u * E : p.Wp + (c * p.nb + u + 1) * E, d);
+    } else if (reflected) {
+        qr_tau<N>(p, c, sm);
     }
 }
-// T column c, T_lc = -RN(tau * P(T[l][l..c), G[l..c))) (linalg.mm:713), then the next column's y_i = P(T[0..i][i],
-// Wp[0..i][c+1]) for i < min(j + 1, rank) - k0 (linalg.mm:668): one warp per entry, 16 warps (a 32-column block's
-// entries in two rounds).  One block, after the dots kernel.
-constexpr int kQrTcolThreads = 512;
-template <int N> __global__ void __launch_bounds__(kQrTcolThreads) qr_tcol_kernel(QrPanel p, u64 c) {
+// T column c, T_lc = -RN(tau * P(T[l][l..c), G[l..c))) (linalg.mm:713), and the next column's y_i = P(T[0..i][i],
+// Wp[0..i][c+1]) for i < min(j + 1, rank) - k0 (linalg.mm:668).  Only y_c needs the new T column, so the T entries and the
+// earlier y_i run side by side, one warp in a block of its own each, and the last block to arrive forms y_c: two dot
+// products in sequence, where one block of 16 warps took up to four.
+template <int N> __global__ void __launch_bounds__(32) qr_tcol_kernel(QrPanel p, u64 c) {
     constexpr u64 E = N + 3;
+    __shared__ u32 rows[32 * dot_row_words<N>()];
     const long long rank = p.st->rank;
     const bool reflected = rank == (long long)p.n;
-    const u64 j = p.k0 + c;
+    const u64 j = p.k0 + c, b = blockIdx.x;
     u32* Tb = p.T + (p.k0 / p.nb) * p.nb * p.nb * E;
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    constexpr int WARPS = kQrTcolThreads / 32;
-    if (reflected) {
-        const Num<N> tj = ldn<N, false>(p.tau + j * E);
-        for (u64 l = warp; l < c; l += WARPS) {
-            const Num<N> d = warp_exact_dot<N, false>(nullptr, false, Tb + (l * p.nb + l) * E, 1, p.G + l * E, 1, c - l, p.error);
-            if (lane == 0) store<N>(Tb + (l * p.nb + c) * E, negate<N>(mulx<N>(tj, d)));
+    const int lane = threadIdx.x;
+    const long long qn = c + 1 < p.kb ? (rank < (long long)j + 1 ? rank : (long long)j + 1) - (long long)p.k0 : 0;   // entries of y
+    const auto y = [&](u64 i) {
+        const Num<N> d = warp_exact_dot<N, false>(nullptr, false, Tb + i * E, (i64)p.nb, p.Wp + (c + 1) * E, (i64)p.nb, i + 1, p.error, rows);
+        if (lane == 0) store<N>(p.y + i * E, d);
+    };
+    if (b < c) {
+        if (reflected) {
+            const Num<N> d = warp_exact_dot<N, false>(nullptr, false, Tb + (b * p.nb + b) * E, 1, p.G + b * E, 1, c - b, p.error, rows);
+            if (lane == 0) store<N>(Tb + (b * p.nb + c) * E, negate<N>(mulx<N>(ldn<N, false>(p.tau + j * E), d)));
         }
+    } else if (b < 2 * c && (long long)(b - c) < qn) {
+        y(b - c);
     }
-    __syncthreads();
-    if (c + 1 < p.kb) {
-        const long long qn = (rank < (long long)j + 1 ? rank : (long long)j + 1) - (long long)p.k0;
-        for (long long i = warp; i < qn; i += WARPS) {
-            const Num<N> d = warp_exact_dot<N, false>(nullptr, false, Tb + i * E, (i64)p.nb, p.Wp + (c + 1) * E, (i64)p.nb,
-                                                      (u64)i + 1, p.error);
-            if (lane == 0) store<N>(p.y + i * E, d);
-        }
+    u32 last = 0;
+    if (lane == 0) {
+        __threadfence();
+        last = atomicAdd(&p.st->arrivals, 1u) == gridDim.x - 1;
+        if (last) p.st->arrivals = 0;
     }
+    if (!__shfl_sync(0xffffffffu, last, 0) || (long long)c >= qn) return;
+    __threadfence();
+    y(c);
 }
 
 // ---- column pivoting (the pivoted branch of linalg.mm:600-719; xGEQP3 order) ----
@@ -478,6 +511,8 @@ template <int N> __global__ void __launch_bounds__(kQrThreads) qrp_gramw_kernel(
         const u64 k = j + 1 + (u - c);
         const Num<N> d = block_exact_dot<N, true>(v, 1, p.Wk + (j * p.n + k) * E, (i64)p.n, len, sm, p.error);
         if (threadIdx.x == 0) store<N>(p.Wr + (c * p.n + k) * E, d);
+    } else {
+        qr_tau<N>(p, c, sm);
     }
     if (threadIdx.x == 0) {
         __threadfence();
@@ -614,14 +649,14 @@ template <int N> void qr_store_launch(const QrPanel& p, cudaStream_t s) {
     if (p.kb * p.mr) qr_store_kernel<N><<<qr_grid(p.kb * p.mr, 128), 128, 0, s>>>(p);
 }
 template <int N> void qr_update_launch(const QrPanel& p, u64 c, cudaStream_t s) {
-    if (p.mr) qr_update_kernel<N><<<qr_grid(p.mr * 32, 256), 256, 0, s>>>(p, c);
+    if (p.mr) qr_update_kernel<N><<<qr_grid(p.mr * 4, kQrUpdateThreads), kQrUpdateThreads, 0, s>>>(p, c);
 }
 template <int N> void qr_reflect_launch(const QrPanel& p, u64 c, cudaStream_t s) { qr_reflect_kernel<N><<<1, kQrThreads, 0, s>>>(p, c); }
 template <int N> void qr_dots_launch(const QrPanel& p, u64 c, cudaStream_t s) {
-    if (p.kb > 1) qr_dots_kernel<N><<<(unsigned)(p.kb - 1), kQrThreads, 0, s>>>(p, c);
+    qr_dots_kernel<N><<<(unsigned)p.kb, kQrThreads, 0, s>>>(p, c);
 }
 template <int N> void qr_tcol_launch(const QrPanel& p, u64 c, cudaStream_t s) {
-    if (p.kb > 1) qr_tcol_kernel<N><<<1, kQrTcolThreads, 0, s>>>(p, c);
+    if (p.kb > 1) qr_tcol_kernel<N><<<(unsigned)(c ? 2 * c : 1), 32, 0, s>>>(p, c);
 }
 template <int N> void qr_extract_launch(const u32* Wk, u32* R, u64 n, const QrState* st, cudaStream_t s) {
     if (n) qr_extract_kernel<N><<<qr_grid(n * n, 128), 128, 0, s>>>(Wk, R, n, st);
@@ -638,8 +673,8 @@ template <int N> void qrp_column_launch(const QrPanel& p, u64 c, cudaStream_t s)
     if (p.mr) qrp_column_kernel<N><<<qr_grid(p.mr * 32, 256), 256, 0, s>>>(p, c);
 }
 template <int N> void qrp_gramw_launch(const QrPanel& p, u64 c, cudaStream_t s) {
-    const u64 trailing = p.n - (p.k0 + c) - 1, blocks = c + trailing;
-    qrp_gramw_kernel<N><<<(unsigned)(blocks ? blocks : 1), kQrThreads, 0, s>>>(p, c);
+    const u64 trailing = p.n - (p.k0 + c) - 1;
+    qrp_gramw_kernel<N><<<(unsigned)(c + trailing + 1), kQrThreads, 0, s>>>(p, c);
 }
 template <int N> void qrp_trailing_launch(const QrPanel& p, u64 c, cudaStream_t s) {
     const u64 trailing = p.n - (p.k0 + c) - 1;
