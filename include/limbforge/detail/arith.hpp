@@ -272,8 +272,8 @@ template <int A, int B, int LO, class Y> __device__ __forceinline__ void mul_row
 }
 #endif
 
-// a (A words) * b (B words) = p (A + B words).
-template <int A, int B> LFD_FN LFD_INLINE void mul_words(const u32 (&a)[A], const u32 (&b)[B], u32 (&p)[A + B]) {
+// a (A words) * b (B words) = p (A + B words).  b: an array, or a pointer whose words are read as their rows come up.
+template <int A, int B, class Y> LFD_FN LFD_INLINE void mul_words(const u32 (&a)[A], const Y& b, u32 (&p)[A + B]) {
 #ifdef __CUDA_ARCH__
     mul_rows<A, B, 0>(a, b, p);
 #else
@@ -289,7 +289,7 @@ template <int A, int B> LFD_FN LFD_INLINE void mul_words(const u32 (&a)[A], cons
     }
 #endif
 }
-template <int N> LFD_FN LFD_INLINE void mant_mul(const u32 (&a)[N], const u32 (&b)[N], u32 (&p)[2 * N]) { mul_words<N, N>(a, b, p); }
+template <int N, class Y> LFD_FN LFD_INLINE void mant_mul(const u32 (&a)[N], const Y& b, u32 (&p)[2 * N]) { mul_words<N, N>(a, b, p); }
 // Round a product of two normalized mantissas: its top bit is bit 64N-1 or 64N-2.
 template <int N> LFD_FN LFD_INLINE Num<N> round_product(const u32 (&p)[2 * N], i64 e_sum, int sign, u32 status) {
     const u32 s = (p[2 * N - 1] >> 31) ? 0u : 1u;      // normalizing left shift

@@ -11,7 +11,10 @@
 
 namespace lfd {
 
-struct Eg4Params { const u32* A; const u32* B; u32* C; u64 count, sa, sb, sc; int accumulate, negative; };
+struct Eg4Params {
+    const u32* A; const u32* B; u32* C; u64 count, sa, sb, sc; int accumulate, negative;
+    int wide;                             // every matrix starts on a 16-byte boundary
+};
 
 // Terms of one component: products x_k y_k with signs (k < cnt) and the old value as the last term.
 template <int N> struct Eg4Terms {
@@ -81,74 +84,125 @@ template <int N, bool CX> __device__ bool eg4_window_sum(const u32* a, const u32
             eg4_term<N, CX>(a, b, k, part, x, y, sg);
             const int sa = (int)x[N + 1], sb = (int)y[N + 1];
             if (!sa || !sb) continue;
-            const Num<N> xa = load_plain<N>(x), yb = load_plain<N>(y);
+            const Num<N> xa = load_plain<N>(x);
             u32 pr[2 * N];
-            mant_mul<N>(xa.m, yb.m, pr);
-            place_words<W, 2 * N>(t, pr, (i64)xa.e + yb.e - 2 * (32 * N - 1) - lo);
+            mant_mul<N>(xa.m, y, pr);                              // y's words come from shared memory as their rows need them
+            place_words<W, 2 * N>(t, pr, (i64)xa.e + (int)y[N] - 2 * (32 * N - 1) - lo);
             accumulate<W>(acc, t, sg * sa * sb < 0);
         }
         if (c.s) {
             place_words<W, N>(t, c.m, cs - lo);
             accumulate<W>(acc, t, c.s < 0);
         }
-        int sign = 1;
-        if (acc[W - 1] >> 31) {
-            sign = -1;
-            u64 cy = 1;
+        const bool neg = acc[W - 1] >> 31;
 #pragma unroll
-            for (int w = 0; w < W; ++w) { const u64 v = (u64)(u32)~acc[w] + cy; acc[w] = (u32)v; cy = v >> 32; }
-        }
-        u32 any = 0;
-#pragma unroll
-        for (int w = 0; w < W; ++w) any |= acc[w];
-        out = any ? round_general<N, W>(acc, lo, sign, 0) : zero<N>();
+        for (int w = 0; w < W; ++w) t[w] = 0;
+        accumulate<W>(t, acc, neg);                                 // the magnitude
+        out = round_general<N, W>(t, lo, neg ? -1 : 1, 0);
         return true;
     }
 }
 
-template <int N, bool CX> __global__ void __launch_bounds__(128) exact_gemm4_kernel(Eg4Params p) {
+// A block's matrices (four complex or eight real ones, a thread per output component) pass through shared memory: every
+// entry is read by eight threads, and from global memory a warp's load of one word touched a cache line an entry.  The
+// results replace the old values in the tile and leave as whole matrices (the padding between output matrices is kept).
+constexpr int kEg4Threads = 128;
+template <bool CX> constexpr int eg4_matrices() { return kEg4Threads / (CX ? 32 : 16); }
+template <int N, bool CX> constexpr int eg4_matrix_words() { return 16 * (CX ? 2 : 1) * (N + 3); }
+template <int N, bool CX> constexpr size_t eg4_smem_bytes() { return (size_t)4 * 3 * eg4_matrices<CX>() * eg4_matrix_words<N, CX>(); }
+__device__ __forceinline__ void eg4_cp_async16(u32* smem, const u32* gmem) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" :: "r"((unsigned)__cvta_generic_to_shared(smem)), "l"(gmem) : "memory");
+}
+__device__ __forceinline__ void eg4_cp_async4(u32* smem, const u32* gmem) {
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" :: "r"((unsigned)__cvta_generic_to_shared(smem)), "l"(gmem) : "memory");
+}
+// Matrices t0 .. t0 + nm - 1 of one operand, `stride` words apart.
+template <int MW> __device__ __forceinline__ void eg4_fetch(u32* tile, const u32* src, u64 t0, int nm, u64 stride, bool wide) {
+    if (wide) {
+        for (int x = threadIdx.x; x < nm * (MW / 4); x += kEg4Threads) {
+            const int m = x / (MW / 4), w = 4 * (x - m * (MW / 4));
+            eg4_cp_async16(tile + m * MW + w, src + (t0 + m) * stride + w);
+        }
+    } else {
+        for (int x = threadIdx.x; x < nm * MW; x += kEg4Threads) {
+            const int m = x / MW, w = x - m * MW;
+            eg4_cp_async4(tile + x, src + (t0 + m) * stride + w);
+        }
+    }
+}
+template <int N, bool CX> __global__ void __launch_bounds__(kEg4Threads) exact_gemm4_kernel(Eg4Params p) {
     constexpr u64 E = N + 3, S = CX ? 2 * E : E, P = CX ? 2 : 1;
-    constexpr int CNT = CX ? 8 : 4;
-    const u64 q = (u64)blockIdx.x * blockDim.x + threadIdx.x;
-    if (q >= p.count * 16 * P) return;
-    const u64 t = q / (16 * P), rest = q % (16 * P), oi = rest / P, part = rest % P;
-    const u64 i = oi / 4, j = oi % 4;
-    const u32* a = p.A + (t * p.sa + i * 4) * S;
-    const u32* b = p.B + (t * p.sb + j) * S;
-    u32* out = p.C + (t * p.sc + oi) * S + part * E;
-    const Num<N> c = p.accumulate ? load_plain<N>(out) : zero<N>();
-    u32 st = c.st;
-    bool products = false;
+    constexpr int CNT = CX ? 8 : 4, NM = eg4_matrices<CX>(), MW = eg4_matrix_words<N, CX>();
+    extern __shared__ __align__(16) u32 eg4_tiles[];
+    u32* const tA = eg4_tiles;
+    u32* const tB = tA + NM * MW;
+    u32* const tC = tB + NM * MW;
+    const u64 t0 = (u64)blockIdx.x * NM;
+    const int nm = p.count - t0 < (u64)NM ? (int)(p.count - t0) : NM;
+    eg4_fetch<MW>(tA, p.A, t0, nm, p.sa * S, p.wide);
+    eg4_fetch<MW>(tB, p.B, t0, nm, p.sb * S, p.wide);
+    if (p.accumulate) eg4_fetch<MW>(tC, p.C, t0, nm, p.sc * S, p.wide);
+    asm volatile("cp.async.commit_group;\n\tcp.async.wait_group 0;" ::: "memory");
+    __syncthreads();
+    const int t = threadIdx.x / (int)(16 * P), rest = threadIdx.x % (int)(16 * P), oi = rest / (int)P, part = rest % (int)P;
+    if (t < nm) {
+        const u32* a = tA + t * MW + (oi / 4) * 4 * S;
+        const u32* b = tB + t * MW + (oi % 4) * S;
+        u32* out = tC + t * MW + oi * S + part * E;
+        const Num<N> c = p.accumulate ? load_plain<N>(out) : zero<N>();
+        u32 st = c.st;
+        bool products = false;
 #pragma unroll 1
-    for (int k = 0; k < CNT; ++k) {
-        const u32 *x, *y; int sg;
-        eg4_term<N, CX>(a, b, k, (int)part, x, y, sg);
-        st |= x[N + 2] | y[N + 2];
-        products = products || (x[N + 1] && y[N + 1]);
+        for (int k = 0; k < CNT; ++k) {
+            const u32 *x, *y; int sg;
+            eg4_term<N, CX>(a, b, k, part, x, y, sg);
+            st |= x[N + 2] | y[N + 2];
+            products = products || (x[N + 1] && y[N + 1]);
+        }
+        Num<N> r;
+        if (st) r = zero<N>(st);
+        else if (!products) r = c;
+        else if (!eg4_window_sum<N, CX>(a, b, part, c, r)) {
+            Eg4Terms<N> src;
+            src.cnt = CNT;
+            for (int k = 0; k < CNT; ++k) eg4_term<N, CX>(a, b, k, part, src.x[k], src.y[k], src.sg[k]);
+            src.c = c;
+            r = cluster_round<N, 8 * N + 8>(src, nullptr);
+        }
+        if (p.negative) r = negate<N>(r);
+        store<N>(out, r);
     }
-    Num<N> r;
-    if (st) r = zero<N>(st);
-    else if (!products) r = c;
-    else if (!eg4_window_sum<N, CX>(a, b, (int)part, c, r)) {
-        Eg4Terms<N> src;
-        src.cnt = CNT;
-        for (int k = 0; k < CNT; ++k) eg4_term<N, CX>(a, b, k, (int)part, src.x[k], src.y[k], src.sg[k]);
-        src.c = c;
-        r = cluster_round<N, 8 * N + 8>(src, nullptr);
+    __syncthreads();
+    if (p.wide) {
+        for (int x = threadIdx.x; x < nm * (MW / 4); x += kEg4Threads) {
+            const int m = x / (MW / 4), w = 4 * (x - m * (MW / 4));
+            *reinterpret_cast<uint4*>(p.C + (t0 + m) * p.sc * S + w) = *reinterpret_cast<const uint4*>(tC + m * MW + w);
+        }
+    } else {
+        for (int x = threadIdx.x; x < nm * MW; x += kEg4Threads) {
+            const int m = x / MW, w = x - m * MW;
+            p.C[(t0 + m) * p.sc * S + w] = tC[x];
+        }
     }
-    if (p.negative) r = negate<N>(r);
-    store<N>(out, r);
 }
 
 struct Eg4Kernels { void (*run)(const Eg4Params&, bool complex_, cudaStream_t); };
 const Eg4Kernels* eg4_kernels(int limbs);
 
+template <int N, bool CX> void eg4_launch_v(const Eg4Params& pin, cudaStream_t s) {
+    constexpr size_t smem = eg4_smem_bytes<N, CX>();
+    constexpr u64 S = (CX ? 2 : 1) * (N + 3);
+    Eg4Params p = pin;
+    // a lone matrix has no stride (its argument may be anything); the others start stride * S words apart
+    const u64 strides = p.count > 1 ? (p.sa | p.sb | p.sc) * S : 0;
+    p.wide = !(((uintptr_t)p.A | (uintptr_t)p.B | (uintptr_t)p.C | 4 * strides) & 15);
+    if constexpr (smem > 48 * 1024) cudaFuncSetAttribute(exact_gemm4_kernel<N, CX>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    const unsigned blocks = (unsigned)((p.count + eg4_matrices<CX>() - 1) / eg4_matrices<CX>());
+    exact_gemm4_kernel<N, CX><<<blocks, kEg4Threads, smem, s>>>(p);
+}
 template <int N> void eg4_launch(const Eg4Params& p, bool cx, cudaStream_t s) {
-    const u64 items = p.count * 16 * (cx ? 2 : 1);
-    if (!items) return;
-    const unsigned blocks = (unsigned)((items + 127) / 128);
-    if (cx) exact_gemm4_kernel<N, true><<<blocks, 128, 0, s>>>(p);
-    else exact_gemm4_kernel<N, false><<<blocks, 128, 0, s>>>(p);
+    if (!p.count) return;
+    if (cx) eg4_launch_v<N, true>(p, s); else eg4_launch_v<N, false>(p, s);
 }
 
 }  // namespace lfd
