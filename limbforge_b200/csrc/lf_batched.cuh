@@ -141,7 +141,8 @@ struct GemmWork {
 // One k step of one complex component: sum <- the composed or fused update with x = a_ik, y = b_kj.
 // Operands are loaded next to their use (the second factor of a product word by word inside it, mul_mem),
 // so only the running sum lives across products; above 8 limbs
-// the step is an out-of-line call, which keeps the kernel's register allocation to that sum.
+// the fused step is an out-of-line call, which keeps the kernel's register allocation to that sum (composed steps above 8
+// limbs run parked, below).
 template <int N, bool FUSED> __device__ __forceinline__ void cx_step_body(Num<N>& sum, const u32* x, const u32* y, int comp) {
     constexpr u64 E = N + 3;
     const u32* yr = y + (comp ? E : 0);                 // im swaps the roles of br and bi
@@ -162,10 +163,12 @@ template <int N, bool FUSED> __device__ __forceinline__ void cx_step(Num<N>& sum
     if constexpr (N > 8) cx_step_call<N, FUSED>(sum, x, y, comp); else cx_step_body<N, FUSED>(sum, x, y, comp);
 }
 
-// Composed complex entries of 17+ limbs park their running sum and first product in shared memory (a slot of
+// Composed complex entries above 8 limbs park their running sum and first product in shared memory (a slot of
 // 2(N+3) words per thread, word w at slot[w * stride]) while the next product runs.  The kernel then needs
-// the registers of one product or one sum at a time (128), which raises the warps an SM holds from 10 to 16 at 1024 bits.
-template <int N, bool CX, bool FUSED> constexpr bool parked_state() { return CX && !FUSED && N >= 17; }
+// the registers of one product or one sum at a time (128 at 1024 bits), which keeps 16 warps an SM there.  The two products
+// of a step are one rolled loop and so are its two sums: unrolled, a step's code passed the instruction caches at 1024 bits (2.5
+// no-instruction stalls an issue).
+template <int N, bool CX, bool FUSED> constexpr bool parked_state() { return CX && !FUSED && N > 8; }
 template <int N> __device__ __forceinline__ void park(u32* slot, u32 stride, const Num<N>& v) {
 #pragma unroll
     for (int w = 0; w < N; ++w) slot[w * stride] = v.m[w];
@@ -187,11 +190,17 @@ template <int N> __device__ void gemm_cell_parked(const u32* A, const u32* B, co
     for (u64 kk = 0; kk < k; ++kk) {
         const u32* x = A + (i * k + kk) * S;
         const u32* y = B + (kk * n + j) * S;
-        park<N>(sp1, stride, mul_mem<N>(load<N>(x), y + (comp ? E : 0)));
-        const Num<N> p2 = mul_mem<N>(load<N>(x + E), y + (comp ? 0 : E));
-        const Num<N> p1 = unpark<N>(sp1, stride);
-        park<N>(sp1, stride, comp ? add<N>(p1, p2) : sub<N>(p1, p2));
-        park<N>(ssum, stride, add<N>(unpark<N>(sp1, stride), unpark<N>(ssum, stride)));
+        // re: a.re b.re - a.im b.im    im: a.re b.im + a.im b.re, then the running sum
+        Num<N> v;
+#pragma unroll 1
+        for (int t = 0; t < 2; ++t) {
+            v = mul_mem<N>(load<N>(x + t * E), y + (t ^ comp) * E);
+            if (t == 0) park<N>(sp1, stride, v);
+        }
+        if (!comp) v.s = -v.s;
+#pragma unroll 1
+        for (int t = 0; t < 2; ++t) v = add<N>(unpark<N>(t ? ssum : sp1, stride), v);
+        park<N>(ssum, stride, v);
     }
     Num<N> sum = unpark<N>(ssum, stride);
     if (negative) sum = negate<N>(sum);
