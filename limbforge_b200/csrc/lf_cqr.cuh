@@ -85,7 +85,7 @@ template <int N> __global__ void __launch_bounds__(kQrUpdateThreads) cqr_update_
 // -sgn(Re alpha) sqrt(s), v0 = (RN(Re alpha - beta), Im alpha), v = 2^-e (v0, x_1, ...) with e = exponent(Re v0) (nothing to
 // reflect: v = e_c, r_jj = alpha).  r_jj = (beta, 0), and the rows of v and i v from row c (Vt, Vi, Vr); tau
 // follows in cqr_tau.  One block.
-template <int N> __global__ void __launch_bounds__(kQrThreads) cqr_reflect_kernel(CqrPanel p, u64 c) {
+template <int N> __global__ void __launch_bounds__(qr_threads<N>()) cqr_reflect_kernel(CqrPanel p, u64 c) {
     __shared__ __align__(16) u32 sm[qr_dot_words<N>()];
     __shared__ u32 s_keep[qr_keep_words<N>()];
     __shared__ long long s_e;
@@ -99,7 +99,7 @@ template <int N> __global__ void __launch_bounds__(kQrThreads) cqr_reflect_kerne
     u32* iv = p.Vi + (c * p.mr + c) * C2;
     const Num<N> s = block_exact_dot<N, true>(xc, 1, xc, 1, 2 * len, sm, p.error, s_keep);
     int below = 0;
-    for (u64 k = 2 + threadIdx.x; k < 2 * len; k += kQrThreads) below |= ldw<true>(xc + k * E + N + 1) != 0;
+    for (u64 k = 2 + threadIdx.x; k < 2 * len; k += qr_threads<N>()) below |= ldw<true>(xc + k * E + N + 1) != 0;
     below = __syncthreads_or(below);
     Num<N> beta = zero<N>(), v0 = qr_pow2<N>(0), are = zero<N>(), aim = zero<N>();
     if (threadIdx.x == 0) {
@@ -124,9 +124,9 @@ template <int N> __global__ void __launch_bounds__(kQrThreads) cqr_reflect_kerne
     if (!s_go) return;
     const long long e = s_e;
     const bool needs = s_needs;
-    for (int w = threadIdx.x; w < qr_keep_words<N>(); w += kQrThreads) st->keep[w] = s_keep[w];
+    for (int w = threadIdx.x; w < qr_keep_words<N>(); w += qr_threads<N>()) st->keep[w] = s_keep[w];
     if (needs)
-        for (u64 r = 1 + threadIdx.x; r < len; r += kQrThreads)
+        for (u64 r = 1 + threadIdx.x; r < len; r += qr_threads<N>())
             cq_store<N>(v + r * C2, qr_scaled<N>(load_plain<N>(xc + r * C2), e), qr_scaled<N>(load_plain<N>(xc + r * C2 + E), e));
     if (threadIdx.x == 0) {
         store<N>(st->keep + kQrKeepMax, are);
@@ -137,7 +137,7 @@ template <int N> __global__ void __launch_bounds__(kQrThreads) cqr_reflect_kerne
         st->have_top = 1;
     }
     __syncthreads();
-    for (u64 r = threadIdx.x; r < len; r += kQrThreads) {
+    for (u64 r = threadIdx.x; r < len; r += qr_threads<N>()) {
         cq_times_i<N>(iv + r * C2, v + r * C2);
         for (u64 w = 0; w < C2; ++w) p.Vr[((c + r) * p.nb + c) * C2 + w] = v[r * C2 + w];
         if (p.pivot) {
@@ -186,7 +186,7 @@ template <int N> __device__ __noinline__ void cqr_tau(const CqrPanel p, u64 c, u
 // After reflector c: block pair u < c gives G[u] = P(v_u^H v_c), with its conjugate and i times that for the T column, block
 // pair u >= c the W row entry Wp[c][u+1] = P(v_c^H a_{u+1}) (the block-start column), over rows [c, mr): one block per real
 // dot, 2 (kb - 1) blocks, and one for tau.
-template <int N> __global__ void __launch_bounds__(kQrThreads) cqr_dots_kernel(CqrPanel p, u64 c) {
+template <int N> __global__ void __launch_bounds__(qr_threads<N>()) cqr_dots_kernel(CqrPanel p, u64 c) {
     __shared__ __align__(16) u32 sm[qr_dot_words<N>()];
     constexpr u64 E = N + 3, C2 = 2 * E;
     const long long rank = p.st->rank;
@@ -345,7 +345,7 @@ template <int N> __global__ void __launch_bounds__(256) cqrp_column_kernel(CqrPa
 // trailing column k = j + 1 + (u - c): W[2c][k] = P(v_j . a_k), W[2c + 1][k] = P(i v_j . a_k) over the split rows
 // from 2j (block-start values).  The last block to arrive writes the T column (cfma, linalg_complex.mm:237) and then
 // the column with i times it for the Y rows.
-template <int N> __global__ void __launch_bounds__(kQrThreads, 2) cqrp_gramw_kernel(CqrPanel p, u64 c) {
+template <int N> __global__ void __launch_bounds__(qr_threads<N>(), (N <= 8 ? 1 : 2)) cqrp_gramw_kernel(CqrPanel p, u64 c) {
     __shared__ __align__(16) u32 sm[qr_dot_words<N>()];
     __shared__ int s_last;
     constexpr u64 E = N + 3, C2 = 2 * E;
@@ -378,8 +378,8 @@ template <int N> __global__ void __launch_bounds__(kQrThreads, 2) cqrp_gramw_ker
     __threadfence();
     u32* Tb = p.T + (p.k0 / p.nb) * p.nb * p.nb * C2;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    constexpr int WARPS = kQrThreads / 32;
-    for (u64 l = threadIdx.x; l < c; l += kQrThreads) { cq_conj<N>(p.Gc + l * C2, p.G + l * C2); cq_i_conj<N>(p.Gic + l * C2, p.G + l * C2); }
+    constexpr int WARPS = qr_threads<N>() / 32;
+    for (u64 l = threadIdx.x; l < c; l += qr_threads<N>()) { cq_conj<N>(p.Gc + l * C2, p.G + l * C2); cq_i_conj<N>(p.Gic + l * C2, p.G + l * C2); }
     __syncthreads();
     const Num<N> tre = ldn<N, false>(p.tau + j * C2), tim = ldn<N, false>(p.tau + j * C2 + E);
     for (u64 l = warp; l < c; l += WARPS) {
@@ -392,7 +392,7 @@ template <int N> __global__ void __launch_bounds__(kQrThreads, 2) cqrp_gramw_ker
         }
     }
     __syncthreads();
-    for (u64 l = threadIdx.x; l <= c; l += kQrThreads) {
+    for (u64 l = threadIdx.x; l <= c; l += qr_threads<N>()) {
         const u32* t = Tb + (l * p.nb + c) * C2;
         for (u64 w = 0; w < C2; ++w) p.tc[l * C2 + w] = ldw<false>(t + w);      // T_cc comes from another block
         cq_times_i<N>(p.tc + (p.nb + l) * C2, p.tc + l * C2);
@@ -457,7 +457,7 @@ template <int N> struct CReducedSquares {
 };
 // Flagged columns: nu_k = nuref_k = P(z^H z) over the reduced column below row j (linalg_complex.mm:251-254).  One
 // block per trailing column; unflagged blocks return at once.
-template <int N> __global__ void __launch_bounds__(kQrThreads) cqrp_recompute_kernel(CqrPanel p, u64 c) {
+template <int N> __global__ void __launch_bounds__(qr_threads<N>()) cqrp_recompute_kernel(CqrPanel p, u64 c) {
     __shared__ __align__(16) u32 sm[qr_dot_words<N>()];
     constexpr u64 E = N + 3;
     if (p.st->rank < (long long)p.n) return;
@@ -531,9 +531,9 @@ template <int N> void cqr_load_launch(const CqrPanel& p, cudaStream_t s) {
 template <int N> void cqr_update_launch(const CqrPanel& p, u64 c, cudaStream_t s) {
     if (p.mr) cqr_update_kernel<N><<<qr_grid(p.mr * 8, kQrUpdateThreads), kQrUpdateThreads, 0, s>>>(p, c);
 }
-template <int N> void cqr_reflect_launch(const CqrPanel& p, u64 c, cudaStream_t s) { cqr_reflect_kernel<N><<<1, kQrThreads, 0, s>>>(p, c); }
+template <int N> void cqr_reflect_launch(const CqrPanel& p, u64 c, cudaStream_t s) { cqr_reflect_kernel<N><<<1, qr_threads<N>(), 0, s>>>(p, c); }
 template <int N> void cqr_dots_launch(const CqrPanel& p, u64 c, cudaStream_t s) {
-    cqr_dots_kernel<N><<<(unsigned)(2 * (p.kb - 1) + 1), kQrThreads, 0, s>>>(p, c);
+    cqr_dots_kernel<N><<<(unsigned)(2 * (p.kb - 1) + 1), qr_threads<N>(), 0, s>>>(p, c);
 }
 template <int N> void cqr_tcol_launch(const CqrPanel& p, u64 c, cudaStream_t s) {
     if (p.kb > 1) cqr_tcol_kernel<N><<<(unsigned)(c ? 2 * c : 1), kCqrTcolThreads, 0, s>>>(p, c);
@@ -551,7 +551,7 @@ template <int N> void cqrp_column_launch(const CqrPanel& p, u64 c, cudaStream_t 
     if (p.mr) cqrp_column_kernel<N><<<qr_grid(p.mr * 32, 256), 256, 0, s>>>(p, c);
 }
 template <int N> void cqrp_gramw_launch(const CqrPanel& p, u64 c, cudaStream_t s) {
-    cqrp_gramw_kernel<N><<<(unsigned)(c + (p.n - (p.k0 + c) - 1) + 1), kQrThreads, 0, s>>>(p, c);
+    cqrp_gramw_kernel<N><<<(unsigned)(c + (p.n - (p.k0 + c) - 1) + 1), qr_threads<N>(), 0, s>>>(p, c);
 }
 template <int N> void cqrp_trailing_launch(const CqrPanel& p, u64 c, cudaStream_t s) {
     const u64 trailing = p.n - (p.k0 + c) - 1;
@@ -559,7 +559,7 @@ template <int N> void cqrp_trailing_launch(const CqrPanel& p, u64 c, cudaStream_
 }
 template <int N> void cqrp_recompute_launch(const CqrPanel& p, u64 c, cudaStream_t s) {
     const u64 trailing = p.n - (p.k0 + c) - 1;
-    if (trailing) cqrp_recompute_kernel<N><<<(unsigned)trailing, kQrThreads, 0, s>>>(p, c);
+    if (trailing) cqrp_recompute_kernel<N><<<(unsigned)trailing, qr_threads<N>(), 0, s>>>(p, c);
 }
 
 }  // namespace lfd

@@ -592,18 +592,18 @@ template <int N> __global__ void __launch_bounds__(kTriThreads) tri_kernel(const
     Num<N> c = zero<N>();
     if (mine) c = ldn<N, false>(x);
     // anchor: x_k is guessed as c_k / coef(k, k), with 96 bits of room above the largest term so guessed
-    constexpr int kNone = INT_MIN / 2;
-    const int guess = mine && c.s ? c.e - (int)diag[lane * S + N] + 1 : kNone;
-    int top = mine && c.s ? c.e : kNone;
+    constexpr i64 kNone = INT64_MIN / 4;
+    const i64 guess = mine && c.s ? (i64)c.e - (int)diag[lane * S + N] + 1 : kNone;
+    i64 top = mine && c.s ? (i64)c.e : kNone;
     for (int k = 0; k < kb; ++k) {
-        const int g = __shfl_sync(FULL, guess, k);
+        const i64 g = __shfl_sync(FULL, guess, k);
         if (mine && lane > k && g != kNone) {
             const u32* f = coef + (tri_step(k, kb) + lane - k - 1) * S;
-            if (f[N + 1]) { const int h = (int)f[N] + g; top = h > top ? h : top; }
+            if (f[N + 1]) { const i64 h = (int)f[N] + g; top = h > top ? h : top; }
         }
     }
     RunningSum<N> sum;
-    sum.start(c, RunningSum<N>::anchor((i64)top + 97));
+    sum.start(c, RunningSum<N>::anchor(top + 97));
     for (int k = 0; k < kb; ++k) {
         Num<N> v = zero<N>();
         const bool redo = __shfl_sync(FULL, (int)sum.bad, k) != 0 && !__shfl_sync(FULL, sum.st, k);

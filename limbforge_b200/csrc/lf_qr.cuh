@@ -44,16 +44,19 @@ struct QrPanel {
 };
 
 constexpr int kQrThreads = 256;
+// Threads of the kernels around a block-wide sum: twice as many where a thread's window leaves it the registers, so that a
+// thread has half the terms (four of 2000), each a memory latency and a product.
+template <int N> __host__ __device__ constexpr int qr_threads() { return N <= 8 ? 512 : 256; }
 constexpr int kQrUpdateThreads = 64;      // 16 rows a block: a column of a few hundred rows still reaches many SMs
 // Window words of the block-wide exact dot: the product width plus headroom for the spread of the products'
 // exponents (about 800 bits up to 512-bit numbers, 320 bits beyond); wider spreads take the cluster method.
 template <int N> __host__ __device__ constexpr int qr_window() { return 2 * N + 10 + (N <= 16 ? 16 : 4); }
-// The block-wide sums reduce the threads' windows with two shuffle levels to kQrRows partial windows, which go to
-// shared memory as rows of qr_row_words words (odd: conflict-free rows and columns) and are summed by columns.
-constexpr int kQrRows = kQrThreads / 4;
+// The block-wide sums reduce the threads' windows with two shuffle levels to qr_rows partial windows, which go to
+// shared memory as rows of qr_row_words words (odd: conflict-free rows and columns) and are summed by columns, 16 rows a job.
+template <int N> __host__ __device__ constexpr int qr_rows() { return qr_threads<N>() / 4; }
 template <int N> __host__ __device__ constexpr int qr_row_words() { return qr_window<N>() | 1; }
 template <int N> __host__ __device__ constexpr int qr_dot_words() {
-    return kQrRows * qr_row_words<N>() + 1 + 8 * qr_window<N>() + 6 * (kQrThreads / 32) + N + 8;
+    return qr_rows<N>() * qr_row_words<N>() + 1 + qr_rows<N>() / 8 * qr_window<N>() + 6 * (qr_threads<N>() / 32) + N + 8;
 }
 
 template <int N> __device__ __forceinline__ Num<N> qr_pow2(int e) {
@@ -81,7 +84,7 @@ template <int N, bool RO> struct StridedPair {
 };
 
 // RN(sum_{k<K} a_k b_k) with one rounding for the operands a_k, b_k that src gives, computed by the whole block
-// (kQrThreads threads) and returned to every thread; the contract of exact_dot (statuses first; no nonzero product
+// (qr_threads<N>() threads) and returned to every thread; the contract of exact_dot (statuses first; no nonzero product
 // gives zero).  Pass 1 reduces the statuses, the number of nonzero products and the range of their scales; each
 // thread then adds its products into a two's-complement window anchored at the lowest scale, the warps sum their
 // windows with shuffles and thread 0 adds the warps' sums and rounds once.  A range wider than the window goes to
@@ -96,19 +99,19 @@ template <int N> __host__ __device__ constexpr int qr_keep_words() {
 }
 template <int N, class Src> __device__ __noinline__ Num<N> block_exact_sum(const Src& src, u64 K, u32* sm, u32* error, u32* keep = nullptr) {
     constexpr int W = qr_window<N>();
-    constexpr int WARPS = kQrThreads / 32;
-    constexpr int WP = qr_row_words<N>(), P0 = (kQrRows * WP + 1) & ~1;
+    constexpr int T = qr_threads<N>(), WARPS = T / 32, ROWS = qr_rows<N>(), PARTS = ROWS / 16;
+    constexpr int WP = qr_row_words<N>(), P0 = (ROWS * WP + 1) & ~1;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    u32* s_rows = sm;                                                // kQrRows partial windows
-    u64* s_part = reinterpret_cast<u64*>(sm + P0);                   // 4 column sums of 16 rows each, per column
-    long long* s_lo = reinterpret_cast<long long*>(s_part + 4 * W);
+    u32* s_rows = sm;                                                // ROWS partial windows
+    u64* s_part = reinterpret_cast<u64*>(sm + P0);                   // PARTS column sums of 16 rows each, per column
+    long long* s_lo = reinterpret_cast<long long*>(s_part + PARTS * W);
     long long* s_hi = s_lo + WARPS;
     u32* s_st = reinterpret_cast<u32*>(s_hi + WARPS);
     u32* s_cnt = s_st + WARPS;
     u32* s_res = s_cnt + WARPS;                                      // N + 3 words
     u32 st = 0, cnt = 0;
     long long lo = INT64_MAX, hi = INT64_MIN;
-    for (u64 k = tid; k < K; k += kQrThreads) {
+    for (u64 k = tid; k < K; k += T) {
         Num<N> a, b;
         src.operands(k, a, b);
         st |= a.st | b.st;
@@ -149,7 +152,7 @@ template <int N, class Src> __device__ __noinline__ Num<N> block_exact_sum(const
     u32 acc[W];
 #pragma unroll
     for (int w = 0; w < W; ++w) acc[w] = 0;
-    for (u64 k = tid; k < K; k += kQrThreads) {
+    for (u64 k = tid; k < K; k += T) {
         Num<N> a, b;
         src.operands(k, a, b);
         if (!a.s || !b.s) continue;
@@ -159,25 +162,25 @@ template <int N, class Src> __device__ __noinline__ Num<N> block_exact_sum(const
         accumulate<W>(acc, t, a.s * b.s < 0);
     }
 #pragma unroll 1
-    for (int o = 16; o >= 32 / (kQrThreads / kQrRows); o >>= 1) {
+    for (int o = 16; o >= 8; o >>= 1) {
         u32 other[W];
 #pragma unroll
         for (int w = 0; w < W; ++w) other[w] = __shfl_down_sync(0xffffffffu, acc[w], o);
         accumulate<W>(acc, other, false);
     }
-    constexpr int PER_WARP = kQrRows / WARPS;
+    constexpr int PER_WARP = ROWS / WARPS;
     if (lane < PER_WARP) {
         u32* row = s_rows + (warp * PER_WARP + lane) * WP;
 #pragma unroll
         for (int w = 0; w < W; ++w) row[w] = acc[w];
     }
     __syncthreads();
-    for (int job = tid; job < 4 * W; job += kQrThreads) {            // job q * W + col: rows [16q, 16q + 16) of col
+    for (int job = tid; job < PARTS * W; job += T) {                 // job q * W + col: rows [16q, 16q + 16) of col
         const int q = job / W, col = job - q * W;
-        const u32* at = s_rows + q * (kQrRows / 4) * WP + col;
+        const u32* at = s_rows + q * 16 * WP + col;
         u64 s0 = 0, s1 = 0;
 #pragma unroll
-        for (int l = 0; l < kQrRows / 4; l += 2) { s0 += at[l * WP]; s1 += at[(l + 1) * WP]; }
+        for (int l = 0; l < 16; l += 2) { s0 += at[l * WP]; s1 += at[(l + 1) * WP]; }
         s_part[job] = s0 + s1;
     }
     __syncthreads();
@@ -187,7 +190,10 @@ template <int N, class Src> __device__ __noinline__ Num<N> block_exact_sum(const
 #pragma unroll
         for (int q = 0; q < R; ++q) {
             const int w = lane + 32 * q;
-            const u64 sum = w < W ? s_part[w] + s_part[W + w] + s_part[2 * W + w] + s_part[3 * W + w] : 0;
+            u64 sum = 0;
+            if (w < W)
+#pragma unroll
+                for (int x = 0; x < PARTS; ++x) sum += s_part[x * W + w];
             v[q] = (u32)sum; h[q] = (u32)(sum >> 32);
         }
         if (keep && lane == 0) {
@@ -283,7 +289,7 @@ template <int N> __global__ void __launch_bounds__(kQrUpdateThreads) qr_update_k
 // status column, or one failing the rank test, ends the factorization there; otherwise beta = -sgn(x0) sqrt(s),
 // v0 = RN(x0 - beta), v = 2^-e (v0, x1, ...) with e = exponent(v0) (nothing below the diagonal: v = e_c,
 // beta = x0); r_jj = beta.  tau follows in qr_tau.  One block.
-template <int N> __global__ void __launch_bounds__(kQrThreads) qr_reflect_kernel(QrPanel p, u64 c) {
+template <int N> __global__ void __launch_bounds__(qr_threads<N>()) qr_reflect_kernel(QrPanel p, u64 c) {
     __shared__ __align__(16) u32 sm[qr_dot_words<N>()];
     __shared__ u32 s_keep[qr_keep_words<N>()];
     __shared__ long long s_e;
@@ -296,7 +302,7 @@ template <int N> __global__ void __launch_bounds__(kQrThreads) qr_reflect_kernel
     u32* v = p.Vt + (c * p.mr + c) * E;
     const Num<N> s = block_exact_dot<N, true>(xc, 1, xc, 1, len, sm, p.error, s_keep);
     int below = 0;
-    for (u64 r = 1 + threadIdx.x; r < len; r += kQrThreads) below |= ldw<true>(xc + r * E + N + 1) != 0;
+    for (u64 r = 1 + threadIdx.x; r < len; r += qr_threads<N>()) below |= ldw<true>(xc + r * E + N + 1) != 0;
     below = __syncthreads_or(below);
     Num<N> beta = zero<N>(), v0 = qr_pow2<N>(0), x0 = zero<N>();
     if (threadIdx.x == 0) {
@@ -315,9 +321,9 @@ template <int N> __global__ void __launch_bounds__(kQrThreads) qr_reflect_kernel
     __syncthreads();
     if (!s_go) return;
     const long long e = s_e;
-    for (int w = threadIdx.x; w < qr_keep_words<N>(); w += kQrThreads) st->keep[w] = s_keep[w];
+    for (int w = threadIdx.x; w < qr_keep_words<N>(); w += qr_threads<N>()) st->keep[w] = s_keep[w];
     if (below)
-        for (u64 r = 1 + threadIdx.x; r < len; r += kQrThreads) store<N>(v + r * E, qr_scaled<N>(load_plain<N>(xc + r * E), e));
+        for (u64 r = 1 + threadIdx.x; r < len; r += qr_threads<N>()) store<N>(v + r * E, qr_scaled<N>(load_plain<N>(xc + r * E), e));
     if (threadIdx.x == 0) {
         store<N>(v, below ? qr_scaled<N>(v0, e) : qr_pow2<N>(0));
         store<N>(st->keep + kQrKeepMax, x0);
@@ -359,7 +365,7 @@ template <int N> __device__ __noinline__ void qr_tau(const QrPanel p, u64 c, u32
 
 // After reflector c: block u < c gives G[u] = P(v_u, v_c), block u >= c the W row entry Wp[c][u+1] = P(v_c,
 // a_{u+1}) (the block-start column), both over rows [c, mr) (linalg.mm:636-645).  kb - 1 blocks, and one for tau.
-template <int N> __global__ void __launch_bounds__(kQrThreads) qr_dots_kernel(QrPanel p, u64 c) {
+template <int N> __global__ void __launch_bounds__(qr_threads<N>()) qr_dots_kernel(QrPanel p, u64 c) {
     __shared__ __align__(16) u32 sm[qr_dot_words<N>()];
     constexpr u64 E = N + 3;
     QrState* st = p.st;
@@ -426,7 +432,7 @@ template <int N> __device__ __forceinline__ int qr_order(const u32* x, const u32
     return a > 0 ? c : -c;
 }
 // nu_k = nuref_k = P(a_k, a_k) over all rows; perm = identity.  One block per column.
-template <int N> __global__ void __launch_bounds__(kQrThreads) qrp_norms_kernel(QrPanel p) {
+template <int N> __global__ void __launch_bounds__(qr_threads<N>()) qrp_norms_kernel(QrPanel p) {
     __shared__ __align__(16) u32 sm[qr_dot_words<N>()];
     constexpr u64 E = N + 3;
     const u64 k = blockIdx.x;
@@ -496,7 +502,7 @@ template <int N> __global__ void __launch_bounds__(256) qrp_column_kernel(QrPane
 // After reflector j: block u < c gives the Gram entry G[u] = P(v_u, v_j) over the panel rows [c, mr); block u >= c
 // the W row entry W[c][k] = P(v_j, a_k) over rows [j, m) of trailing column k = j + 1 + (u - c) (block-start values,
 // linalg.mm:636-645).  The last block to arrive writes the T column (linalg.mm:713).
-template <int N> __global__ void __launch_bounds__(kQrThreads) qrp_gramw_kernel(QrPanel p, u64 c) {
+template <int N> __global__ void __launch_bounds__(qr_threads<N>()) qrp_gramw_kernel(QrPanel p, u64 c) {
     __shared__ __align__(16) u32 sm[qr_dot_words<N>()];
     __shared__ int s_last;
     constexpr u64 E = N + 3;
@@ -526,7 +532,7 @@ template <int N> __global__ void __launch_bounds__(kQrThreads) qrp_gramw_kernel(
     u32* Tb = p.T + (p.k0 / p.nb) * p.nb * p.nb * E;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const Num<N> tj = ldn<N, false>(p.tau + j * E);
-    for (u64 l = warp; l < c; l += kQrThreads / 32) {
+    for (u64 l = warp; l < c; l += qr_threads<N>() / 32) {
         const Num<N> d = warp_exact_dot<N, false>(nullptr, false, Tb + (l * p.nb + l) * E, 1, p.G + l * E, 1, c - l, p.error);
         if (lane == 0) store<N>(Tb + (l * p.nb + c) * E, negate<N>(mulx<N>(tj, d)));
     }
@@ -588,7 +594,7 @@ template <int N> struct ReducedSquares {
 };
 // Flagged columns: nu_k = nuref_k = P(z, z) over the reduced column below row j (linalg.mm:724-727).  One block per
 // trailing column; unflagged blocks return at once.
-template <int N> __global__ void __launch_bounds__(kQrThreads) qrp_recompute_kernel(QrPanel p, u64 c) {
+template <int N> __global__ void __launch_bounds__(qr_threads<N>()) qrp_recompute_kernel(QrPanel p, u64 c) {
     __shared__ __align__(16) u32 sm[qr_dot_words<N>()];
     constexpr u64 E = N + 3;
     if (p.st->rank < (long long)p.n) return;
@@ -651,9 +657,9 @@ template <int N> void qr_store_launch(const QrPanel& p, cudaStream_t s) {
 template <int N> void qr_update_launch(const QrPanel& p, u64 c, cudaStream_t s) {
     if (p.mr) qr_update_kernel<N><<<qr_grid(p.mr * 4, kQrUpdateThreads), kQrUpdateThreads, 0, s>>>(p, c);
 }
-template <int N> void qr_reflect_launch(const QrPanel& p, u64 c, cudaStream_t s) { qr_reflect_kernel<N><<<1, kQrThreads, 0, s>>>(p, c); }
+template <int N> void qr_reflect_launch(const QrPanel& p, u64 c, cudaStream_t s) { qr_reflect_kernel<N><<<1, qr_threads<N>(), 0, s>>>(p, c); }
 template <int N> void qr_dots_launch(const QrPanel& p, u64 c, cudaStream_t s) {
-    qr_dots_kernel<N><<<(unsigned)p.kb, kQrThreads, 0, s>>>(p, c);
+    qr_dots_kernel<N><<<(unsigned)p.kb, qr_threads<N>(), 0, s>>>(p, c);
 }
 template <int N> void qr_tcol_launch(const QrPanel& p, u64 c, cudaStream_t s) {
     if (p.kb > 1) qr_tcol_kernel<N><<<(unsigned)(c ? 2 * c : 1), 32, 0, s>>>(p, c);
@@ -666,7 +672,7 @@ template <int N> void qr_copy_launch(const u32* src, u64 ld_src, u32* dst, u64 l
 }
 
 template <int N> void qrp_norms_launch(const QrPanel& p, cudaStream_t s) {
-    if (p.n) qrp_norms_kernel<N><<<(unsigned)p.n, kQrThreads, 0, s>>>(p);
+    if (p.n) qrp_norms_kernel<N><<<(unsigned)p.n, qr_threads<N>(), 0, s>>>(p);
 }
 template <int N> void qrp_pivot_launch(const QrPanel& p, u64 c, cudaStream_t s) { qrp_pivot_kernel<N><<<1, kQrThreads, 0, s>>>(p, c); }
 template <int N> void qrp_column_launch(const QrPanel& p, u64 c, cudaStream_t s) {
@@ -674,7 +680,7 @@ template <int N> void qrp_column_launch(const QrPanel& p, u64 c, cudaStream_t s)
 }
 template <int N> void qrp_gramw_launch(const QrPanel& p, u64 c, cudaStream_t s) {
     const u64 trailing = p.n - (p.k0 + c) - 1;
-    qrp_gramw_kernel<N><<<(unsigned)(c + trailing + 1), kQrThreads, 0, s>>>(p, c);
+    qrp_gramw_kernel<N><<<(unsigned)(c + trailing + 1), qr_threads<N>(), 0, s>>>(p, c);
 }
 template <int N> void qrp_trailing_launch(const QrPanel& p, u64 c, cudaStream_t s) {
     const u64 trailing = p.n - (p.k0 + c) - 1;
@@ -682,7 +688,7 @@ template <int N> void qrp_trailing_launch(const QrPanel& p, u64 c, cudaStream_t 
 }
 template <int N> void qrp_recompute_launch(const QrPanel& p, u64 c, cudaStream_t s) {
     const u64 trailing = p.n - (p.k0 + c) - 1;
-    if (trailing) qrp_recompute_kernel<N><<<(unsigned)trailing, kQrThreads, 0, s>>>(p, c);
+    if (trailing) qrp_recompute_kernel<N><<<(unsigned)trailing, qr_threads<N>(), 0, s>>>(p, c);
 }
 
 }  // namespace lfd
