@@ -390,9 +390,11 @@ def _ptr(a) -> C.c_void_p | None:
     return C.c_void_p(int(a))
 
 
+_CONTIGUOUS = _Broadcast(1, 0)          # passed by value, never written
+
+
 def _bc(b: Broadcast | None) -> _Broadcast:
-    b = b or Broadcast()
-    return _Broadcast(b.stride, b.period)
+    return _CONTIGUOUS if b is None else _Broadcast(b.stride, b.period)
 
 
 def _timing(t: _Timing) -> Timing:
@@ -497,23 +499,26 @@ class CommandBatch:
     def run(self, op, a: Buffer, b: Buffer | None = None, c: Buffer | None = None, out: Buffer | None = None,
             b_index: Broadcast | None = None, c_index: Broadcast | None = None) -> None:
         """run(op, a, b, out[, b_index]) / run(op, a, b, c, out[, b_index, c_index]) / run(op, a, out)"""
-        op = Operation(op)
-        if operation_is_unary(op):
+        if type(op) is not Operation:
+            op = Operation(op)
+        if op in (7, 8):                                             # unary
             out = out if out is not None else b
             b = None
-        elif not operation_is_ternary(op):
+        elif op < 9:                                                 # binary
             out = out if out is not None else c
             c = None
         if out is None:
             raise InvalidArgument("operation requires a different number of inputs")
+        n = a.count
         if b_index is None and c_index is None:
-            same = [x for x in (a, b, c, out) if x is not None]
-            if any(x.count != a.count for x in same):
+            if out.count != n or (b is not None and b.count != n) or (c is not None and c.count != n):
                 raise InvalidArgument("buffer counts must match")
-        elif a.count != out.count:
+        elif n != out.count:
             raise InvalidArgument("buffer counts do not match the broadcast")
-        check(lib.lf_batch_run(self.handle, a.bits, int(a.complex), int(op), a.handle, b.handle if b else None,
-                               c.handle if c else None, out.handle, a.count, _bc(b_index), _bc(c_index)))
+        rc = lib.lf_batch_run(self.handle, a.bits, int(a.complex), int(op), a.handle, None if b is None else b.handle,
+                              None if c is None else c.handle, out.handle, n, _bc(b_index), _bc(c_index))
+        if rc:
+            check(rc)
 
     def lu4(self, shape: Batched4, A: Buffer, B: Buffer | None, X: Buffer, det: Buffer | None, status: Buffer) -> None:
         s = _Batched4(shape.count, shape.rhs, int(shape.inverse), int(shape.determinant), int(shape.fused))

@@ -30,10 +30,10 @@ Batch::~Batch() { for (auto* r : resources) release(r); }
 
 void Submission::finish() {
     if (done) return;
-    cudaError_t e = cudaEventSynchronize(end);
+    cudaError_t e = cudaEventSynchronize(ev.end);
     if (e == cudaSuccess) {
         float ms = 0;
-        cudaEventElapsedTime(&ms, start, end);
+        cudaEventElapsedTime(&ms, ev.start, ev.end);
         timing.gpu_seconds = ms * 1e-3;
     } else {
         error = cudaGetErrorString(e);
@@ -45,9 +45,8 @@ void Submission::finish() {
     done = true;
 }
 Submission::~Submission() {
-    finish();
-    if (start) cudaEventDestroy(start);
-    if (end) cudaEventDestroy(end);
+    if (ev.end) finish();                                  // else the submission never reached its stream
+    if (pool) pool->give(ev);
 }
 
 void launch_elementwise(int bits, int op, const void* a, const void* b, const void* c, void* out, size_t count,
@@ -416,12 +415,12 @@ int lf_batch_submit(lf_batch* bt, lf_submission** out) {
     sub->wall0 = std::chrono::steady_clock::now();
     try {
         e.activate();
-        cuda_check(cudaEventCreate(&sub->start), "event");
-        cuda_check(cudaEventCreate(&sub->end), "event");
+        sub->pool = e.events;
+        sub->ev = sub->pool->take();
         for (auto* r : bt->resources) r->sync_to_device(e.stream);
-        cuda_check(cudaEventRecord(sub->start, e.stream), "event");
+        cuda_check(cudaEventRecord(sub->ev.start, e.stream), "event");
         launch_ops(e, bt->ops);
-        cuda_check(cudaEventRecord(sub->end, e.stream), "event");
+        cuda_check(cudaEventRecord(sub->ev.end, e.stream), "event");
     } catch (...) {
         cudaStreamSynchronize(e.stream);
         for (auto* r : bt->resources) r->busy.store(false);
@@ -438,7 +437,7 @@ int lf_submission_ready(lf_submission* s, int* ready) {
     LF_API_BEGIN
     if (!s || !ready) throw logic_error("empty submission");
     if (s->done) { *ready = 1; return LF_OK; }
-    cudaError_t r = cudaEventQuery(s->end);
+    cudaError_t r = cudaEventQuery(s->ev.end);
     *ready = (r == cudaSuccess || r != cudaErrorNotReady) ? 1 : 0;
     LF_API_END
 }

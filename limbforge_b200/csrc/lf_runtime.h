@@ -81,11 +81,42 @@ struct PinnedBuf {
     ~PinnedBuf() { if (p) cudaFreeHost(p); }
 };
 
+// Timing events of finished submissions, kept for the next ones (creating and destroying the pair costs a small submission
+// several microseconds).  Shared with the submissions, which may outlive their engine and finish on other threads;
+// at most kKept pairs are kept, and the last owner destroys them.
+struct EventPool {
+    static constexpr size_t kKept = 16;
+    struct Pair { cudaEvent_t start = nullptr, end = nullptr; };
+    std::mutex lock;
+    std::vector<Pair> idle;
+    Pair take() {
+        {
+            std::lock_guard<std::mutex> g(lock);
+            if (!idle.empty()) { const Pair p = idle.back(); idle.pop_back(); return p; }
+        }
+        Pair p;
+        cuda_check(cudaEventCreate(&p.start), "event");
+        const cudaError_t e = cudaEventCreate(&p.end);
+        if (e != cudaSuccess) { cudaEventDestroy(p.start); cuda_check(e, "event"); }
+        return p;
+    }
+    void give(const Pair& p) {
+        if (!p.start) return;
+        {
+            std::lock_guard<std::mutex> g(lock);
+            if (idle.size() < kKept) { idle.push_back(p); return; }
+        }
+        cudaEventDestroy(p.start); cudaEventDestroy(p.end);
+    }
+    ~EventPool() { for (const Pair& p : idle) { cudaEventDestroy(p.start); cudaEventDestroy(p.end); } }
+};
+
 struct Engine {
     int device = 0;
     uint64_t identity = 0;
     cudaStream_t stream = nullptr;
     cudaEvent_t e0 = nullptr, e1 = nullptr;
+    std::shared_ptr<EventPool> events = std::make_shared<EventPool>();
     DevBuf scratch[6];
     PinnedBuf staging[2];
     std::string name;
@@ -132,7 +163,8 @@ struct Batch {
 
 struct Submission {
     Engine* engine = nullptr;
-    cudaEvent_t start = nullptr, end = nullptr;
+    std::shared_ptr<EventPool> pool;
+    EventPool::Pair ev;
     std::vector<Buffer*> resources;
     std::vector<std::shared_ptr<void>> keep;
     bool done = false; std::string error;
