@@ -1,3 +1,18 @@
 // The limb arithmetic lives in include/limbforge/detail/arith.hpp, shared with the host-side scalar API.
 #pragma once
 #include "limbforge/detail/arith.hpp"
+#include <cuda_runtime.h>
+
+namespace lfd {
+// Asynchronous copies from global to shared memory, 16 or 4 bytes each.
+__device__ __forceinline__ void cp_async16(void* smem, const void* gmem) {
+    const unsigned a = (unsigned)__cvta_generic_to_shared(smem);
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" :: "r"(a), "l"(gmem) : "memory");
+}
+__device__ __forceinline__ void cp_async4(void* smem, const void* gmem) {
+    const unsigned a = (unsigned)__cvta_generic_to_shared(smem);
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" :: "r"(a), "l"(gmem) : "memory");
+}
+__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+template <int G> __device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;" :: "n"(G) : "memory"); }
+}  // namespace lfd

@@ -95,10 +95,8 @@ template <int N, bool CX> __device__ bool eg4_window_sum(const u32* a, const u32
             accumulate<W>(acc, t, c.s < 0);
         }
         const bool neg = acc[W - 1] >> 31;
-#pragma unroll
-        for (int w = 0; w < W; ++w) t[w] = 0;
-        accumulate<W>(t, acc, neg);                                 // the magnitude
-        out = round_general<N, W>(t, lo, neg ? -1 : 1, 0);
+        negate_words<W>(acc, neg);                                  // the magnitude
+        out = round_general<N, W>(acc, lo, neg ? -1 : 1, 0);
         return true;
     }
 }
@@ -110,23 +108,17 @@ constexpr int kEg4Threads = 128;
 template <bool CX> constexpr int eg4_matrices() { return kEg4Threads / (CX ? 32 : 16); }
 template <int N, bool CX> constexpr int eg4_matrix_words() { return 16 * (CX ? 2 : 1) * (N + 3); }
 template <int N, bool CX> constexpr size_t eg4_smem_bytes() { return (size_t)4 * 3 * eg4_matrices<CX>() * eg4_matrix_words<N, CX>(); }
-__device__ __forceinline__ void eg4_cp_async16(u32* smem, const u32* gmem) {
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" :: "r"((unsigned)__cvta_generic_to_shared(smem)), "l"(gmem) : "memory");
-}
-__device__ __forceinline__ void eg4_cp_async4(u32* smem, const u32* gmem) {
-    asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" :: "r"((unsigned)__cvta_generic_to_shared(smem)), "l"(gmem) : "memory");
-}
 // Matrices t0 .. t0 + nm - 1 of one operand, `stride` words apart.
 template <int MW> __device__ __forceinline__ void eg4_fetch(u32* tile, const u32* src, u64 t0, int nm, u64 stride, bool wide) {
     if (wide) {
         for (int x = threadIdx.x; x < nm * (MW / 4); x += kEg4Threads) {
             const int m = x / (MW / 4), w = 4 * (x - m * (MW / 4));
-            eg4_cp_async16(tile + m * MW + w, src + (t0 + m) * stride + w);
+            cp_async16(tile + m * MW + w, src + (t0 + m) * stride + w);
         }
     } else {
         for (int x = threadIdx.x; x < nm * MW; x += kEg4Threads) {
             const int m = x / MW, w = x - m * MW;
-            eg4_cp_async4(tile + x, src + (t0 + m) * stride + w);
+            cp_async4(tile + x, src + (t0 + m) * stride + w);
         }
     }
 }
@@ -142,7 +134,8 @@ template <int N, bool CX> __global__ void __launch_bounds__(kEg4Threads) exact_g
     eg4_fetch<MW>(tA, p.A, t0, nm, p.sa * S, p.wide);
     eg4_fetch<MW>(tB, p.B, t0, nm, p.sb * S, p.wide);
     if (p.accumulate) eg4_fetch<MW>(tC, p.C, t0, nm, p.sc * S, p.wide);
-    asm volatile("cp.async.commit_group;\n\tcp.async.wait_group 0;" ::: "memory");
+    cp_async_commit();
+    cp_async_wait<0>();
     __syncthreads();
     const int t = threadIdx.x / (int)(16 * P), rest = threadIdx.x % (int)(16 * P), oi = rest / (int)P, part = rest % (int)P;
     if (t < nm) {

@@ -25,17 +25,6 @@ __device__ __forceinline__ u64 bidx(u64 i, u64 s, u64 p) { u64 j = s > 1 ? i / s
 
 constexpr int kEwThreads = 128;
 
-__device__ __forceinline__ void cp_async16(void* smem, const void* gmem) {
-    const unsigned a = (unsigned)__cvta_generic_to_shared(smem);
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" :: "r"(a), "l"(gmem) : "memory");
-}
-__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
-template <int G> __device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;" :: "n"(G) : "memory"); }
-__device__ __forceinline__ void cp_async4(void* smem, const void* gmem) {
-    const unsigned a = (unsigned)__cvta_generic_to_shared(smem);
-    asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" :: "r"(a), "l"(gmem) : "memory");
-}
-
 // A block's rows (elements, or components of complex values) pass through shared memory: a thread's own N + 3 words lie
 // (N + 3) words from its neighbour's, so a load of one word by a warp touches some N + 3 cache lines, and the element-wise
 // kernels were bound by those (300,000 512-bit sums: 35 us, 1.9 TB/s).  Tiles are copied with cp.async, in

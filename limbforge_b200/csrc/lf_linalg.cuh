@@ -106,7 +106,7 @@ template <int N, bool RO> struct LineTerms {
         const Num<N> a = ldn<N, RO>(x + (i64)k * sx * E), b = ldn<N, RO>(y + (i64)k * sy * E);
         u32 prod[2 * N];
         mant_mul<N>(a.m, b.m, prod);
-        acc_add(acc, len, prod, 2 * N, off);
+        acc_add(acc, len, prod, off);
     }
 };
 template <int N, bool RO = true> __device__ __noinline__ Num<N> exact_dot_add_dev(const u32* cp, bool subtract, const u32* x, i64 sx, const u32* y, i64 sy,
@@ -217,10 +217,8 @@ template <int N, bool RO> __device__ __forceinline__ Num<N> quad_exact_dot(const
         accumulate<W>(acc, t, false);
     }
     const bool neg = acc[W - 1] >> 31;
-#pragma unroll
-    for (int w = 0; w < W; ++w) t[w] = 0;
-    accumulate<W>(t, acc, neg);                                   // the magnitude
-    return round_general<N, W>(t, lo, neg ? -1 : 1, 0);
+    negate_words<W>(acc, neg);                                    // the magnitude
+    return round_general<N, W>(acc, lo, neg ? -1 : 1, 0);
 }
 
 // Products whose every output sums a few dozen terms, as the factorizations make between their blocks: four lanes an output, no line
@@ -543,8 +541,8 @@ template <int N> struct RunningSum {
         u32 x[W];
         const bool neg = acc[W - 1] >> 31;
 #pragma unroll
-        for (int w = 0; w < W; ++w) x[w] = 0;
-        accumulate<W>(x, acc, neg);                                 // the magnitude
+        for (int w = 0; w < W; ++w) x[w] = acc[w];
+        negate_words<W>(x, neg);                                    // the magnitude
         return round_general<N, W>(x, lo, neg ? -1 : 1, 0);
     }
 };
