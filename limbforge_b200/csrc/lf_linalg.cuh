@@ -19,21 +19,26 @@ namespace lfd {
 struct LineView { const u32* base; u64 ls, ks; };
 struct LineInfo { u32 status; int top; int bottom; u32 nonzero; };
 
-// One warp per line: OR of statuses, largest and smallest exponent of the nonzero, status-free
-// entries (linalg.mm:82-112 pass 1).
-template <int N> __global__ void analyze_kernel(LineView v, u64 lines, u64 K, LineInfo* out) {
-    const u64 line = (u64)blockIdx.x * (blockDim.x / 32) + threadIdx.x / 32;
-    const int lane = threadIdx.x & 31;
-    if (line >= lines) return;
+// OR of statuses, largest and smallest exponent of the nonzero, status-free entries of every line (linalg.mm:82-112 pass 1).
+// `per_line` warps share a line (1, 2 or 4 of the block's four): an entry's three words are a memory latency, and a thousand
+// lines of a thousand entries on a warp each kept too few of them in flight (1000 lines of 2000 entries at 256 bits: 39 us, with four warps a line 27).
+constexpr int kAnalyzeWarps = 4;
+template <int N> __global__ void __launch_bounds__(32 * kAnalyzeWarps) analyze_kernel(LineView v, u64 lines, u64 K, int per_line, LineInfo* out) {
+    __shared__ LineInfo part[kAnalyzeWarps];
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, share = warp % per_line;
+    const u64 line = (u64)blockIdx.x * (kAnalyzeWarps / per_line) + warp / per_line;
     constexpr u64 E = N + 3;
     u32 st = 0, nz = 0;
     int top = INT_MIN, bottom = INT_MAX;
-    for (u64 k = lane; k < K; k += 32) {
-        const u32* p = v.base + (line * v.ls + k * v.ks) * E;
-        const u32 s = __ldg(p + N + 2);
-        const int sg = (int)__ldg(p + N + 1), e = (int)__ldg(p + N);
-        st |= s;
-        if (!s && sg) { nz += 1; top = max(top, e); bottom = min(bottom, e); }
+    if (line < lines) {
+#pragma unroll 4
+        for (u64 k = share * 32 + lane; k < K; k += 32 * per_line) {
+            const u32* p = v.base + (line * v.ls + k * v.ks) * E;
+            const u32 s = __ldg(p + N + 2);
+            const int sg = (int)__ldg(p + N + 1), e = (int)__ldg(p + N);
+            st |= s;
+            if (!s && sg) { nz += 1; top = max(top, e); bottom = min(bottom, e); }
+        }
     }
 #pragma unroll
     for (int o = 16; o; o >>= 1) {
@@ -42,7 +47,15 @@ template <int N> __global__ void analyze_kernel(LineView v, u64 lines, u64 K, Li
         top = max(top, __shfl_xor_sync(0xffffffffu, top, o));
         bottom = min(bottom, __shfl_xor_sync(0xffffffffu, bottom, o));
     }
-    if (!lane) out[line] = LineInfo{st, top, bottom, nz};
+    if (!lane) part[warp] = LineInfo{st, top, bottom, nz};
+    __syncthreads();
+    if (lane || share || line >= lines) return;
+    LineInfo r = part[warp];
+    for (int w = 1; w < per_line; ++w) {
+        const LineInfo& x = part[warp + w];
+        r.status |= x.status; r.nonzero += x.nonzero; r.top = max(r.top, x.top); r.bottom = min(r.bottom, x.bottom);
+    }
+    out[line] = r;
 }
 
 // Plan of a product whose engine is chosen on the GPU (resident products): mode 1 runs the residue
@@ -251,7 +264,8 @@ const LinalgKernels* linalg_kernels(int limbs);
 
 template <int N> void analyze_launch(LineView v, u64 lines, u64 K, LineInfo* out, cudaStream_t s) {
     if (!lines) return;
-    analyze_kernel<N><<<(unsigned)((lines + 3) / 4), 128, 0, s>>>(v, lines, K, out);
+    const int per_line = K >= 512 ? 4 : K >= 128 ? 2 : 1, per_block = kAnalyzeWarps / per_line;
+    analyze_kernel<N><<<(unsigned)((lines + per_block - 1) / per_block), 32 * kAnalyzeWarps, 0, s>>>(v, lines, K, per_line, out);
 }
 template <int N> void dot_launch(const DotParams& p, cudaStream_t s) {
     if (!p.M || !p.Nc) return;
