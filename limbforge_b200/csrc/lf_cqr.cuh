@@ -125,9 +125,7 @@ template <int N> __global__ void __launch_bounds__(qr_threads<N>()) cqr_reflect_
     const long long e = s_e;
     const bool needs = s_needs;
     for (int w = threadIdx.x; w < qr_keep_words<N>(); w += qr_threads<N>()) st->keep[w] = s_keep[w];
-    if (needs)
-        for (u64 r = 1 + threadIdx.x; r < len; r += qr_threads<N>())
-            cq_store<N>(v + r * C2, qr_scaled<N>(load_plain<N>(xc + r * C2), e), qr_scaled<N>(load_plain<N>(xc + r * C2 + E), e));
+    if (needs) qr_scale_rows<N>(v + C2, xc + C2, (len - 1) * C2, e);
     if (threadIdx.x == 0) {
         store<N>(st->keep + kQrKeepMax, are);
         store<N>(st->keep + kQrKeepMax + E, v0);
@@ -137,12 +135,17 @@ template <int N> __global__ void __launch_bounds__(qr_threads<N>()) cqr_reflect_
         st->have_top = 1;
     }
     __syncthreads();
-    for (u64 r = threadIdx.x; r < len; r += qr_threads<N>()) {
-        cq_times_i<N>(iv + r * C2, v + r * C2);
-        for (u64 w = 0; w < C2; ++w) p.Vr[((c + r) * p.nb + c) * C2 + w] = v[r * C2 + w];
+    // i v = (-im, re), v by rows, and with pivoting conj(v) = (re, -im) and i conj(v) = (im, re), word by word
+    for (u64 x = threadIdx.x; x < len * C2; x += qr_threads<N>()) {
+        const u64 r = x / C2;
+        const u32 w = (u32)(x - r * C2), part = w >= E, i = w - part * (u32)E;
+        const u32 own = v[x], other = v[r * C2 + (part ? i : E + i)];
+        const u64 row = ((c + r) * p.nb + c) * C2 + w;
+        iv[x] = !part && i == N + 1 ? 0u - other : other;
+        p.Vr[row] = own;
         if (p.pivot) {
-            cq_conj<N>(p.Vrc + ((c + r) * p.nb + c) * C2, v + r * C2);
-            cq_i_conj<N>(p.Vri + ((c + r) * p.nb + c) * C2, v + r * C2);
+            p.Vrc[row] = part && i == N + 1 ? 0u - own : own;
+            p.Vri[row] = other;
         }
     }
 }
