@@ -252,7 +252,7 @@ bool ResidueEngine::run(int bits, lfd::LineView left, lfd::LineView right, uint6
     const uint64_t aplane = (uint64_t)L * Mp * Kp, bplane = same ? 0 : (uint64_t)L * Np * Kp;
     auto* pl = static_cast<signed char*>(planes.get(2 * (aplane + bplane) + 256));
     signed char *a1 = pl, *a0 = pl + aplane, *b1 = same ? a1 : pl + 2 * aplane, *b0 = same ? a0 : pl + 2 * aplane + bplane;
-    auto* res = static_cast<uint16_t*>(residues.get(sizeof(uint16_t) * (uint64_t)L * M * Nc + 64));
+    auto* res = static_cast<uint16_t*>(residues.get(sizeof(uint16_t) * L * lfd::crt_pitch(M * Nc) + 64));
     const int xwords = n + (G + 31) / 32 + 1;
     int sms = 0;
     cuda_check(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev), "SM count");
@@ -269,19 +269,17 @@ bool ResidueEngine::run(int bits, lfd::LineView left, lfd::LineView right, uint6
         if (!same) planes_of(right, Nc, Np, rinfo, b1, b0);
         cuda_check(cudaGetLastError(), "digit planes");
     }
-    lfd::MmaParams mp{res, tab.dev, M, Nc, Kp, lower ? 1 : 0, error, nullptr, 0, 0, 1};
+    lfd::MmaParams mp{res, tab.dev, M, Nc, Kp, lower ? 1 : 0, error, nullptr, 0, 0, 1, lfd::crt_pitch(M * Nc)};
     residue_mma_launch(plane_map(a1, Kp, Mp, L, lfd::kTileM), plane_map(a0, Kp, Mp, L, lfd::kTileM),
                        plane_map(b1, Kp, same ? Mp : Np, L, lfd::kTileN), plane_map(b0, Kp, same ? Mp : Np, L, lfd::kTileN), L, mp, s);
     {
         // persistent CRT: as many CTAs per SM as TMEM holds (512 columns per SM), shared memory sized
         // so that no more than that are resident
-        const int kblocks = (tab.Kp + 127) / 128;
         unsigned grid = 0; size_t smem = 0;
-        tmem_launch_shape(tab.tmem_cols, 1024 + (size_t)kblocks * 16384 + (size_t)kblocks * tab.NB * 128, sms, (M * Nc + 127) / 128,
-                          grid, smem);
+        tmem_launch_shape(tab.tmem_cols, lfd::crt_smem_bytes(tab.Kp, tab.NB, L), sms, (M * Nc + 127) / 128, grid, smem);
         auto* sf = static_cast<uint32_t*>(misc.get(sizeof(uint32_t) * (uint64_t)(tab.qwords + lfd::kCrtExtraWords) * M * Nc + 64));
         lfd::CrtParams cp{res, tab.dev, tab.bimg, L, tab.qwords, tab.NB, tab.Kp, tab.NS, tab.tmem_cols, linfo, rinfo, C, ldc, M, Nc,
-                          subtract ? 1 : 0, lower ? 1 : 0, error, nullptr, sf};
+                          subtract ? 1 : 0, lower ? 1 : 0, error, nullptr, sf, lfd::crt_pitch(M * Nc)};
         rk->crt(cp, grid, smem, s);
         cuda_check(cudaGetLastError(), "reconstruction");
     }
@@ -420,7 +418,7 @@ std::shared_ptr<ResidentProduct> resident_product_create(int bits, lfd::LineView
     const uint64_t aplane = (uint64_t)r->Lmax * r->Mp * r->Kp, bplane = r->same ? 0 : (uint64_t)r->Lmax * r->Np * r->Kp;
     auto* pl = static_cast<signed char*>(r->planes.get(2 * (aplane + bplane) + 256));
     signed char *a1 = pl, *a0 = pl + aplane, *b1 = r->same ? a1 : pl + 2 * aplane, *b0 = r->same ? a0 : pl + 2 * aplane + bplane;
-    r->res.get(sizeof(uint16_t) * (uint64_t)r->Lmax * M * Nc + 64);
+    r->res.get(sizeof(uint16_t) * r->Lmax * lfd::crt_pitch(M * Nc) + 64);
     int maxq = 0;
     for (const auto& c : cand) maxq = std::max(maxq, c.qwords);
     r->sf.get(sizeof(uint32_t) * (uint64_t)(maxq + lfd::kCrtExtraWords) * M * Nc + 64);
@@ -462,14 +460,13 @@ void resident_product_launch(ResidentProduct& r, cudaStream_t s) {
         planes_of(r.left, r.M, r.Mp, linfo, a1, a0);
         if (!r.same) planes_of(r.right, r.Nc, r.Np, rinfo, b1, b0);
         cuda_check(cudaGetLastError(), "digit planes");
-        lfd::MmaParams mp{res, nullptr, r.M, r.Nc, r.Kp, r.lower ? 1 : 0, err, plan, 0, 0, 1};
+        lfd::MmaParams mp{res, nullptr, r.M, r.Nc, r.Kp, r.lower ? 1 : 0, err, plan, 0, 0, 1, lfd::crt_pitch(r.M * r.Nc)};
         residue_mma_launch(r.ta1, r.ta0, r.tb1, r.tb0, r.Lmax, mp, s);
         cuda_check(cudaGetLastError(), "residue products");
-        const int ckb = (r.maxKp + 127) / 128;
         unsigned cgrid = 0; size_t csmem = 0;
-        tmem_launch_shape(r.maxTmem, 1024 + (size_t)ckb * 16384 + (size_t)ckb * r.maxNB * 128, r.sms, (r.M * r.Nc + 127) / 128, cgrid, csmem);
+        tmem_launch_shape(r.maxTmem, lfd::crt_smem_bytes(r.maxKp, r.maxNB, r.Lmax), r.sms, (r.M * r.Nc + 127) / 128, cgrid, csmem);
         lfd::CrtParams cp{res, nullptr, nullptr, 0, 0, 0, 0, 0, 0, linfo, rinfo, r.C, r.ldc, r.M, r.Nc, r.subtract ? 1 : 0, r.lower ? 1 : 0, err, plan,
-                          static_cast<uint32_t*>(r.sf.p)};
+                          static_cast<uint32_t*>(r.sf.p), lfd::crt_pitch(r.M * r.Nc)};
         rk->crt(cp, cgrid, csmem, s);
         cuda_check(cudaGetLastError(), "reconstruction");
     }

@@ -82,10 +82,11 @@ template <int N> __global__ void __launch_bounds__(128) digits_kernel(DigitParam
 }
 
 // ---------------------------------------------------------------- 2. tcgen05 residue products
-// Output tiles of 128 x 64: the three accumulators take 192 of 256 allocated TMEM columns and two stages 96 KB, so two
+// Output tiles of 128 x 80: the three accumulators take 240 of 256 allocated TMEM columns and two stages 104 KB, so two
 // CTAs share an SM and one's epilogue runs under the other's loads and MMAs (a 128 x 128 tile fills TMEM and leaves
-// the tensor pipe idle during its epilogue: 33% active).
-constexpr int kTileM = 128, kTileN = 64, kTileK = 128;       // K tile in int8 elements = one 128-byte row
+// the tensor pipe idle during its epilogue: 33% active).  The operands' way from L2 then bounds the kernel (128 x 64 tiles: 8.5 TB/s
+// over 1024^3 products of 75 moduli, 0.435 ms), so the tile is the widest that leaves room for the second CTA (0.374 ms).
+constexpr int kTileM = 128, kTileN = 80, kTileK = 128;       // K tile in int8 elements = one 128-byte row
 constexpr int kKAlign = 32;                                   // planes hold K rounded up to one MMA step, not a whole tile
 constexpr int kStages = 2;
 constexpr int kTileABytes = kTileM * kTileK, kTileBBytes = kTileN * kTileK;
@@ -97,7 +98,7 @@ constexpr int kDigitThreads = 256;                            // digit planes: t
 constexpr int kCrtThreads = 256;                              // CRT column sums: the same lane sharing
 
 struct MmaParams {
-    u16* res;                               // [L][M][Nc] residues (0 <= r < m), times w_l mod m_l when weighted
+    u16* res;                               // L times [M][Nc] residues (0 <= r < m), times w_l mod m_l when weighted
     const ResTables* tab;
     u64 M, Nc, Kp;
     int lower;                              // skip tiles strictly above the diagonal (SYRK)
@@ -106,6 +107,7 @@ struct MmaParams {
     u32 poll_limit;                         // polls of a barrier wait before it gives up (0: kSpinLimit)
     int no_loads;                           // failure test only: the producer issues no loads, so the first wait runs out
     int weighted;                           // store t_l = r w_l mod m_l, the operand of the tensor-core CRT
+    u64 pitch;                              // residues from one modulus to the next, 0: M * Nc
 };
 
 __device__ __forceinline__ u32 smem_u32(const void* p) { return (u32)__cvta_generic_to_shared(p); }
@@ -158,12 +160,19 @@ __device__ __forceinline__ void tmem_ld32(u32 taddr, u32 (&r)[32]) {
                  : "r"(taddr));
 }
 
+__device__ __forceinline__ void tmem_ld16(u32 taddr, u32 (&r)[16]) {
+    asm volatile("tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]),
+                   "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
+                 : "r"(taddr));
+}
+
 #ifdef LF_RESIDUE_MMA_KERNEL
 // x mod m in [0, 2m) for any 32-bit x, rr = floor(2^32 / m).
 __device__ __forceinline__ u32 mod_lazy(u32 x, u32 m, u32 rr) { return x - __umulhi(x, rr) * m; }
-// One CTA = one 128 x 64 output tile of one modulus (grid z).  Warp 0 lane 0 issues TMA loads,
+// One CTA = one 128 x 80 output tile of one modulus (grid z).  Warp 0 lane 0 issues TMA loads,
 // warp 1 lane 0 issues the MMAs; then all eight warps reduce the accumulators: warp w reads TMEM lanes
-// 32 (w % 4) .. + 31 (rows) for the columns of half w / 4 and stores 32 residues of a row with four
+// 32 (w % 4) .. + 31 (rows) for every second group of 16 columns and stores 16 residues of a row with two
 // 16-byte stores when the row stride allows.  The planes end at K rounded up to one MMA step of 32; the last
 // K tile's rows beyond it are zeros that the TMA load fills in, and no MMA reads them.
 __global__ void __launch_bounds__(kMmaThreads, 2) residue_mma_kernel(const __grid_constant__ CUtensorMap ta1, const __grid_constant__ CUtensorMap ta0,
@@ -257,18 +266,19 @@ __global__ void __launch_bounds__(kMmaThreads, 2) residue_mma_kernel(const __gri
         const u64 row = (u64)tm * kTileM + q * 32 + lane;
         const u32 lane_base = (u32)(q * 32) << 16;
         const bool vec = (p.Nc & 7) == 0;                      // rows start on 16-byte boundaries
-        for (int c0 = half * (kTileN / 2); c0 < (half + 1) * (kTileN / 2); c0 += 32) {
-            u32 s11[32], s00[32], sm[32];
-            tmem_ld32(acc11 + lane_base + c0, s11);
-            tmem_ld32(acc00 + lane_base + c0, s00);
-            tmem_ld32(accm + lane_base + c0, sm);
+        const u64 pitch = p.pitch ? p.pitch : p.M * p.Nc;
+        for (int c0 = half * 16; c0 < kTileN; c0 += 32) {
+            u32 s11[16], s00[16], sm[16];
+            tmem_ld16(acc11 + lane_base + c0, s11);
+            tmem_ld16(acc00 + lane_base + c0, s00);
+            tmem_ld16(accm + lane_base + c0, sm);
             asm volatile("tcgen05.wait::ld.sync.aligned;");
             if (row < p.M) {
                 const u64 col0 = (u64)tn * kTileN + c0;
-                u16* out = p.res + ((u64)l * p.M + row) * p.Nc + col0;
-                u32 r[32];
+                u16* out = p.res + (u64)l * pitch + row * p.Nc + col0;
+                u32 r[16];
 #pragma unroll
-                for (int c = 0; c < 32; ++c) {
+                for (int c = 0; c < 16; ++c) {
                     // 65536 S11 + 256 Smid + S00 by Horner's rule in 32-bit words: every mod_lazy leaves [0, 2m), 2m < 2^17
                     const u32 hi = mod_lazy(s11[c] + off30, m, rr) * 256u + mod_lazy(sm[c] + off31, m, rr);
                     const u32 x = mod_lazy(hi, m, rr) * 256u + (s00[c] + off30);
@@ -277,15 +287,15 @@ __global__ void __launch_bounds__(kMmaThreads, 2) residue_mma_kernel(const __gri
                     t = mod_lazy(t * w, m, rr);
                     r[c] = min(t, t - m);
                 }
-                if (vec && col0 + 32 <= p.Nc) {
+                if (vec && col0 + 16 <= p.Nc) {
                     uint4* o = reinterpret_cast<uint4*>(out);
 #pragma unroll
-                    for (int v = 0; v < 4; ++v)
+                    for (int v = 0; v < 2; ++v)
                         o[v] = make_uint4(r[8 * v] | (r[8 * v + 1] << 16), r[8 * v + 2] | (r[8 * v + 3] << 16),
                                           r[8 * v + 4] | (r[8 * v + 5] << 16), r[8 * v + 6] | (r[8 * v + 7] << 16));
                 } else {
 #pragma unroll
-                    for (int c = 0; c < 32; ++c)
+                    for (int c = 0; c < 16; ++c)
                         if (col0 + c < p.Nc) out[c] = (u16)r[c];
                 }
             }
@@ -584,8 +594,10 @@ template <int N> __global__ void __launch_bounds__(128) reconstruct_kernel(RecPa
 // (shifted) bytes, uploaded once per modulus count already in the 128-byte-swizzled K-major layout
 // of shared memory.  Each P[b] is below 2L * 255^2 < 2^25, so the int32 accumulators are exact.  One
 // CTA computes 128 outputs per tile and is persistent over the tiles:
-//   - eight warps copy the rows of A from the t_l that the residue products stored, two moduli a shared store,
-//     warps q and q + 4 taking alternate groups of 16 moduli of the same rows;
+//   - the t_l that the residue products stored (16 bytes of one modulus at a time, its residues on a 16-byte boundary) arrive
+//     while the tile before is carried; eight warps then write the rows of A, eight moduli a shared store, warps q and q + 4
+//     taking alternate groups of eight moduli of the same rows.  Loaded when their tile began, 16 at a time, the t_l
+//     left the warps waiting on memory (1024^2 outputs of 75 moduli: 0.284 ms, staged 0.136);
 //   - one thread issues tcgen05.mma kind::i8 (u8 x u8 -> s32, M = 128, N <= 256 per instruction)
 //     into TMEM;
 //   - warps q and q + 4 read the same TMEM lanes and carry the byte columns of the lower and of the upper words into
@@ -610,7 +622,12 @@ __host__ __device__ __forceinline__ int crt_split_word(int qwords) {
     return 8 * (chunks < 2 ? chunks : (chunks + 2) / 2);
 }
 __device__ __forceinline__ void mma_i8_u(u32 d_tmem, u64 a, u64 b, u32 idesc, bool accumulate) {
+    u64 pitch;                             // residues of a modulus in res: M * Nc rounded up to 8
     asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
+__host__ __device__ constexpr u64 crt_pitch(u64 outputs) { return (outputs + 7) / 8 * 8; }
+__host__ __device__ constexpr size_t crt_smem_bytes(int Kp, int NB, int L) {
+    return 1024 + (size_t)((Kp + 127) / 128) * (16384 + (size_t)NB * 128) + (size_t)L * 256;
+}
                  "tcgen05.mma.cta_group::1.kind::i8 [%0], %1, %2, %3, {%5, %5, %5, %5}, p;\n\t}"
                  :: "r"(d_tmem), "l"(a), "l"(b), "r"(idesc), "r"((u32)accumulate), "r"(0u));
 }
@@ -643,6 +660,7 @@ template <int N> __global__ void __launch_bounds__(kCrtThreads, 2) crt_mma_kerne
     for (u32 o = threadIdx.x * 16u; o < (u32)kblocks * 16384u; o += blockDim.x * 16u)      // bytes beyond 2 L stay zero
         *reinterpret_cast<uint4*>(sA + o) = make_uint4(0, 0, 0, 0);
     if (threadIdx.x == 0) {
+    u16* sR = reinterpret_cast<u16*>(sB + kblocks * p.NB * 128);     // [L][128 outputs]
         mbar_init(&done, 1);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
@@ -659,30 +677,39 @@ template <int N> __global__ void __launch_bounds__(kCrtThreads, 2) crt_mma_kerne
     const u32 id1 = (2u << 4) | ((u32)(N1 >> 3) << 17) | ((u32)(128 >> 4) << 24);
     const u32 id2 = (2u << 4) | ((u32)(N2 >> 3) << 17) | ((u32)(128 >> 4) << 24);
     const u64 outputs = p.M * p.Nc, tiles = (outputs + 127) / 128;
-    // Warps q and q + 4 stage alternate groups of 16 moduli of the same 128 rows; warps 0-3 then carry the
-    // byte columns of their TMEM lanes 32 q .. into S and F.
+    // Warps q and q + 4 share the rows of A and the TMEM lanes 32 q ..
     const int half = warp >> 2;
     const u32 row = (u32)((warp & 3) * 32 + (threadIdx.x & 31)), lane_base = (u32)((warp & 3) * 32) << 16;
-    u32 phase = 0;
-    for (u64 tile = blockIdx.x; tile < tiles; tile += gridDim.x) {
-        if (p.lower) {                                         // a tile inside one row, wholly above the diagonal
-            const u64 o0 = tile * 128, o1 = (o0 + 127 < outputs ? o0 + 127 : outputs - 1);
-            if (o0 / p.Nc == o1 / p.Nc && o0 % p.Nc > o0 / p.Nc) continue;
+    auto following = [&](u64 t) {                              // the next tile from t on that is not wholly above the diagonal
+        while (p.lower && t < tiles) {
+            const u64 o0 = t * 128, o1 = (o0 + 127 < outputs ? o0 + 127 : outputs - 1);
+            if (o0 / p.Nc != o1 / p.Nc || o0 % p.Nc <= o0 / p.Nc) break;
+            t += gridDim.x;
         }
         const u64 o = tile * 128 + row;
         const bool valid = o < outputs;
-        const u16* src = p.res + o;
-        for (int l0 = half * 16; l0 < p.L; l0 += 32) {          // row of A: t_l as two bytes; 16 loads in flight
-            u32 t[16];
-#pragma unroll
-            for (int q = 0; q < 16; ++q) t[q] = (valid && l0 + q < p.L) ? __ldg(src + (u64)(l0 + q) * outputs) : 0u;
-            unsigned char* base = sA + (l0 >> 6) * 16384u;
-            const u32 k0 = 2u * (l0 & 63);
-#pragma unroll
-            for (int q = 0; q < 16; q += 2) {
-                if (l0 + q >= p.L) break;
-                *reinterpret_cast<u32*>(base + sw128_offset(row, k0 + 2u * q)) = t[q] | (t[q + 1] << 16);
+        for (int l0 = half * 8; l0 < p.L; l0 += 16) {           // row of A: t_l as two bytes
+            u32 t[8];
+        return t;
+    };
+    auto stage = [&](u64 t) {
+        if (t < tiles)
+            for (int x = threadIdx.x; x < p.L * 16; x += kCrtThreads) {
+                const u64 at = t * 128 + 8 * (x & 15);
+                if (at < outputs) cp_async16(sR + (x >> 4) * 128 + 8 * (x & 15), p.res + (u64)(x >> 4) * p.pitch + at);
             }
+        cp_async_commit();
+    };
+    u32 phase = 0;
+    u64 tile = following(blockIdx.x);
+    stage(tile);
+    cp_async_wait<0>();
+    __syncthreads();
+    while (tile < tiles) {
+#pragma unroll
+            for (int q = 0; q < 8; ++q) t[q] = l0 + q < p.L ? sR[(l0 + q) * 128 + row] : 0u;
+            *reinterpret_cast<uint4*>(sA + (l0 >> 6) * 16384u + sw128_offset(row, 2u * (l0 & 63))) =
+                make_uint4(t[0] | (t[1] << 16), t[2] | (t[3] << 16), t[4] | (t[5] << 16), t[6] | (t[7] << 16));
         }
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");   // generic writes -> tensor core reads
         __syncthreads();
@@ -707,6 +734,8 @@ template <int N> __global__ void __launch_bounds__(kCrtThreads, 2) crt_mma_kerne
         const int split = crt_split_word(p.qwords), chunks = p.qwords / 8;     // 8-word chunks wholly inside S
         u32* dst = p.sf + o;
         u64 acc = 0;
+        const u64 next = following(tile + gridDim.x);
+        stage(next);                                            // every thread has read sR
         for (int ch = half ? split / 8 : 0; ch < (half ? chunks : split / 8); ++ch) {
             u32 P[32];
             tmem_ld32(tmem + lane_base + (u32)ch * 32u, P);
@@ -745,7 +774,9 @@ template <int N> __global__ void __launch_bounds__(kCrtThreads, 2) crt_mma_kerne
             }
         }
         asm volatile("tcgen05.fence::before_thread_sync;");
-        __syncthreads();                                        // TMEM and A are free for the next tile
+        cp_async_wait<0>();
+        __syncthreads();                                        // TMEM and A are free for the next tile, whose residues are here
+        tile = next;
     }
     asm volatile("tcgen05.fence::before_thread_sync;");
     __syncthreads();
@@ -756,6 +787,7 @@ template <int N> __global__ void __launch_bounds__(kCrtThreads, 2) crt_mma_kerne
 // X mod m_l for all L moduli as two unsigned int8 GEMMs: with x_b the bytes of X (4 xwords of them) and
 // 2^(8b) mod m_l = 256 th + tl, P0 = [tl] x [x bytes] and P1 = [th] x [x bytes] give
 // X == P0 + 256 P1 (mod m_l), each P below 160 * 255^2 < 2^24.  The moduli are the rows (TMEM lanes) and 128 padded
+    cp_async_wait<0>();
 // entries (line, k) in plane order the columns: a thread then has its modulus in registers and 32 consecutive entries
 // of one plane, whose digits it packs and stores as 32 bytes.  With entries as rows every digit was a store of
 // its own byte and every residue two shared loads of its modulus (0.21 ms for 1024^2 512-bit entries).  Up to 64 (32)

@@ -1,5 +1,5 @@
 """GPU: the residue engine at the edges of its tiles and tables, bit for bit against the limb kernel on the same data:
-inner dimensions around one MMA step (32) and one K tile (128), output sizes around the 128 x 64 tile, modulus counts on both
+inner dimensions around one MMA step (32) and one K tile (128), output sizes around the 128 x 80 tile, modulus counts on both
 sides of the digit table's copies (32 and 64) and of its second row tile (128), and old entries far above and far below the
 product, which the rounding cannot take in one pass."""
 import numpy as np
@@ -12,9 +12,9 @@ pytestmark = pytest.mark.gpu
 
 
 @pytest.mark.parametrize("bits,m,n,k,span,lo,hi", [
-    (64, 63, 64, 1, 4, 8, 16), (128, 65, 129, 31, 10, 17, 32), (192, 128, 63, 32, 8, 25, 32), (224, 127, 65, 33, 40, 33, 64),
-    (256, 129, 130, 127, 20, 33, 64), (448, 64, 64, 128, 20, 57, 64), (512, 100, 70, 129, 40, 65, 128),
-    (1024, 66, 130, 160, 2, 129, 160), (1024, 33, 35, 40, 60, 129, 160)])
+    (64, 63, 64, 1, 4, 8, 16), (128, 65, 129, 31, 10, 17, 32), (192, 128, 79, 32, 8, 25, 32), (224, 127, 65, 33, 40, 33, 64),
+    (256, 129, 130, 127, 20, 33, 64), (448, 64, 80, 128, 20, 57, 64), (512, 100, 81, 129, 40, 65, 128),
+    (1024, 66, 161, 160, 2, 129, 160), (1024, 33, 35, 40, 60, 129, 160)])
 def test_tile_and_table_edges(engine, bits, m, n, k, span, lo, hi):
     rng = np.random.default_rng(bits + k)
     residue, limb = (api.Linalg(engine, api.LinalgOptions(method=x)) for x in (2, 1))
