@@ -613,7 +613,12 @@ struct CrtParams {
     const ResPlan* plan;                   // planned on the GPU: L and its operand come from the plan
     u32* sf;                               // S (qwords + 2 words), F (2 words) and the carry into word crt_split_word of
                                            // S, word-major (word w of output o at sf[w * M * Nc + o])
+    u64 pitch;                             // residues of a modulus in res: M * Nc rounded up to 8
 };
+__host__ __device__ constexpr u64 crt_pitch(u64 outputs) { return (outputs + 7) / 8 * 8; }
+__host__ __device__ constexpr size_t crt_smem_bytes(int Kp, int NB, int L) {
+    return 1024 + (size_t)((Kp + 127) / 128) * (16384 + (size_t)NB * 128) + (size_t)L * 256;
+}
 constexpr int kCrtExtraWords = 5;          // words of an output in sf beyond qwords
 // S words below this one are carried by warps 0-3, the others by warps 4-7: whole 32-column chunks, the larger part below
 // (the chunk with F and the last words costs more).
@@ -622,12 +627,7 @@ __host__ __device__ __forceinline__ int crt_split_word(int qwords) {
     return 8 * (chunks < 2 ? chunks : (chunks + 2) / 2);
 }
 __device__ __forceinline__ void mma_i8_u(u32 d_tmem, u64 a, u64 b, u32 idesc, bool accumulate) {
-    u64 pitch;                             // residues of a modulus in res: M * Nc rounded up to 8
     asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
-__host__ __device__ constexpr u64 crt_pitch(u64 outputs) { return (outputs + 7) / 8 * 8; }
-__host__ __device__ constexpr size_t crt_smem_bytes(int Kp, int NB, int L) {
-    return 1024 + (size_t)((Kp + 127) / 128) * (16384 + (size_t)NB * 128) + (size_t)L * 256;
-}
                  "tcgen05.mma.cta_group::1.kind::i8 [%0], %1, %2, %3, {%5, %5, %5, %5}, p;\n\t}"
                  :: "r"(d_tmem), "l"(a), "l"(b), "r"(idesc), "r"((u32)accumulate), "r"(0u));
 }
@@ -651,6 +651,7 @@ template <int N> __global__ void __launch_bounds__(kCrtThreads, 2) crt_mma_kerne
     const int kblocks = p.Kp / 128 + (p.Kp % 128 ? 1 : 0);
     unsigned char* sA = smem;                                  // kblocks x [128 rows][128 B]
     unsigned char* sB = smem + kblocks * 16384;                // kblocks x [NB rows][128 B]
+    u16* sR = reinterpret_cast<u16*>(sB + kblocks * p.NB * 128);     // [L][128 outputs]
     __shared__ __align__(8) u64 done;
     __shared__ u32 tmem_slot;
     const int warp = threadIdx.x >> 5;
@@ -660,7 +661,6 @@ template <int N> __global__ void __launch_bounds__(kCrtThreads, 2) crt_mma_kerne
     for (u32 o = threadIdx.x * 16u; o < (u32)kblocks * 16384u; o += blockDim.x * 16u)      // bytes beyond 2 L stay zero
         *reinterpret_cast<uint4*>(sA + o) = make_uint4(0, 0, 0, 0);
     if (threadIdx.x == 0) {
-    u16* sR = reinterpret_cast<u16*>(sB + kblocks * p.NB * 128);     // [L][128 outputs]
         mbar_init(&done, 1);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
@@ -686,10 +686,6 @@ template <int N> __global__ void __launch_bounds__(kCrtThreads, 2) crt_mma_kerne
             if (o0 / p.Nc != o1 / p.Nc || o0 % p.Nc <= o0 / p.Nc) break;
             t += gridDim.x;
         }
-        const u64 o = tile * 128 + row;
-        const bool valid = o < outputs;
-        for (int l0 = half * 8; l0 < p.L; l0 += 16) {           // row of A: t_l as two bytes
-            u32 t[8];
         return t;
     };
     auto stage = [&](u64 t) {
@@ -706,6 +702,10 @@ template <int N> __global__ void __launch_bounds__(kCrtThreads, 2) crt_mma_kerne
     cp_async_wait<0>();
     __syncthreads();
     while (tile < tiles) {
+        const u64 o = tile * 128 + row;
+        const bool valid = o < outputs;
+        for (int l0 = half * 8; l0 < p.L; l0 += 16) {           // row of A: t_l as two bytes
+            u32 t[8];
 #pragma unroll
             for (int q = 0; q < 8; ++q) t[q] = l0 + q < p.L ? sR[(l0 + q) * 128 + row] : 0u;
             *reinterpret_cast<uint4*>(sA + (l0 >> 6) * 16384u + sw128_offset(row, 2u * (l0 & 63))) =
@@ -725,6 +725,8 @@ template <int N> __global__ void __launch_bounds__(kCrtThreads, 2) crt_mma_kerne
             }
             mma_commit(&done);
         }
+        const u64 next = following(tile + gridDim.x);
+        stage(next);                                            // every thread has read sR
         const bool fine = __syncthreads_and(mbar_wait(&done, phase, p.error));
         phase ^= 1u;
         asm volatile("tcgen05.fence::after_thread_sync;");
@@ -734,8 +736,6 @@ template <int N> __global__ void __launch_bounds__(kCrtThreads, 2) crt_mma_kerne
         const int split = crt_split_word(p.qwords), chunks = p.qwords / 8;     // 8-word chunks wholly inside S
         u32* dst = p.sf + o;
         u64 acc = 0;
-        const u64 next = following(tile + gridDim.x);
-        stage(next);                                            // every thread has read sR
         for (int ch = half ? split / 8 : 0; ch < (half ? chunks : split / 8); ++ch) {
             u32 P[32];
             tmem_ld32(tmem + lane_base + (u32)ch * 32u, P);
@@ -778,6 +778,7 @@ template <int N> __global__ void __launch_bounds__(kCrtThreads, 2) crt_mma_kerne
         __syncthreads();                                        // TMEM and A are free for the next tile, whose residues are here
         tile = next;
     }
+    cp_async_wait<0>();
     asm volatile("tcgen05.fence::before_thread_sync;");
     __syncthreads();
     if (warp == 0) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" :: "r"(tmem), "r"(p.tmem_cols));
@@ -787,7 +788,6 @@ template <int N> __global__ void __launch_bounds__(kCrtThreads, 2) crt_mma_kerne
 // X mod m_l for all L moduli as two unsigned int8 GEMMs: with x_b the bytes of X (4 xwords of them) and
 // 2^(8b) mod m_l = 256 th + tl, P0 = [tl] x [x bytes] and P1 = [th] x [x bytes] give
 // X == P0 + 256 P1 (mod m_l), each P below 160 * 255^2 < 2^24.  The moduli are the rows (TMEM lanes) and 128 padded
-    cp_async_wait<0>();
 // entries (line, k) in plane order the columns: a thread then has its modulus in registers and 32 consecutive entries
 // of one plane, whose digits it packs and stores as 32 bytes.  With entries as rows every digit was a store of
 // its own byte and every residue two shared loads of its modulus (0.21 ms for 1024^2 512-bit entries).  Up to 64 (32)
