@@ -966,31 +966,18 @@ template <int N> __device__ __noinline__ Num<N> crt_tail_call(const u32* S, int 
     for (int w = 0; w < qwords + 2; ++w) X[w] = S[w];
     return crt_tail<N>(X, qwords, F, tab, scale, subtract, c, scratch);
 }
-template <int N> __global__ void __launch_bounds__(kCrtRoundThreads) crt_round_kernel(const CrtParams pin) {
-    CrtParams p = pin;
-    if (pin.plan) {
-        if (pin.plan->mode != 1) return;
-        p.tab = static_cast<const ResTables*>(pin.plan->tab); p.qwords = pin.plan->qwords;
-    }
-    extern __shared__ u32 crt_round_park[];
-    __shared__ u32 s_M[kResMaxQWords + 2];
+// One output: leaves its entry in T and returns whether there is one to write.  The words of S are loaded eight ahead of the pass
+// (one a step left it waiting on memory: 1024^2 outputs at 512 bits took 0.217 ms, with this and the coalesced writes 0.146).
+template <int N> __device__ __forceinline__ bool crt_round_one(const CrtParams& p, const u32* s_M, u64 o, u64 i, u64 j, u32* T, const u32* out) {
     const int xw = p.qwords + 2;
-    for (int w = threadIdx.x; w < xw; w += kCrtRoundThreads) s_M[w] = w <= p.qwords ? p.tab->M[w] : 0u;
-    __syncthreads();
-    const u64 outputs = p.M * p.Nc, o = (u64)blockIdx.x * kCrtRoundThreads + threadIdx.x;
-    if (o >= outputs) return;
-    const u64 i = o / p.Nc, j = o % p.Nc;
-    if (p.lower && j > i) return;
-    constexpr u64 E = N + 3;
-    u32* out = p.C + (i * p.ldc + j) * E;
+    const u64 outputs = p.M * p.Nc;
     const LineInfo li = p.linfo[i], ri = p.rinfo[j];
     int ce = 0, cs = 0;
     u32 cst = 0;
     if (p.subtract) { ce = (int)out[N]; cs = (int)out[N + 1]; cst = out[N + 2]; }
     const u32 st = cst | li.status | ri.status;
-    if (st) { store<N>(out, zero<N>(st)); return; }
-    if (!li.nonzero || !ri.nonzero) { if (!p.subtract) store<N>(out, zero<N>()); return; }      // C stays
-    u32* T = crt_round_park + threadIdx.x * crt_round_words(p.qwords);
+    if (st) { store<N>(T, zero<N>(st)); return true; }
+    if (!li.nonzero || !ri.nonzero) { store<N>(T, zero<N>()); return !p.subtract; }      // C stays
     const u32* sf = p.sf + o;
     const u64 F = (u64)sf[(u64)(p.qwords + 2) * outputs] | ((u64)sf[(u64)(p.qwords + 3) * outputs] << 32);
     const int split = crt_split_word(p.qwords);
@@ -1003,8 +990,8 @@ template <int N> __global__ void __launch_bounds__(kCrtRoundThreads) crt_round_k
             const u64 v = (u64)sf[(u64)w * outputs] + (w == split ? up : 0u) + cy;
             T[w] = (u32)v; cy = v >> 32;
         }
-        store<N>(out, crt_tail_call<N>(T, p.qwords, F, p.tab, scale, true, load_plain<N>(out)));
-        return;
+        store<N>(T, crt_tail_call<N>(T, p.qwords, F, p.tab, scale, true, load_plain<N>(out)));
+        return true;
     }
     // T = S - q M - c (two's complement); without an old entry T = X
     const u32 q = (u32)((F + (1ull << 47)) >> 48);              // round(F) <= L: X = S - q M
@@ -1013,26 +1000,32 @@ template <int N> __global__ void __launch_bounds__(kCrtRoundThreads) crt_round_k
     u64 cy = 0, qm = 0, ca = mask & 1u;
     u32 prev = 0, low = 0xffffffffu;                              // lowest nonzero word of T
     int borrow = 0;
-    for (int w = 0; w < xw; ++w) {
-        const u64 sv = (u64)sf[(u64)w * outputs] + (w == split ? up : 0u) + cy;
-        cy = sv >> 32;
-        qm += (u64)s_M[w] * q;
-        const i64 d = (i64)(sv & 0xffffffffull) - (i64)(qm & 0xffffffffull) - borrow;
-        qm >>= 32;
-        borrow = d < 0;
-        u32 cur = 0, add = 0;
-        const int k = w - ws;
-        if (k >= 0 && k <= N) {
-            if (k < N) cur = out[k];
-            add = __funnelshift_l(prev, cur, bs);
-            prev = cur;
+    for (int w0 = 0; w0 < xw; w0 += 8) {
+        u32 sw[8], cw[8];
+#pragma unroll
+        for (int x = 0; x < 8; ++x) {
+            sw[x] = w0 + x < xw ? __ldg(sf + (u64)(w0 + x) * outputs) : 0u;
+            cw[x] = (u32)(w0 + x - ws) < (u32)N ? out[w0 + x - ws] : 0u;
         }
-        const u64 v = (u64)(u32)d + (add ^ mask) + ca;
-        ca = v >> 32;
-        T[w] = (u32)v;
-        if ((u32)v && low == 0xffffffffu) low = (u32)w;
+#pragma unroll
+        for (int x = 0; x < 8; ++x) {
+            const int w = w0 + x;
+            if (w >= xw) break;
+            const u64 sv = (u64)sw[x] + (w == split ? up : 0u) + cy;
+            cy = sv >> 32;
+            qm += (u64)s_M[w] * q;
+            const i64 d = (i64)(sv & 0xffffffffull) - (i64)(qm & 0xffffffffull) - borrow;
+            qm >>= 32;
+            borrow = d < 0;
+            const u32 add = __funnelshift_l(prev, cw[x], bs);     // zero outside words [ws, ws + N]
+            prev = cw[x];
+            const u64 v = (u64)(u32)d + (add ^ mask) + ca;
+            ca = v >> 32;
+            T[w] = (u32)v;
+            if ((u32)v && low == 0xffffffffu) low = (u32)w;
+        }
     }
-    if (low == 0xffffffffu) { store<N>(out, zero<N>()); return; }
+    if (low == 0xffffffffu) { store<N>(T, zero<N>()); return true; }
     const bool neg = T[xw - 1] >> 31;
     auto mag = [&](int w) -> u32 {                                // word w of |T|
         if (w < (int)low) return 0u;
@@ -1052,7 +1045,36 @@ template <int N> __global__ void __launch_bounds__(kCrtRoundThreads) crt_round_k
     const u32 next = mag(t - N - 1), g = __funnelshift_l(next, hi, lz);
     const bool sticky = (g & 0x7fffffffu) || (next << lz) || (int)low < t - N - 1;
     // subtract: the result is c - X = -T
-    store<N>(out, finish<N>(m, scale + 32 * (i64)t + 31 - lz, neg != (p.subtract != 0) ? -1 : 1, (g >> 31) && (sticky || (m[0] & 1u)), 0));
+    store<N>(T, finish<N>(m, scale + 32 * (i64)t + 31 - lz, neg != (p.subtract != 0) ? -1 : 1, (g >> 31) && (sticky || (m[0] & 1u)), 0));
+    return true;
+}
+template <int N> __global__ void __launch_bounds__(kCrtRoundThreads) crt_round_kernel(const CrtParams pin) {
+    CrtParams p = pin;
+    if (pin.plan) {
+        if (pin.plan->mode != 1) return;
+        p.tab = static_cast<const ResTables*>(pin.plan->tab); p.qwords = pin.plan->qwords;
+    }
+    extern __shared__ u32 crt_round_park[];
+    __shared__ u32 s_M[kResMaxQWords + 2];
+    const int xw = p.qwords + 2;
+    for (int w = threadIdx.x; w < xw; w += kCrtRoundThreads) s_M[w] = w <= p.qwords ? p.tab->M[w] : 0u;
+    __syncthreads();
+    const u64 outputs = p.M * p.Nc, o = (u64)blockIdx.x * kCrtRoundThreads + threadIdx.x;
+    const u64 i = o / p.Nc, j = o % p.Nc;
+    constexpr u64 E = N + 3;
+    u32* out = p.C + (i * p.ldc + j) * E;
+    u32* T = crt_round_park + threadIdx.x * crt_round_words(p.qwords);
+    const bool put = o < outputs && !(p.lower && j > i) && crt_round_one<N>(p, s_M, o, i, j, T, out);
+    // a warp writes its 32 entries word by word, neighbouring words to neighbouring lanes
+    const u32 live = __ballot_sync(0xffffffffu, put);
+    if (!live) return;                                           // the whole warp: above the diagonal, or beyond the outputs
+    const u32 lane = threadIdx.x & 31;
+    const u32* rows = T - lane * crt_round_words(p.qwords);
+    for (u32 w = lane; w < 32 * E; w += 32) {
+        const u32 r = w / (u32)E, x = w - r * (u32)E;
+        u32* to = reinterpret_cast<u32*>(__shfl_sync(0xffffffffu, reinterpret_cast<unsigned long long>(out), r));
+        if ((live >> r) & 1u) to[x] = rows[r * crt_round_words(p.qwords) + x];
+    }
 }
 
 typedef void (*DigitFn)(const DigitParams&, cudaStream_t);
