@@ -7,6 +7,7 @@
 #include "lf_linalg.cuh"
 #include "lf_residue.h"
 #include "lf_residue.cuh"
+#include "lf_longdot.cuh"
 #include "lf_qr.cuh"
 #include "lf_cqr.cuh"
 
@@ -81,16 +82,27 @@ void exact_product_on(Linalg& la, const ProductLane& lane, int bits, lfd::LineVi
     if (method != 1 && !la.options.force_fallback)
         used_residue = lane.residue->run(bits, left, right, M, Nc, K, C, ldc, subtract, lower, err, s, method == 2, la.report);
     if (!used_residue) {
-        // the tiled limb kernel: line analysis, then one exact window per output (cluster method for wide outputs)
         lfd::WinParams wp{};
         lfd::DotParams& p = wp.d;
         p.left = left; p.right = right; p.C = C; p.ldc = ldc; p.M = M; p.Nc = Nc; p.K = K;
         p.row0 = 0; p.col0 = 0; p.subtract = subtract; p.lower = lower; p.error = err;
-        auto* linfo = static_cast<lfd::LineInfo*>(lane.lines->get(sizeof(lfd::LineInfo) * (M + Nc) + 64));
-        lfd::linalg_kernels(n)->analyze(left, M, K, linfo, s);
-        lfd::linalg_kernels(n)->analyze(right, Nc, K, linfo + M, s);
-        wp.linfo = linfo; wp.rinfo = linfo + M;
-        lfd::residue_kernels(n)->window_dot(wp, s);
+        // a refused engine has analysed the lines: their widest spread says whether the block's window holds the products
+        const bool seen = method != 1 && !la.options.force_fallback && lane.residue->left_info;
+        wp.spread = seen ? lane.residue->spread : -1;
+        if (lfd::long_dot_fits(n, M, Nc, K, wp.spread)) {
+            lfd::long_dot_launcher(n)(p, s);                   // few outputs, long sums: a block per output
+        } else {
+            // the tiled limb kernel: line analysis, then one exact window per output (cluster method for wide outputs)
+            if (seen) {
+                wp.linfo = lane.residue->left_info; wp.rinfo = lane.residue->right_info;
+            } else {
+                auto* linfo = static_cast<lfd::LineInfo*>(lane.lines->get(sizeof(lfd::LineInfo) * (M + Nc) + 64));
+                lfd::linalg_kernels(n)->analyze(left, M, K, linfo, s);
+                lfd::linalg_kernels(n)->analyze(right, Nc, K, linfo + M, s);
+                wp.linfo = linfo; wp.rinfo = linfo + M;
+            }
+            lfd::residue_kernels(n)->window_dot(wp, s);
+        }
         cuda_check(cudaGetLastError(), "exact product launch");
     }
     if (method_used) *method_used = used_residue ? 2 : 1;

@@ -211,6 +211,7 @@ bool ResidueEngine::run(int bits, lfd::LineView left, lfd::LineView right, uint6
         if (forced) throw runtime_error(std::string("residue engine: ") + why);
         return false;
     };
+    left_info = right_info = nullptr; spread = -1;
     if (!K) return refuse("empty inner dimension");
     if (K > kMaxK) return refuse("inner dimension above 65472");
     const bool same = left.base == right.base && left.ls == right.ls && left.ks == right.ks && M == Nc;
@@ -233,6 +234,7 @@ bool ResidueEngine::run(int bits, lfd::LineView left, lfd::LineView right, uint6
         if (i < M) (live ? report.left_lines : report.left_zero_lines) += 1;
         if (i >= M || same) (live ? report.right_lines : report.right_zero_lines) += 1;
     }
+    left_info = linfo; right_info = rinfo; spread = G;
     if (!any) return refuse("no nonzero lines");
     if (G > kMaxBand) return refuse("a line spans more than 192 exponent bits");
     const int P = 32 * n + G;

@@ -443,14 +443,20 @@ template <int N> __device__ __forceinline__ Num<N> crt_tail(u32* S, int qwords, 
 // stages the 8 + 8 lines' next kWinTK entries in shared memory, so each entry is read from memory once per tile
 // instead of once per output; the column sums live in shared memory (one row per thread, an odd number of 64-bit
 // words apart).
+// The window has p.words words: win_words(N) for lines whose spread is not known or narrow, up to win_max_words(N) where
+// the host saw it (each word more costs a block 512 bytes of shared memory, two passes over a word an output, and at
+// 1024 bits the widest window still leaves two blocks an SM); the cluster method costs each output some six passes over
+// its terms' exponents in memory and one lane's sums in local memory (178 x 226 x 47 at 192 bits and exponents of +-185:
+// 0.64 ms by clusters, 0.14 ms in wide windows; 250 x 280 x 250 at 736 bits: 61.7 and 4.0).
 constexpr int kWinTM = 8, kWinTN = 8, kWinThreads = kWinTM * kWinTN, kWinTK = 8;
 template <int N> __host__ __device__ constexpr int win_words() { return 2 * N + 8; }
 // Row of one thread: W + 1 64-bit column sums (the sum's sign in the last), later the window (round_sum2's scratch is
 // thread-local, used once per output); the row is an odd number of 64-bit words long.
-template <int N> __host__ __device__ constexpr int win_row_words() { return 2 * ((win_words<N>() + 1) | 1); }
+__host__ __device__ constexpr int win_row_words(int words) { return 2 * ((words + 1) | 1); }
+template <int N> __host__ __device__ constexpr int win_max_words() { return 2 * N + 64; }
 constexpr unsigned long long kWinMaxK = 1ull << 28;          // column sums of 32-bit words stay below 2^62
-template <int N> __host__ __device__ constexpr size_t win_smem_bytes() {
-    return (size_t)4 * ((kWinTM + kWinTN) * kWinTK * (N + 3) + kWinThreads * win_row_words<N>());
+template <int N> __host__ __device__ constexpr size_t win_smem_bytes(int words) {
+    return (size_t)4 * ((kWinTM + kWinTN) * kWinTK * (N + 3) + kWinThreads * win_row_words(words));
 }
 // col (len signed 64-bit column sums) +/-= t (TW words) << (32 ws + bs), one independent add per word
 template <int TW> __device__ __forceinline__ void win_add_cols(long long* col, int len, const u32 (&t)[TW], int ws, int bs, bool negative) {
@@ -465,15 +471,18 @@ template <int TW> __device__ __forceinline__ void win_add_cols(long long* col, i
 struct WinParams {
     DotParams d;                    // operands, output, modes, error word
     const LineInfo* linfo; const LineInfo* rinfo;   // analysis of the M left and Nc right lines
+    int spread = -1;                // the widest line's exponent spread where the host knows it, or -1
+    int words = 0;                  // of a window (set by the launch)
 };
 template <int N> __global__ void __launch_bounds__(kWinThreads) window_dot_kernel(const WinParams wp) {
     const DotParams& p = wp.d;
-    constexpr int E = N + 3, W = win_words<N>();
+    constexpr int E = N + 3;
+    const int W = wp.words;
     extern __shared__ __align__(16) u32 win_park[];
     u32* sA = win_park;                                  // [kWinTK][kWinTM] entries
     u32* sB = sA + kWinTK * kWinTM * E;                  // [kWinTK][kWinTN] entries
     const int t = threadIdx.x, r = t / kWinTN, q = t % kWinTN;
-    u32* row = sB + kWinTK * kWinTN * E + t * win_row_words<N>();
+    u32* row = sB + kWinTK * kWinTN * E + t * win_row_words(W);
     long long* col = reinterpret_cast<long long*>(row);  // W column sums; then the window
     const u64 r0 = (u64)blockIdx.y * kWinTM, q0 = (u64)blockIdx.x * kWinTN;
     const u64 ro = r0 + r, qo = q0 + q;                  // this thread's output (local row, column)
@@ -489,7 +498,7 @@ template <int N> __global__ void __launch_bounds__(kWinThreads) window_dot_kerne
     while ((1ull << logk) < p.K) ++logk;
     const i64 span = products ? (i64)(li.top - li.bottom) + (ri.top - ri.bottom) + 64 * N + logk : 0;
     const bool window = live && !st && products && span <= 32 * W && p.K < kWinMaxK;
-    constexpr int W1 = W + 1;                            // one more column for the sign of the signed sum
+    const int W1 = W + 1;                                // one more column for the sign of the signed sum
     if (window) for (int w = 0; w < W1; ++w) col[w] = 0;
     const int ebase = li.bottom + ri.bottom;
     // all threads stage the tiles (the barriers include threads without a window)
@@ -549,7 +558,7 @@ template <int N> __global__ void __launch_bounds__(kWinThreads) window_dot_kerne
         for (int w = 0; w < W1 && !cmp; ++w) if (X[w]) cmp = 1;
     }
     // round_sum2 adds the old entry c with its own sign (it computes RN(sign * X * 2^scale + c))
-    u32 scratch[round_sum2_words<N>(W1)];
+    u32 scratch[round_sum2_words<N>(win_max_words<N>() + 1)];
     store<N>(out, round_sum2<N>(X, W1, (i64)ebase - 2 * (32 * N - 1), cmp, c, scratch));
 }
 
@@ -1081,7 +1090,7 @@ typedef void (*DigitFn)(const DigitParams&, cudaStream_t);
 typedef void (*RecFn)(const RecParams&, cudaStream_t);
 typedef void (*CrtFn)(const CrtParams&, unsigned grid, size_t smem, cudaStream_t);
 typedef void (*DigitMmaFn)(const DigitMmaParams&, unsigned grid, size_t smem, cudaStream_t);
-typedef void (*WindowDotFn)(const WinParams&, cudaStream_t);
+typedef void (*WindowDotFn)(WinParams, cudaStream_t);
 struct ResidueKernels { DigitFn digits; RecFn rec; CrtFn crt; DigitMmaFn digits_mma; WindowDotFn window_dot; };
 const ResidueKernels* residue_kernels(int limbs);
 
@@ -1104,9 +1113,14 @@ template <int N> void digits_mma_launch(const DigitMmaParams& p, unsigned grid, 
     cudaFuncSetAttribute(digits_mma_kernel<N>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     digits_mma_kernel<N><<<grid, kDigitThreads, smem, s>>>(p);
 }
-template <int N> void window_dot_launch(const WinParams& p, cudaStream_t s) {
+template <int N> void window_dot_launch(WinParams p, cudaStream_t s) {
     if (!p.d.M || !p.d.Nc) return;
-    const size_t smem = win_smem_bytes<N>();
+    // a window for every output where the widest pair of lines fits one
+    int logk = 0;
+    while ((1ull << logk) < p.d.K) ++logk;
+    const i64 need = p.spread < 0 ? 0 : (2 * (i64)p.spread + 64 * N + logk + 31) / 32;
+    p.words = need <= win_words<N>() || need > win_max_words<N>() ? win_words<N>() : (int)need;
+    const size_t smem = win_smem_bytes<N>(p.words);
     if (smem > 48 * 1024) cudaFuncSetAttribute(window_dot_kernel<N>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     dim3 grid((unsigned)((p.d.Nc + kWinTN - 1) / kWinTN), (unsigned)((p.d.M + kWinTM - 1) / kWinTM));
     window_dot_kernel<N><<<grid, kWinThreads, smem, s>>>(p);

@@ -10,6 +10,10 @@ namespace lfr {
 
 struct ResidueEngine {
     DevBuf lines, planes, residues, tables, misc;
+    // What the last run() learned before it refused: the line analysis (in `lines`, the right one the left one's for a SYRK) and
+    // the widest line's exponent spread; null and -1 when it refused before the analysis.
+    const lfd::LineInfo *left_info = nullptr, *right_info = nullptr;
+    int spread = -1;
     size_t bytes() const { return lines.bytes + planes.bytes + residues.bytes + tables.bytes + misc.bytes; }
     void release() { lines = DevBuf{}; planes = DevBuf{}; residues = DevBuf{}; tables = DevBuf{}; misc = DevBuf{}; }
     bool run(int bits, lfd::LineView left, lfd::LineView right, uint64_t M, uint64_t Nc, uint64_t K, uint32_t* C,
