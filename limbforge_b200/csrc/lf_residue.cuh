@@ -1077,6 +1077,7 @@ template <int N> __global__ void __launch_bounds__(kCrtRoundThreads) crt_round_k
     // a warp writes its 32 entries word by word, neighbouring words to neighbouring lanes
     const u32 live = __ballot_sync(0xffffffffu, put);
     if (!live) return;                                           // the whole warp: above the diagonal, or beyond the outputs
+    __syncwarp();                                                // every lane's entry is in T: a vote orders no memory
     const u32 lane = threadIdx.x & 31;
     const u32* rows = T - lane * crt_round_words(p.qwords);
     for (u32 w = lane; w < 32 * E; w += 32) {
