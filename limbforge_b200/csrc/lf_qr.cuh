@@ -432,6 +432,7 @@ template <int N> __global__ void __launch_bounds__(32) qr_tcol_kernel(QrPanel p,
         last = atomicAdd(&p.st->arrivals, 1u) == gridDim.x - 1;
         if (last) p.st->arrivals = 0;
     }
+    __syncwarp();                                                  // the arrival comes before the lanes' reads: a shuffle orders no memory
     if (!__shfl_sync(0xffffffffu, last, 0) || (long long)c >= qn) return;
     __threadfence();
     y(c);
