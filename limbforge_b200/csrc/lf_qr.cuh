@@ -106,7 +106,7 @@ template <int N, bool RO> struct StridedPair {
 
 // RN(sum_{k<K} a_k b_k) with one rounding for the operands a_k, b_k that src gives, computed by the whole block
 // (qr_threads<N>() threads) and returned to every thread; the contract of exact_dot (statuses first; no nonzero product
-// gives zero).  Pass 1 reduces the statuses, the number of nonzero products and the range of their scales; each
+// gives zero).  Pass 1 reduces the statuses, whether any product is nonzero and the range of their scales; each
 // thread then adds its products into a two's-complement window anchored at the lowest scale, the warps sum their
 // windows with shuffles and thread 0 adds the warps' sums and rounds once.  A range wider than the window goes to
 // src.fallback (the cluster method) on thread 0.  sm: qr_dot_words<N>() words of shared memory, 8-byte aligned.
@@ -128,9 +128,9 @@ template <int N, class Src> __device__ __noinline__ Num<N> block_exact_sum(const
     long long* s_lo = reinterpret_cast<long long*>(s_part + PARTS * W);
     long long* s_hi = s_lo + WARPS;
     u32* s_st = reinterpret_cast<u32*>(s_hi + WARPS);
-    u32* s_cnt = s_st + WARPS;
-    u32* s_res = s_cnt + WARPS;                                      // N + 3 words
-    u32 st = 0, cnt = 0;
+    u32* s_any = s_st + WARPS;
+    u32* s_res = s_any + WARPS;                                      // N + 3 words
+    u32 st = 0, any = 0;
     long long lo = INT64_MAX, hi = INT64_MIN;
     for (u64 k = tid; k < K; k += T) {
         Num<N> a, b;
@@ -138,30 +138,30 @@ template <int N, class Src> __device__ __noinline__ Num<N> block_exact_sum(const
         st |= a.st | b.st;
         if (a.s && b.s) {
             const long long s = (long long)a.e + b.e - 2 * (32 * N - 1);
-            lo = s < lo ? s : lo; hi = s + 64 * N > hi ? s + 64 * N : hi; ++cnt;
+            lo = s < lo ? s : lo; hi = s + 64 * N > hi ? s + 64 * N : hi; any = 1;
         }
     }
 #pragma unroll
     for (int o = 16; o; o >>= 1) {
         st |= __shfl_xor_sync(0xffffffffu, st, o);
-        cnt += __shfl_xor_sync(0xffffffffu, cnt, o);
+        any |= __shfl_xor_sync(0xffffffffu, any, o);
         const long long l2 = __shfl_xor_sync(0xffffffffu, lo, o), h2 = __shfl_xor_sync(0xffffffffu, hi, o);
         lo = l2 < lo ? l2 : lo; hi = h2 > hi ? h2 : hi;
     }
-    if (lane == 0) { s_lo[warp] = lo; s_hi[warp] = hi; s_st[warp] = st; s_cnt[warp] = cnt; }
+    if (lane == 0) { s_lo[warp] = lo; s_hi[warp] = hi; s_st[warp] = st; s_any[warp] = any; }
     __syncthreads();
-    st = 0; cnt = 0; lo = INT64_MAX; hi = INT64_MIN;
+    st = 0; any = 0; lo = INT64_MAX; hi = INT64_MIN;
 #pragma unroll
     for (int w = 0; w < WARPS; ++w) {
-        st |= s_st[w]; cnt += s_cnt[w];
+        st |= s_st[w]; any |= s_any[w];
         lo = s_lo[w] < lo ? s_lo[w] : lo; hi = s_hi[w] > hi ? s_hi[w] : hi;
     }
     __syncthreads();                                                 // the slots are reused by the next call
     if (keep && tid == 0) keep[0] = 0;
     if (st) return zero<N>(st);
-    if (!cnt) return zero<N>();
-    int logc = 0;
-    while ((1u << logc) < cnt + 2) ++logc;
+    if (!any) return zero<N>();
+    int logc = 0;                                                    // K terms and one more sum below 2^logc of the largest
+    while ((1ull << logc) < K + 2) ++logc;
     Num<N> r = zero<N>();
     if (hi - lo + logc + 1 >= 32 * (long long)W) {
         if (tid == 0) store<N>(s_res, src.fallback(error));
