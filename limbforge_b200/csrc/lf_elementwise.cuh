@@ -28,8 +28,10 @@ constexpr int kEwThreads = 128;
 // A block's rows (elements, or components of complex values) pass through shared memory: a thread's own N + 3 words lie
 // (N + 3) words from its neighbour's, so a load of one word by a warp touches some N + 3 cache lines, and the element-wise
 // kernels were bound by those (300,000 512-bit sums: 35 us, 1.9 TB/s).  Tiles are copied with cp.async, in
-// 16-byte pieces where the block is whole and the arrays are aligned, word by word otherwise (a last block, a broadcast
-// operand, an even row length: those rows are padded to an odd stride, free of bank conflicts).
+// 16-byte pieces where the block is whole and the arrays are aligned, word by word otherwise (a last block, an even row
+// length: those rows are padded to an odd stride, free of bank conflicts).  A thread copies its own row of a broadcast operand, whose few
+// elements L1 holds, and forms its index once (formed for every word, the index's two divisions cost 500,000 96-bit products
+// 6 us of 41).
 template <int N> constexpr int ew_stride() { return (N + 3) | 1; }
 template <int N> __device__ __forceinline__ void ew_fetch(u32* tile, const u32* src, u64 row0, int rows, u64 bs, u64 bp, int parts, bool wide) {
     constexpr int E = N + 3, S = ew_stride<N>();
@@ -40,12 +42,11 @@ template <int N> __device__ __forceinline__ void ew_fetch(u32* tile, const u32* 
         } else {
             for (int w = threadIdx.x; w < rows * E; w += kEwThreads) cp_async4(tile + w + (w / E) * (S - E), src + w);
         }
-    } else {
-        for (int w = threadIdx.x; w < rows * E; w += kEwThreads) {
-            const int e = w / E;
-            const u64 row = row0 + e, j = parts == 2 ? 2 * bidx(row >> 1, bs, bp) + (row & 1) : bidx(row, bs, bp);
-            cp_async4(tile + w + e * (S - E), src + j * E + (w - e * E));
-        }
+    } else if ((int)threadIdx.x < rows) {
+        const u64 row = row0 + threadIdx.x, j = parts == 2 ? 2 * bidx(row >> 1, bs, bp) + (row & 1) : bidx(row, bs, bp);
+        u32* const mine = tile + threadIdx.x * S;
+#pragma unroll
+        for (int w = 0; w < E; ++w) mine[w] = __ldg(src + j * E + w);
     }
 }
 template <int N> __device__ __forceinline__ void ew_put(const u32* tile, u32* dst, u64 row0, int rows, bool wide) {
