@@ -90,7 +90,8 @@ void exact_product_on(Linalg& la, const ProductLane& lane, int bits, lfd::LineVi
         const bool seen = method != 1 && !la.options.force_fallback && lane.residue->left_info;
         wp.spread = seen ? lane.residue->spread : -1;
         if (lfd::long_dot_fits(n, M, Nc, K, wp.spread)) {
-            lfd::long_dot_launcher(n)(p, s);                   // few outputs, long sums: a block per output
+            // few outputs, long sums: a block per output (left, the outputs it could not hold)
+            lfd::long_dot_launcher(n)(p, static_cast<uint32_t*>(lane.lines->get(sizeof(uint32_t) * M * Nc + 64)), s);
         } else {
             // the tiled limb kernel: line analysis, then one exact window per output (cluster method for wide outputs)
             if (seen) {
