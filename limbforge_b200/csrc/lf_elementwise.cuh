@@ -335,6 +335,10 @@ template <int N, int OP> void launch_ew_op(const EwParams& p, cudaStream_t s) {
     const unsigned blocks = (unsigned)(((ew_complex(OP) ? 2 * p.count : p.count) + kEwThreads - 1) / kEwThreads);
     if constexpr (ew_complex(OP)) {
         if constexpr (smem > 48 * 1024) cudaFuncSetAttribute(ew_pair_kernel<N, OP>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        // Fused operations whose exponents lie far apart sum by clusters in thread-local windows, which need L1: up to 8 limbs the tiles of three or
+        // four blocks fit a 64 KB step of shared memory.  60,000 values, exponents of +-3000: 8 limbs 137 us by default, 100 so; 5 limbs 69
+        // and 50; wider, and with near exponents (8 limbs 24 us), the default serves as well.
+        if constexpr (OP >= 11 && N <= 8) cudaFuncSetAttribute(ew_pair_kernel<N, OP>, cudaFuncAttributePreferredSharedMemoryCarveout, 28);
         ew_pair_kernel<N, OP><<<blocks, kEwThreads, smem, s>>>(p);
     } else {
         if constexpr (smem > 48 * 1024) cudaFuncSetAttribute(ew_kernel<N, OP>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);

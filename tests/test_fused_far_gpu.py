@@ -1,0 +1,21 @@
+"""GPU: fused complex operations whose terms lie too far apart for one window (they sum by clusters), beside near ones in the same
+block, at the widths around the kernels' shared-memory rule, against the oracle."""
+import numpy as np
+import pytest
+
+from limbforge_b200 import api
+from limbforge_b200 import numbers as nb
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("bits", [64, 256, 288, 1024])
+@pytest.mark.parametrize("op", ["complex_fma", "complex_fms"])
+def test_far_terms(engine, oracle, bits, op):
+    op = api.Operation[op]
+    rng = np.random.default_rng(bits + int(op))
+    count = 1000
+    ins = [nb.random_complex(rng, count, bits, span, zero_frac=0.02, sparse_frac=0.05) for span in (8, 3000, 300)]
+    ins[1][::3] = nb.random_complex(rng, len(ins[1][::3]), bits, 8)
+    out, _ = engine.run_ternary(bits, op, *ins)
+    assert (out == oracle.elementwise(bits, int(op), *ins)).all()
