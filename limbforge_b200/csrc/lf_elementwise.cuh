@@ -191,8 +191,12 @@ template <int N, bool MUL_ONLY> __global__ void __launch_bounds__(kChainThreads)
 // a block of 32 values copies the next step's 32 factors (one contiguous tile of 32 (N+3) words, a
 // multiple of 16 bytes) into shared memory with cp.async while the current products run, so the product
 // reads its factor words from shared memory.  A partial last block reads its factors directly.
+// Above 24 limbs the registers are held to 128, 16 blocks an SM, where the compiler would take some 160 (12 blocks): a block is one warp, and the
+// products leave the pipe idle with twelve.  Eight products of 1,000 to 500,000 values at 800, 896, 960 and 1024 bits, 12 blocks against 16:
+// 65,536 values 45 / 63 / 70 / 71 us and 42 / 54 / 59 / 67, 500,000 values 224 / 292 / 324 / 358 and 218 / 278 / 306 / 347; of 32 counts and
+// widths two were slower (1024 bits: 30,000 values by 2%, 131,072 by 5%).
 constexpr int kStagedThreads = 32;
-template <int N> __global__ void __launch_bounds__(kStagedThreads, (N > 24 ? 14 : 1)) chain_staged_kernel(const __grid_constant__ ChainParams p) {
+template <int N> __global__ void __launch_bounds__(kStagedThreads, (N > 24 ? 16 : 1)) chain_staged_kernel(const __grid_constant__ ChainParams p) {
     constexpr u64 E = N + 3;
     constexpr int T = kStagedThreads, TILE = T * (int)E, CH = TILE / 4;
     static_assert(TILE % 4 == 0, "tiles of whole 16-byte chunks");
