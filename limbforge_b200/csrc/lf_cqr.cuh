@@ -449,7 +449,7 @@ template <int N> struct CReducedSquares {
         const Num<N> a = z(t);
         u32 prod[2 * N];
         mant_mul<N>(a.m, a.m, prod);
-        acc_add(acc, len, prod, 2 * N, off);
+        acc_add(acc, len, prod, off);
     }
     __device__ Num<N> fallback(u32* error) const {
         u32 st = 0;
