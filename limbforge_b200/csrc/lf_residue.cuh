@@ -4,12 +4,13 @@
 //  1. digits: every entry of a line becomes the exact integer X = mantissa * 2^(e - bottom(line))
 //     (< 2^(32N+G), G = widest line spread), reduced modulo L primes m_l < 2^16 to a balanced
 //     residue r = 256 d1 + d0 with int8 digits; planes D1/D0 [L][rows][Kp] (K-major, zero padded).
-//  2. mma: per modulus and 128x128 output tile, tcgen05.mma kind::i8 with int32 accumulators in
+//  2. mma: per modulus and 128x80 output tile, tcgen05.mma kind::i8 with int32 accumulators in
 //     TMEM: S11 = D1a D1b^T, S00 = D0a D0b^T, Smid = D1a D0b^T + D0a D1b^T; operands fed by TMA
-//     (128-byte swizzle, no multicast); epilogue r = (65536 S11 + 256 Smid + S00) mod m -> uint16.
+//     (128-byte swizzle, no multicast); epilogue r = (65536 S11 + 256 Smid + S00) mod m -> uint16, for the tensor-core
+//     CRT already weighted: t = r (M/m_l)^-1 mod m_l.
 //  3. reconstruct: per output, CRT of the L residues (X = sum_l t_l (M/m_l) - q M, q = round of the
 //     fixed-point sum of t_l/m_l; the modulus product exceeds 4 max|X| so the rounding of q is never
-//     close), then RN(c - X 2^scale) (or RN(X 2^scale)) with one rounding.
+//     close), then RN(c - X 2^scale) (or RN(X 2^scale)) with one rounding; the sums over l are a second int8 product.
 // Every step is exact integer arithmetic, so the outputs equal the generic limb kernel's bit for bit.
 #pragma once
 #include "lf_linalg.cuh"
