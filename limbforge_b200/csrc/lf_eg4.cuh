@@ -8,6 +8,7 @@
 // is summed on the GPU.
 #pragma once
 #include "lf_linalg.cuh"
+#include "lf_carveout.h"
 
 namespace lfd {
 
@@ -214,7 +215,10 @@ template <int N, bool CX> void eg4_launch_v(const Eg4Params& pin, cudaStream_t s
     const u64 strides = p.count > 1 ? (p.sa | p.sb | p.sc) * S : 0;
     p.wide = !(((uintptr_t)p.A | (uintptr_t)p.B | (uintptr_t)p.C | 4 * strides) & 15);
     static_assert(smem <= 48 * 1024, "tiles need no larger limit");
-    if constexpr (smem > 0) cudaFuncSetAttribute(exact_gemm4_kernel<N, CX>, cudaFuncAttributePreferredSharedMemoryCarveout, eg4_carveout<N, CX>());
+    if constexpr (smem > 0) {
+        static std::atomic<uint64_t> asked{0};
+        prefer_carveout(exact_gemm4_kernel<N, CX>, eg4_carveout<N, CX>(), asked);
+    }
     const unsigned blocks = (unsigned)((p.count + eg4_matrices<CX>() - 1) / eg4_matrices<CX>());
     exact_gemm4_kernel<N, CX><<<blocks, kEg4Threads, smem, s>>>(p);
 }

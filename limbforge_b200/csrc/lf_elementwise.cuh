@@ -4,6 +4,7 @@
 // registers across every step (the fused form of a resident CommandBatch chain).
 #pragma once
 #include "lf_arith.cuh"
+#include "lf_carveout.h"
 #include <cuda_runtime.h>
 #include <cstdint>
 
@@ -61,7 +62,15 @@ template <int N> __device__ __forceinline__ void ew_put(const u32* tile, u32* ds
 }
 constexpr bool ew_complex(int op) { return op == 4 || op == 5 || op == 6 || op == 11 || op == 12; }
 constexpr int ew_inputs(int op) { return op == 7 || op == 8 ? 1 : op >= 9 ? 3 : 2; }
-template <int N> constexpr size_t ew_smem_bytes(int op) { return (size_t)ew_inputs(op) * kEwThreads * ew_stride<N>() * 4; }
+// Fused complex operations whose exponents lie far apart sum by clusters in thread-local windows, which need L1: shared memory that the driver sets
+// aside for more blocks costs them more than it brings.  Up to 12 limbs the kernels therefore read the addend straight from memory (two
+// tiles) and run in the 64 KB step of shared memory (28% of 228 KB), four blocks of 12 limbs.  200,000 values, us, a thread a value / three tiles by
+// default / this: 8 limbs, near exponents 91 / 52 / 51, +-300 238 / 254 / 223, +-3000 292 / 335 / 284; 12 limbs 173 / 79 / 75, 448 / 343 / 321,
+// 661 / 618 / 568; 5 limbs 62 / 38 / 38, 163 / 198 / 175, 158 / 173 / 154; 3 limbs 34 / 32 / 30, 95 / 120 / 104, 84 / 94 / 82.  (32 KB would
+// take 5 limbs to 131 and 125 there, and from 38 to 44 with near exponents.)  Wider kernels hold few blocks anyway (13 limbs, near: default
+// 89, 64 KB 95).
+template <int N> constexpr int ew_tiles(int op) { return op >= 11 && N <= 12 ? 2 : ew_inputs(op); }
+template <int N> constexpr size_t ew_smem_bytes(int op) { return (size_t)ew_tiles<N>(op) * kEwThreads * ew_stride<N>() * 4; }
 // The block's rows of every operand, in tiles of kEwThreads rows; returns how many rows the block has.
 template <int N, int OP> __device__ __forceinline__ int ew_load_tiles(const EwParams& p, u32* tile, u64 row0, bool& wide) {
     constexpr int parts = ew_complex(OP) ? 2 : 1, T = kEwThreads * ew_stride<N>();
@@ -70,7 +79,7 @@ template <int N, int OP> __device__ __forceinline__ int ew_load_tiles(const EwPa
     wide = p.aligned && rows == kEwThreads;
     ew_fetch<N>(tile, p.a, row0, rows, 1, 0, parts, wide);
     if constexpr (ew_inputs(OP) > 1) ew_fetch<N>(tile + T, p.b, row0, rows, p.bs, p.bp, parts, wide);
-    if constexpr (ew_inputs(OP) > 2) ew_fetch<N>(tile + 2 * T, p.c, row0, rows, p.cs, p.cp, parts, wide);
+    if constexpr (ew_tiles<N>(OP) > 2) ew_fetch<N>(tile + 2 * T, p.c, row0, rows, p.cs, p.cp, parts, wide);
     cp_async_commit();
     cp_async_wait<0>();
     __syncthreads();
@@ -79,11 +88,11 @@ template <int N, int OP> __device__ __forceinline__ int ew_load_tiles(const EwPa
 
 template <int N, int OP> __global__ void __launch_bounds__(kEwThreads) ew_kernel(EwParams p) {
     constexpr int S = ew_stride<N>(), T = kEwThreads * S;
-    extern __shared__ __align__(16) u32 ew_tiles[];
+    extern __shared__ __align__(16) u32 ew_park[];
     const u64 row0 = (u64)blockIdx.x * kEwThreads;
     bool wide;
-    const int rows = ew_load_tiles<N, OP>(p, ew_tiles, row0, wide);
-    u32* const mine = ew_tiles + threadIdx.x * S;
+    const int rows = ew_load_tiles<N, OP>(p, ew_park, row0, wide);
+    u32* const mine = ew_park + threadIdx.x * S;
     if ((int)threadIdx.x < rows) {
         const Num<N> x = load_plain<N>(mine);
         Num<N> z;
@@ -103,7 +112,7 @@ template <int N, int OP> __global__ void __launch_bounds__(kEwThreads) ew_kernel
         store<N>(mine, z);
     }
     __syncthreads();
-    ew_put<N>(ew_tiles, p.out, row0, rows, wide);
+    ew_put<N>(ew_park, p.out, row0, rows, wide);
 }
 
 // Complex operations: two lanes per value, one component each (lane 2q real, 2q + 1 imaginary).  The components are
@@ -115,12 +124,18 @@ template <int N, int OP> __global__ void __launch_bounds__(kEwThreads) ew_kernel
 // either writes its result over the first operand's row.
 template <int N, int OP> __global__ void __launch_bounds__(kEwThreads, (N > 16 && OP <= 6 ? 3 : 1)) ew_pair_kernel(EwParams p) {
     constexpr int S = ew_stride<N>(), T = kEwThreads * S;
-    extern __shared__ __align__(16) u32 ew_tiles[];
+    extern __shared__ __align__(16) u32 ew_park[];
     const u64 row0 = (u64)blockIdx.x * kEwThreads;
+    constexpr bool kAddendTile = ew_tiles<N>(OP) > 2;
+    Num<N> w = zero<N>();
+    if constexpr (OP >= 11 && !kAddendTile) {                     // this lane's component of the addend
+        const u64 row = row0 + threadIdx.x;
+        if (row < 2 * p.count) w = load<N>(p.c + (p.cs == 1 && !p.cp ? row : 2 * bidx(row >> 1, p.cs, p.cp) + (row & 1)) * (N + 3));
+    }
     bool wide;
-    const int rows = ew_load_tiles<N, OP>(p, ew_tiles, row0, wide);
+    const int rows = ew_load_tiles<N, OP>(p, ew_park, row0, wide);
     const int im = (int)(threadIdx.x & 1);
-    u32* const a = ew_tiles + (threadIdx.x & ~1u) * S;            // the value's real row; its imaginary row follows
+    u32* const a = ew_park + (threadIdx.x & ~1u) * S;            // the value's real row; its imaginary row follows
     const u32* const b = a + T;
     if ((int)threadIdx.x < rows) {                                // rows is even: both lanes of a pair, or neither
         const u32 pair = 3u << (threadIdx.x & 30u);
@@ -152,14 +167,15 @@ template <int N, int OP> __global__ void __launch_bounds__(kEwThreads, (N > 16 &
             }
             if constexpr (OP == 6) z = div<N>(z, first); else z = first;
         } else {
-            const Num<N> ai = load_plain<N>(a + S), w = load_plain<N>(a + 2 * T + im * S);
+            if constexpr (kAddendTile) w = load_plain<N>(a + 2 * T + im * S);
+            const Num<N> ai = load_plain<N>(a + S);
             z = dot2_add<N>(load_plain<N>(a), load_plain<N>(b + im * S), im ? ai : negate<N>(ai), load_plain<N>(b + (im ^ 1) * S), OP == 12 ? negate<N>(w) : w);
         }
         __syncwarp(pair);
         store<N>(a + im * S, z);
     }
     __syncthreads();
-    ew_put<N>(ew_tiles, p.out, row0, rows, wide);
+    ew_put<N>(ew_park, p.out, row0, rows, wide);
 }
 
 // v <- op_s(v, b_s[...]) for every step; out_s written where non-null.  Steps are uniform across
@@ -339,10 +355,10 @@ template <int N, int OP> void launch_ew_op(const EwParams& p, cudaStream_t s) {
     const unsigned blocks = (unsigned)(((ew_complex(OP) ? 2 * p.count : p.count) + kEwThreads - 1) / kEwThreads);
     if constexpr (ew_complex(OP)) {
         if constexpr (smem > 48 * 1024) cudaFuncSetAttribute(ew_pair_kernel<N, OP>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        // Fused operations whose exponents lie far apart sum by clusters in thread-local windows, which need L1: up to 8 limbs the tiles of three or
-        // four blocks fit a 64 KB step of shared memory.  60,000 values, exponents of +-3000: 8 limbs 137 us by default, 100 so; 5 limbs 69
-        // and 50; wider, and with near exponents (8 limbs 24 us), the default serves as well.
-        if constexpr (OP >= 11 && N <= 8) cudaFuncSetAttribute(ew_pair_kernel<N, OP>, cudaFuncAttributePreferredSharedMemoryCarveout, 28);
+        if constexpr (ew_tiles<N>(OP) < ew_inputs(OP)) {
+            static std::atomic<uint64_t> asked{0};
+            prefer_carveout(ew_pair_kernel<N, OP>, 28, asked);
+        }
         ew_pair_kernel<N, OP><<<blocks, kEwThreads, smem, s>>>(p);
     } else {
         if constexpr (smem > 48 * 1024) cudaFuncSetAttribute(ew_kernel<N, OP>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
