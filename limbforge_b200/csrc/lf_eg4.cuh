@@ -115,8 +115,8 @@ template <int N, bool CX> __device__ bool eg4_window_sum(const u32* a, const u32
 // an entry.  The results replace A's matrices in the tile and leave as whole matrices (the padding between output matrices is kept).
 // The tiles take L1 from the thread-local windows of cluster_round, so components that need it lose what the others gain:
 //   - above 16 limbs every component sums by clusters: unstaged (20,000 complex matrices of 32 limbs: 5.25 ms staged, 2.66 not);
-//   - real matrices up to 8 limbs have few lines an entry, and staging gains nothing (8 limbs: 43 us either way; exponents of +-1000,
-//     by clusters: 2.8 ms staged, 2.3 not);
+//   - real matrices up to 7 limbs have few lines an entry, and staging gains nothing (7 limbs: 39 us either way; exponents of +-1000,
+//     by clusters: 1.96 ms staged, 1.52 not);
 //   - the others stage and leave the rest of the array to L1 (eg4_carveout).
 constexpr int kEg4Threads = 128;
 template <bool CX> constexpr int eg4_matrices() { return kEg4Threads / (CX ? 32 : 16); }
@@ -136,7 +136,7 @@ template <int MW> __device__ __forceinline__ void eg4_fetch(u32* tile, const u32
         }
     }
 }
-template <int N, bool CX> constexpr bool eg4_staged() { return N <= 16 && (CX || N > 8); }
+template <int N, bool CX> constexpr bool eg4_staged() { return N <= 16 && (CX || N > 7); }
 // Shared memory to set aside, in percent of 228 KB: the hardware's step of 32, 64 or 100 KB that holds four blocks (N + 4 KB each, the system's
 // included).  Left to the driver, shared memory got what it could and cluster sums slowed: 20,000 complex matrices of 14 limbs with
 // exponents of +-200 took 6.6 ms, so 1.11; +-30: 0.23 either way.  Real matrices of 13 limbs do with three blocks (72 us,
